@@ -8,12 +8,39 @@ namespace mayo {
 
 __host__ __device__ constexpr size_t pad16(size_t x) { return (x + 15) / 16 * 16; }
 
+// CTAs per instance of the per-instance sign and verify: a batch that leaves SMs idle gives each
+// instance a cluster of them, as many as one wave holds (16, 36 and 72 clusters of 8, 4 and 2 run at
+// once; 12 and 32 leave room for other work).  MAYO_5 verify, us: batch 8 31 (8 CTAs) against 41
+// (4), 18 58 against 41; 24 42 (4) against 63 (2), 36 79 against 64; 72 64 (2) against 109 (1),
+// 100 125 against 109.
+inline int cluster_ctas(size_t batch) { return batch <= 12 ? 8 : batch <= 32 ? 4 : batch <= 72 ? 2 : 1; }
+
 // Opt `kernel` into `bytes` of dynamic shared memory on the current device.  The attribute is
 // per kernel and per device; setting it is a cheap host call that is not a stream operation.
 template <class K>
 inline bool set_smem_attr(K kernel, size_t bytes) {
     if (bytes <= 48 * 1024) return true;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+}
+
+// Launch `kernel` on clusters of `cl` CTAs (cl = 1: a plain launch); ctas is a multiple of cl.
+template <class... P, class... A>
+inline cudaError_t launch_cluster(void (*kernel)(P...), unsigned ctas, unsigned threads, size_t smem, unsigned cl,
+                                  cudaStream_t st, const A &...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (cl > 1) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cl;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 }  // namespace mayo

@@ -244,12 +244,12 @@ template <int SET>
 __device__ void queue_sign(uint8_t *smem, int tid, const QueueArgs &q, const ItemRefs &r, uint32_t inst, int ctr,
                            uint32_t item) {
     using S = Set<SET>;
-    constexpr int NT = QueueCfg<SET, MAYO_B200_OP_SIGN>::NT;
-    sign_hash_cta<SET, NT>(smem, tid, r.key, r.msg, r.mlen, ctr);
-    const bool ok = sign_attempt<SET, NT>(smem, tid, r.key);
+    using C = SignCfg<SET>;
+    sign_hash_cta<C>(smem, tid, r.key, r.msg, r.mlen, ctr);
+    const bool ok = sign_attempt<C>(smem, tid, r.key);
     if (ok || ctr >= 254) {
         // success, or the 255th rejection: the reference emits the last attempt (x = r)
-        sign_write<SET, NT>(smem, tid, r.key, q.ops.sg_sig + (size_t)inst * S::sig);
+        sign_write<C>(smem, tid, r.key, q.ops.sg_sig + (size_t)inst * S::sig);
     } else if (tid == 0) {
         queue_push(q, (item & ~(0xFFu << 20)) | ((uint32_t)(ctr + 1) << 20));
     }
@@ -276,8 +276,7 @@ __global__ void __launch_bounds__(QueueCfg<SET, OP>::NT, QueueFit<SET, OP>::MINB
         } else if constexpr (OP == MAYO_B200_OP_SIGN) {
             queue_sign<SET>(smem, tid, q, r, inst, (int)((item >> 20) & 0xFF), item);
         } else {
-            verify_instance<SET, VerifyCfg<SET>::NC>(smem, tid, r.key, r.msg, r.mlen,
-                                                     q.ops.vf_sig + (size_t)inst * S::sig, q.ops.vf_res + inst);
+            verify_instance<SET>(smem, tid, r.key, r.msg, r.mlen, q.ops.vf_sig + (size_t)inst * S::sig, q.ops.vf_res + inst);
         }
         __syncthreads();
         if (tid == 0) {

@@ -911,7 +911,7 @@ struct TailShape {
     // MAYO_2: 69); the engine's row slots shrink with them (R = 3 / 12).  More signatures per SM
     // at the same registers: MAYO_2 G = 4, 4 CTAs of 384 threads at 40 registers (16 signatures
     // per SM against 12 with 128 threads), 1.643 -> 1.494 ms at 65,536.
-    static constexpr int TNT = (SET == 1 || SET == 2) ? 96 : SignCfg<SET>::NT;
+    static constexpr int TNT = (SET == 1 || SET == 2) ? 96 : (SET == 5 ? 160 : 128);
     static constexpr int NT = TNT * G;
     // MAYO_5: 5 CTAs of 160 threads per SM held to a register budget (72 registers)
     // MAYO_2: the elimination's per-step chain needs signatures in flight more than registers.
@@ -919,15 +919,17 @@ struct TailShape {
     // G = 2 with 5 CTAs (48 registers) 1.739 ms (4 CTAs: 1.889, 6: 1.777); G = 4 with 3 CTAs
     // (40 registers, 12 signatures per SM) 1.661 ms (2 CTAs: 2.055).  With 96 threads: G = 2 at 7
     // CTAs and G = 4 at 4 CTAs per SM (the same registers).
-    static constexpr int MINB = SET == 5 ? (G == 1 ? 5 : 2) : (SET == 2 ? (G == 1 ? 1 : G == 2 ? 7 : 4) : 1);
-    static constexpr size_t SMEM = (size_t)G * SignCfg<SET, TNT, true>::total;
+    static constexpr int MINB = SET == 5 ? (G == 1 ? 5 : 2)
+                                : SET == 2 ? (G == 1 ? 1 : G == 2 ? 7 : 4)
+                                : SET == 1 ? (G == 1 ? 8 : G == 2 ? 4 : 2) : 1;
+    static constexpr size_t SMEM = (size_t)G * SignTailCfg<SET, TNT>::total;
 };
 template <int SET, int G>
 __global__ void __launch_bounds__(TailShape<SET, G>::NT, TailShape<SET, G>::MINB)
     sign_shared_tail_kernel(const uint8_t *esk, uint8_t *sig, size_t sig_stride, const uint8_t *wsi, size_t wsi_stride,
                             const uint4 *planes, const uint4 *opl, uint32_t *ctl, uint32_t *retry, uint32_t batch) {
     using P = SharedProb<SET, false>;
-    using C = SignCfg<SET, TailShape<SET, G>::TNT, true>;
+    using C = SignTailCfg<SET, TailShape<SET, G>::TNT>;
     constexpr int NT = C::NT;
     extern __shared__ __align__(16) uint8_t smem0[];
     if (ctl[0]) return;  // the product gave up: the fix-up kernel signs everything
@@ -936,33 +938,33 @@ __global__ void __launch_bounds__(TailShape<SET, G>::NT, TailShape<SET, G>::MINB
     const bool live = inst < batch;
     const uint32_t src = live ? inst : batch - 1;
     uint8_t *smem = smem0 + (size_t)g * C::total;
-    sign_load_ws<SET, NT, true>(smem, tid, esk, wsi + (size_t)src * wsi_stride);
-    const bool ok = sign_attempt<SET, NT, true, G>(smem0, T, esk, planes + (size_t)src * P::PLANES);
-    sign_write<SET, NT, true>(smem, tid, esk, ok && live ? sig + (size_t)inst * sig_stride : nullptr, opl);
+    sign_load_ws<C>(smem, tid, esk, wsi + (size_t)src * wsi_stride);
+    const bool ok = sign_attempt<C, G>(smem0, T, esk, planes + (size_t)src * P::PLANES);
+    sign_write<C>(smem, tid, esk, ok && live ? sig + (size_t)inst * sig_stride : nullptr, opl);
     if (!ok && live && tid == 0) retry[atomicAdd(&ctl[1], 1u)] = inst;
 }
 
 // Retries (attempts ctr >= 1 of the listed instances) with the engine, or every instance from
 // ctr = 0 if the product gave up.  A grid-stride loop over a count read on the device.
 template <int SET>
-__global__ void __launch_bounds__(SignCfg<SET>::NT)
+__global__ void __launch_bounds__(SignCfg<SET>::NT, SignCfg<SET>::MINB)
     sign_shared_fix_kernel(const uint8_t *esk, uint8_t *sig, size_t sig_stride, const uint8_t *wsi, size_t wsi_stride,
                            const uint4 *opl, const uint32_t *ctl, const uint32_t *retry, uint32_t batch) {
     extern __shared__ __align__(16) uint8_t smem[];
-    constexpr int NT = SignCfg<SET>::NT;
+    using C = SignCfg<SET>;
     const int tid = threadIdx.x;
     const bool all = ctl[0] != 0;
     const uint32_t count = all ? batch : ctl[1];
 #pragma unroll 1
     for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
         const uint32_t inst = all ? idx : retry[idx];
-        sign_load_ws<SET, NT>(smem, tid, esk, wsi + (size_t)inst * wsi_stride);
+        sign_load_ws<C>(smem, tid, esk, wsi + (size_t)inst * wsi_stride);
 #pragma unroll 1
         for (int ctr = all ? 0 : 1; ctr < 255; ctr++) {
-            if (ctr > 0) sign_next_vr<SET, NT>(smem, tid, ctr);
-            if (sign_attempt<SET, NT>(smem, tid, esk)) break;
+            if (ctr > 0) sign_next_vr<C>(smem, tid, ctr);
+            if (sign_attempt<C>(smem, tid, esk)) break;
         }
-        sign_write<SET, NT>(smem, tid, esk, sig + (size_t)inst * sig_stride, opl);
+        sign_write<C>(smem, tid, esk, sig + (size_t)inst * sig_stride, opl);
         __syncthreads();
     }
 }
@@ -1007,7 +1009,8 @@ struct VTailCfg {
     static constexpr size_t off_masks = 0;
     static constexpr size_t off_x = off_masks + (size_t)S::n * J * 16;
     static constexpr size_t off_upk = off_x + (size_t)J * J * W * 16;
-    static constexpr size_t off_t = off_upk + pad16((size_t)S::pairs * NW * 4);
+    static constexpr size_t off_yext = off_upk + pad16((size_t)S::pairs * NW * 4);
+    static constexpr size_t off_t = off_yext + 128;
     static constexpr size_t total = off_t + pad16((size_t)NW * 4);
 };
 
@@ -1025,8 +1028,10 @@ __global__ void __launch_bounds__(VTailCfg<SET>::NT)
     uint4 *xacc = reinterpret_cast<uint4 *>(smem + C::off_x);
     uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);
     uint32_t *s_t = reinterpret_cast<uint32_t *>(smem + C::off_t);
+    uint32_t *yext = reinterpret_cast<uint32_t *>(smem + C::off_yext);
     const int tid = threadIdx.x;
     const size_t inst = blockIdx.x;
+    if (tid < 32) yext[tid] = 0;
     const uint8_t *sig = io.sig + inst * io.sig_stride;
     for (int idx = tid; idx < S::n * J; idx += C::NT) {  // column c of s_j (src/verify.cu:62-70)
         const int c = idx / J, jj = idx - c * J;
@@ -1066,37 +1071,32 @@ __global__ void __launch_bounds__(VTailCfg<SET>::NT)
         if (i != j) u = g4_xor(u, g4_ld(xacc + ((size_t)j * J + i) * W + ww));
         const uint4 pk = g4_to_packed(u);
         const uint32_t wd[4] = {pk.x, pk.y, pk.z, pk.w};
+        const int l = pair_ell(i, j, J);
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            if (4 * ww + q < NW) upk[pid * NW + 4 * ww + q] = wd[q];
+            if (4 * ww + q < NW) upk[l * NW + 4 * ww + q] = wd[q];
     }
     __syncthreads();
-    if (tid < 32) {  // y = Horner over the pairs (i = k-1..0, j = i..k-1), compare (src/verify.cu:185-211)
-        const int lane = tid;
-        uint32_t y = 0;
-#pragma unroll 1
-        for (int i = S::k - 1; i >= 0; i--)
-#pragma unroll 1
-            for (int j = i; j < S::k; j++) {
-                y = times_z_lane<SET>(y, lane);
-                if (lane < NW) y ^= upk[pair_index(i, j, S::k) * NW + lane];
-            }
-        const uint32_t tw = lane < NW ? s_t[lane] : 0u;
+    y_accumulate<SET>(upk, yext, tid >> 5, C::NT / 32, tid & 31);  // y = sum z^l U_l, compare (src/verify.cu:185-211)
+    __syncthreads();
+    if (tid < 32) {
+        const uint32_t y = y_fold<SET>(yext, tid);
+        const uint32_t tw = tid < NW ? s_t[tid] : 0u;
         const bool eq = __all_sync(0xffffffffu, y == tw);
-        if (lane == 0) io.res[inst * io.res_stride] = eq ? 0 : 1;
+        if (tid == 0) io.res[inst * io.res_stride] = eq ? 0 : 1;
     }
 }
 
 // Every instance with the engine, only if the product gave up.
 template <int SET>
-__global__ void __launch_bounds__(VerifyCfg<SET>::NT)
+__global__ void __launch_bounds__(VerifyCfg<SET>::NT, VerifyCfg<SET>::MINB)
     verify_shared_fix_kernel(const VerifyIO io, const uint32_t *ctl, uint32_t batch) {
     extern __shared__ __align__(16) uint8_t smem[];
     if (!ctl[0]) return;
 #pragma unroll 1
     for (uint32_t inst = blockIdx.x; inst < batch; inst += gridDim.x) {
-        verify_instance<SET, VerifyCfg<SET>::NC>(smem, threadIdx.x, io.epk, io.m.ptr(inst), io.m.len(inst),
-                                                 io.sig + (size_t)inst * io.sig_stride, io.res + inst * io.res_stride);
+        verify_instance<SET>(smem, threadIdx.x, io.epk, io.m.ptr(inst), io.m.len(inst),
+                             io.sig + (size_t)inst * io.sig_stride, io.res + inst * io.res_stride);
         __syncthreads();
     }
 }
@@ -1277,10 +1277,10 @@ int shared_timing_read(float *ms) {
 // Shared memory a sign-tail CTA of g instances needs (0 for a bad set).
 static size_t tail_smem(int set, int g) {
     switch (set) {
-        case 1: return (size_t)g * SignCfg<1, TailShape<1, 1>::TNT, true>::total;
-        case 2: return (size_t)g * SignCfg<2, TailShape<2, 1>::TNT, true>::total;
-        case 3: return (size_t)g * SignCfg<3, 0, true>::total;
-        case 5: return (size_t)g * SignCfg<5, 0, true>::total;
+        case 1: return (size_t)g * SignTailCfg<1, TailShape<1, 1>::TNT>::total;
+        case 2: return (size_t)g * SignTailCfg<2, TailShape<2, 1>::TNT>::total;
+        case 3: return (size_t)g * SignTailCfg<3, TailShape<3, 1>::TNT>::total;
+        case 5: return (size_t)g * SignTailCfg<5, TailShape<5, 1>::TNT>::total;
         default: return 0;
     }
 }

@@ -65,29 +65,47 @@ __global__ void sign_hash_kernel(const SignIO io, uint32_t batch, const uint32_t
     }
 }
 
-template <int SET>
-__global__ void __launch_bounds__(SignCfg<SET>::NT) sign_kernel(const SignIO io) {
+template <int SET, int CL>
+__global__ void __launch_bounds__(SignCfg<SET, CL>::NT, SignCfg<SET, CL>::MINB) sign_kernel(const SignIO io) {
     extern __shared__ __align__(16) uint8_t smem[];
-    constexpr int NT = SignCfg<SET>::NT;
-    const int tid = threadIdx.x;
-    const size_t inst = blockIdx.x;
+    using C = SignCfg<SET, CL>;
+    const int tid = threadIdx.x, rank = CL > 1 ? (int)cluster_rank() : 0;
+    const size_t inst = blockIdx.x / CL;
     const uint8_t *esk = io.esk + inst * io.esk_stride;
-    sign_load_ws<SET, NT>(smem, tid, esk, io.ws + inst * io.ws_stride);
+    sign_load_ws<C>(smem, tid, esk, io.ws + inst * io.ws_stride);
 #pragma unroll 1
     for (int ctr = 0; ctr < 255; ctr++) {
-        if (ctr > 0) sign_next_vr<SET, NT>(smem, tid, ctr);
-        if (sign_attempt<SET, NT>(smem, tid, esk)) break;
+        if (ctr > 0) sign_next_vr<C>(smem, tid, ctr);
+        bool ok = sign_attempt<C>(smem, tid, esk, nullptr, rank);
+        if constexpr (CL > 1) {  // rank 0's verdict
+            cluster_barrier();
+            ok = ld_cluster(reinterpret_cast<const uint32_t *>(smem + C::off_flag), 0) != 0;
+            cluster_barrier();
+        }
+        if (ok) break;
     }
-    sign_write<SET, NT>(smem, tid, esk, io.sig + inst * io.sig_stride);
+    if (rank == 0) sign_write<C>(smem, tid, esk, io.sig + inst * io.sig_stride);
+}
+
+template <int SET, int CL>
+static int sign_cl(const SignIO &io, size_t batch, cudaStream_t st) {
+    using C = SignCfg<SET, CL>;
+    if (!set_smem_attr(sign_kernel<SET, CL>, C::total)) return ST_CUDA;
+    return launch_cluster(sign_kernel<SET, CL>, (unsigned)(batch * CL), C::NT, C::total, CL, st, io) == cudaSuccess
+               ? ST_OK
+               : ST_CUDA;
 }
 
 template <int SET>
 static int sign_t(const SignIO &io, size_t batch, cudaStream_t st) {
-    using C = SignCfg<SET>;
     sign_hash_kernel<SET><<<(unsigned)((batch + HASH_NT - 1) / HASH_NT), HASH_NT, 0, st>>>(io, (uint32_t)batch, nullptr);
-    if (!set_smem_attr(sign_kernel<SET>, C::total)) return ST_CUDA;
-    sign_kernel<SET><<<(unsigned)batch, C::NT, C::total, st>>>(io);
-    return cudaPeekAtLastError() == cudaSuccess ? ST_OK : ST_CUDA;
+    if (cudaPeekAtLastError() != cudaSuccess) return ST_CUDA;
+    switch (cluster_ctas(batch)) {
+        case 8: return sign_cl<SET, 8>(io, batch, st);
+        case 4: return sign_cl<SET, 4>(io, batch, st);
+        case 2: return sign_cl<SET, 2>(io, batch, st);
+        default: return sign_cl<SET, 1>(io, batch, st);
+    }
 }
 
 int launch_sign_hash(int set, const SignIO &io, size_t batch, cudaStream_t st, const uint32_t *order, int nt) {

@@ -5,30 +5,32 @@
 
 namespace mayo {
 
-template <int SET>
-__device__ __forceinline__ void verify_cta(const VerifyIO &io) {
+template <int SET, int CL>
+__global__ void __launch_bounds__(VerifyCfg<SET, CL>::NT, VerifyCfg<SET, CL>::MINB) verify_kernel(const VerifyIO io) {
     extern __shared__ __align__(16) uint8_t smem[];
-    const size_t inst = blockIdx.x;
-    verify_instance<SET, VerifyCfg<SET>::NC>(smem, threadIdx.x, io.epk + inst * io.epk_stride, io.m.ptr(inst),
-                                             io.m.len(inst), io.sig + inst * io.sig_stride,
-                                             io.res + inst * io.res_stride);
+    const size_t inst = blockIdx.x / CL;
+    verify_instance<SET, CL>(smem, threadIdx.x, io.epk + inst * io.epk_stride, io.m.ptr(inst), io.m.len(inst),
+                             io.sig + inst * io.sig_stride, io.res + inst * io.res_stride,
+                             CL > 1 ? (int)cluster_rank() : 0);
 }
-template <int SET>
-__global__ void __launch_bounds__(VerifyCfg<SET>::NT) verify_kernel(const VerifyIO io) {
-    verify_cta<SET>(io);
-}
-// MAYO_3: its shared memory allows 6 CTAs per SM; registers capped to match
-template <>
-__global__ void __launch_bounds__(VerifyCfg<3>::NT, 6) verify_kernel<3>(const VerifyIO io) {
-    verify_cta<3>(io);
+
+template <int SET, int CL>
+static int verify_cl(const VerifyIO &io, size_t batch, cudaStream_t st) {
+    using C = VerifyCfg<SET, CL>;
+    if (!set_smem_attr(verify_kernel<SET, CL>, C::total)) return ST_CUDA;
+    return launch_cluster(verify_kernel<SET, CL>, (unsigned)(batch * CL), C::NT, C::total, CL, st, io) == cudaSuccess
+               ? ST_OK
+               : ST_CUDA;
 }
 
 template <int SET>
 static int verify_t(const VerifyIO &io, size_t batch, cudaStream_t st) {
-    using C = VerifyCfg<SET>;
-    if (!set_smem_attr(verify_kernel<SET>, C::total)) return ST_CUDA;
-    verify_kernel<SET><<<(unsigned)batch, C::NT, C::total, st>>>(io);
-    return cudaPeekAtLastError() == cudaSuccess ? ST_OK : ST_CUDA;
+    switch (cluster_ctas(batch)) {
+        case 8: return verify_cl<SET, 8>(io, batch, st);
+        case 4: return verify_cl<SET, 4>(io, batch, st);
+        case 2: return verify_cl<SET, 2>(io, batch, st);
+        default: return verify_cl<SET, 1>(io, batch, st);
+    }
 }
 
 int launch_verify_io(int set, const VerifyIO &io, size_t batch, cudaStream_t st) {

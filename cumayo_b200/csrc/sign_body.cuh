@@ -1,8 +1,8 @@
 // sign_body.cuh -- one MAYO signature on one CTA (reference src/sign.cu:10-477), shared by the
 // batched sign kernel and the persistent work-queue kernel.
 //
-//   U = V^T P1 V and y = sum z^l U_l + t        engine over P1 rows          (sign.cu:396-460)
-//   M_i = V_i L                                  engine over the columns of L (sign.cu:256-330)
+//   U = V^T P1 V and y = sum z^l U_l + t, M_i = V_i L: the quads of rows of P1 and of columns of L
+//       in one pass over the key (quad.cuh; sign.cu:256-330, 396-460)
 //   A = sum z^l M                                packed z-shifts, one thread per column (sign.cu:333-393)
 //   x = solve(A, y, r)                           Gauss-Jordan over bit-planes, no data branches (sign.cu:10-145)
 // No branch and no memory address depends on a value derived from the secret key; only the
@@ -21,6 +21,7 @@
 #include "engine.cuh"
 #include "launch_util.cuh"
 #include "ops.h"
+#include "quad.cuh"
 
 namespace mayo {
 
@@ -33,70 +34,115 @@ struct SignWs {
     static_assert(total <= S::scratch, "workspace fits the reference scratch region");
 };
 
-// COMPACT: no engine staging (the first attempt from precomputed products only); the bit-plane
-// columns of A then get a region of their own.
-template <int SET, int NT_ = 0, bool COMPACT = false>
-struct SignCfg {
+// Shared memory of what follows the key products, from `at`: M, the pivot buffer, y, hashes, x.
+#define MAYO_SIGN_TAIL_LAYOUT(at)                                                                        \
+    static constexpr int NCOL = S::ko + 1;  /* columns of [A | y] */                                    \
+    static constexpr int CPT = (NCOL + NT - 1) / NT;                                                     \
+    static constexpr int NW = (S::menc + 3) / 4;                                                         \
+    static constexpr size_t sz_acol = (size_t)NCOL * W * 16;                                             \
+    static constexpr size_t off_mpk = (at);                                                              \
+    static constexpr size_t off_piv = off_mpk + pad16((size_t)S::k * S::o * NW * 4);                     \
+    /* pivot buffer (uint4 items, two of them: step parity): the published pivot column ([w]), the      \
+       pivot row's one-hot words (2 items), the basis multiples of a_p^-1 (1 item; sign_eliminate) */   \
+    static constexpr int PIVQ = W + 3;                                                                   \
+    static_assert(W <= 8, "one-hot words fit in two items");                                             \
+    static constexpr size_t off_rhs = off_piv + (size_t)2 * PIVQ * 16;                                   \
+    static constexpr size_t off_y = off_rhs + (size_t)W * 16;                                            \
+    static constexpr size_t off_key = off_y + pad16(NW * 4);                                             \
+    static constexpr size_t off_t = off_key + pad16(S::digest + 2 * S::sk + 1);                          \
+    static constexpr size_t off_vr = off_t + pad16(NW * 4);                                              \
+    static constexpr size_t off_xs = off_vr + pad16(S::vr);                                              \
+    static constexpr size_t off_flag = off_xs + pad16(S::ko); /* [0] full rank, [1] work counter */      \
+    static constexpr size_t total = off_flag + 16
+
+// The compact CTA of the shared-key path (op_shared.cu): the first attempt from precomputed
+// products only.
+template <int SET_, int NT_>
+struct SignTailCfg {
+    static constexpr int SET = SET_;
     using S = Set<SET>;
-    static constexpr int J = S::k, W = S::W;
-    static constexpr int NT = NT_ ? NT_ : (SET == 5 ? 160 : 128);
-    // engine row slots: J * W * R threads run the engine, so fewer threads get fewer slots
+    static constexpr bool CP = true;
+    static constexpr int J = S::k, W = S::W, NT = NT_, CL = 1;
+    // row slots: J * W * R threads take the rows of the precomputed planes
     static constexpr int R0 = SET == 2 ? 16 : (SET == 1 ? 4 : 2);
     static constexpr int R = NT / (J * W) < R0 ? NT / (J * W) : R0;
-    static constexpr int NCOL = S::ko + 1;  // columns of [A | y]
-    static constexpr int CPT = (NCOL + NT - 1) / NT;
-    static constexpr int NW = (S::menc + 3) / 4;
-    static_assert(J * W * R <= NT, "engine threads");
-    // shared memory (bytes); the bit-plane columns of A reuse the engine staging area
+    static_assert(J * W * R <= NT, "row slots");
     static constexpr size_t off_masks = 0;
-    static constexpr size_t off_bs = off_masks + (size_t)S::v * J * 16;
-    static constexpr size_t sz_bs = COMPACT ? 0 : (size_t)R * S::n * W * 16;
-    static constexpr size_t sz_acol = (size_t)NCOL * W * 16;
-    static constexpr size_t sz_x = (size_t)J * J * W * 16;
-    // With engine staging, the U accumulators reuse it: they are written after the U loop's last
-    // read of the staging area and consumed before the M loop's first write.
-    static constexpr bool X_IN_BS = !COMPACT && sz_bs >= sz_x;
-    static constexpr size_t off_x = X_IN_BS ? off_bs : off_bs + (sz_bs > sz_acol ? sz_bs : sz_acol);
-    static constexpr size_t off_upk = X_IN_BS ? off_bs + (sz_bs > sz_acol ? sz_bs : sz_acol) : off_x + sz_x;
-    static constexpr size_t off_mpk = off_upk + pad16((size_t)S::pairs * NW * 4);
-    static constexpr size_t off_piv = off_mpk + pad16((size_t)S::k * S::o * NW * 4);
-    // pivot buffer (uint4 items, two of them: step parity): the published pivot column ([w]), the
-    // pivot row's one-hot words (2 items), the basis multiples of a_p^-1 (1 item; see sign_eliminate)
-    static constexpr int PIVQ = W + 3;
-    static_assert(W <= 8, "one-hot words fit in two items");
-    static constexpr size_t off_rhs = off_piv + (size_t)2 * PIVQ * 16;
-    static constexpr size_t off_y = off_rhs + (size_t)W * 16;
-    static constexpr size_t off_key = off_y + pad16(NW * 4);
-    static constexpr size_t off_t = off_key + pad16(S::digest + 2 * S::sk + 1);
-    static constexpr size_t off_vr = off_t + pad16(NW * 4);
-    static constexpr size_t off_xs = off_vr + pad16(S::vr);
-    static constexpr size_t off_flag = off_xs + pad16(S::ko);
-    static constexpr size_t total = off_flag + 16;
+    static constexpr size_t off_bs = off_masks + (size_t)S::v * J * 16;  // bit-plane columns of A
+    static constexpr size_t off_x = off_bs + (size_t)(S::ko + 1) * W * 16;
+    static constexpr size_t off_upk = off_x + (size_t)J * J * W * 16;
+    static constexpr size_t off_yext = off_upk + pad16((size_t)S::pairs * ((S::menc + 3) / 4) * 4);
+    MAYO_SIGN_TAIL_LAYOUT(off_yext + 128);
 };
 
-template <int SET>
-struct P1Rows {  // rows r < v of the upper-triangular P1 (sign.cu:402-418)
+// The CTA, or cluster of CL CTAs, of a signature under its own key.  The quads -- MQ of columns of L,
+// then UQ of rows of P1 -- are dealt out to NP parts as in VerifyCfg.
+template <int SET_, int CL_ = 1>
+struct SignCfg {
+    static constexpr int SET = SET_;
     using S = Set<SET>;
-    const uint8_t *P1;
-    __device__ __forceinline__ int count(int r) const { return S::v - r; }
-    __device__ __forceinline__ const uint8_t *entry(int r, int e) const {
-        return P1 + (size_t)tri(r, r + e, S::v) * S::menc;
-    }
-    __device__ __forceinline__ int col(int r, int e) const { return r + e; }
+    static constexpr bool CP = false;
+    static constexpr int J = S::k, W = S::W, NQ = QuadCfg<SET>::NQ, ST = QuadAcc<J>::ST, CL = CL_;
+    static constexpr int MQ = (S::o + 3) / 4, UQ = (S::v + 3) / 4, QN = MQ + UQ;
+    static constexpr int NR = CL > 1 ? 1 : (SET == 3 ? 2 : 1);
+    static constexpr int NP = CL * NR;
+    static constexpr int QL = (QN + NP - 1) / NP;
+    static constexpr int CH = (QL * NQ + 31) / 32;
+    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 3 : SET == 3 ? 4 : 11);
+    static constexpr int NT = 32 * CW;
+    static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;
+    static constexpr int CH2 = (J * NQ + 31) / 32;
+    static constexpr int P2 = CH2 >= CW ? (SET == 5 ? 3 : 1) : (CW + CH2 - 1) / CH2;
+    static constexpr int D = SET == 3 ? 2 : 1;
+    static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 2 ? 6 : SET == 3 ? 2 : 1);
+    // slots of T a part needs: its quads of P1 (a chunk's last lanes write past them)
+    static constexpr int TU = CH * 32;
+    static constexpr size_t off_masks = 0;
+    static constexpr size_t sz_masks = (size_t)S::v * ST * 16;
+    static constexpr size_t sz_mask2 = (size_t)QL * ST * 16, sz_upk = pad16((size_t)S::pairs * NQ * 4);
+    static constexpr size_t off_mask2 = NR == 1 ? 0 : sz_masks;
+    static constexpr size_t off_upk = off_mask2 + sz_mask2;
+    static_assert(NR > 1 || sz_mask2 + sz_upk <= sz_masks, "second-step masks and U fit");
+    // T; afterwards the bit-plane columns of A, then the planes of O and the accumulators of s
+    static constexpr size_t off_bs = NR == 1 ? sz_masks : off_upk + sz_upk;
+    static constexpr size_t cmax(size_t a, size_t b) { return a > b ? a : b; }
+    static constexpr size_t sz_bs =
+        cmax(cmax((size_t)J * TU * 16, (size_t)(S::ko + 1) * W * 16), (size_t)(S::o + S::k) * W * 16);
+    static constexpr size_t off_yext = off_bs + sz_bs;
+    MAYO_SIGN_TAIL_LAYOUT(off_yext + 128);
 };
 
+// Columns of L (units of quads x < MQ) and rows of P1 (the others): off0 is the byte offset of row or
+// column 0's word from the aligned base, r0 the quad's first row of P1 (or < 0 for a quad of L).
 template <int SET>
-struct LColRows {  // "row" b = column b of L: entries L[a][b], a < v (sign.cu:274-319)
+struct SignRows {
     using S = Set<SET>;
-    const uint8_t *L;
-    __device__ __forceinline__ int count(int) const { return S::v; }
-    __device__ __forceinline__ const uint8_t *entry(int b, int a) const {
-        return L + (size_t)(a * S::o + b) * S::menc;
+    uint32_t p1, q4;
+    int x;  // quad
+    int row_l;
+    static constexpr int MQ = (S::o + 3) / 4;
+    __device__ __forceinline__ void start(uint32_t (&bit)[4], int c) const {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int e = x < MQ ? S::e1 + c * S::o + min(4 * x + i, S::o - 1)
+                                 : tri(min(4 * (x - MQ) + i, S::v - 1), c, S::v);
+            bit[i] = 8u * (p1 + (uint32_t)(e * S::menc) + q4);
+        }
     }
-    __device__ __forceinline__ int col(int, int a) const { return a; }
+    __device__ __forceinline__ void next(uint32_t (&bit)[4], int) const {
+        const uint32_t d = 8u * S::menc * (x < MQ ? S::o : 1);
+#pragma unroll
+        for (int i = 0; i < 4; i++) bit[i] += d;
+    }
+    __device__ __forceinline__ bool keep(int i, int c) const { return x < MQ || c >= 4 * (x - MQ) + i; }
+    __device__ __forceinline__ void ahead(const uint32_t *base4, int c) const { row_ahead(base4, p1, row_l, c); }
+    // columns c .. of row r of P1
+    __device__ static __forceinline__ void row_ahead(const uint32_t *base4, uint32_t p1, int r, int c) {
+        if (r >= 0 && r < S::v && c >= r && c < S::v)
+            l2_prefetch(base4, p1 + (uint32_t)(tri(r, c, S::v) * S::menc), (uint32_t)(min(S::v - c, QUAD_AHEAD) * S::menc));
+    }
 };
 
-__device__ __forceinline__ int pair_index_s(int i, int j, int k) { return i * k - (i * (i - 1)) / 2 + (j - i); }
 // Position of pair (a <= b) in the A-assembly order (sign.cu:333-392): i = 0..k-1, j = k-1..i.
 __device__ __forceinline__ int ell_of(int a, int b, int k) { return a * k - (a * (a - 1)) / 2 + (k - 1 - b); }
 
@@ -128,31 +174,30 @@ __device__ __forceinline__ uint32_t zdown_word(const uint32_t *u, int q, int shi
 }
 
 // Shared-memory views of one signing CTA.
-#define MAYO_SIGN_VIEWS                                                                       \
-    using S = Set<SET>;                                                                       \
-    using C = SignCfg<SET, NT_, CP_>;                                                         \
-    constexpr int J = C::J, W = C::W, R = C::R, NT = C::NT, NW = C::NW, KO = S::ko, CPT = C::CPT; \
-    (void)J; (void)R; (void)KO; (void)CPT; (void)NW;
+#define MAYO_SIGN_VIEWS                                                                           \
+    constexpr int SET = C::SET;                                                                   \
+    constexpr bool CP_ = C::CP;                                                                   \
+    using S = Set<SET>;                                                                           \
+    constexpr int J = C::J, W = C::W, NT = C::NT, NW = C::NW, KO = S::ko, CPT = C::CPT;              \
+    (void)J; (void)KO; (void)CPT; (void)NW; (void)CP_;                                            \
+    uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);                                \
+    uint4 *acol = reinterpret_cast<uint4 *>(smem + C::off_bs);        /* [NCOL][W] */             \
+    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);                              \
+    uint32_t *mpk = reinterpret_cast<uint32_t *>(smem + C::off_mpk);  /* [k][o][NW] */            \
+    uint32_t *ypk = reinterpret_cast<uint32_t *>(smem + C::off_y);                                \
+    uint4 *rhsacc = reinterpret_cast<uint4 *>(smem + C::off_rhs);     /* [W] */                   \
+    uint8_t *s_key = smem + C::off_key;  /* digest || salt || seed_sk || ctr */                   \
+    uint8_t *s_t = smem + C::off_t;                                                               \
+    uint8_t *s_vr = smem + C::off_vr;                                                             \
+    uint8_t *s_x = smem + C::off_xs;                                                              \
+    int *s_flag = reinterpret_cast<int *>(smem + C::off_flag);                                    \
+    (void)masks; (void)acol; (void)upk; (void)mpk; (void)ypk; (void)rhsacc; (void)s_key; (void)s_t; (void)s_vr; \
+    (void)s_x; (void)s_flag;
 
 // Plain path: digest, salt, t and V||r(ctr = 0) from the workspace written by sign_hash_kernel.
-template <int SET, int NT_, bool CP_ = false>
+template <class C>
 __device__ __forceinline__ void sign_load_ws(uint8_t *smem, int tid, const uint8_t *esk, const uint8_t *ws) {
     MAYO_SIGN_VIEWS
-    uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
-    uint4 *bs = reinterpret_cast<uint4 *>(smem + C::off_bs);
-    uint4 *acol = reinterpret_cast<uint4 *>(smem + C::off_bs);  // [NCOL][W], after the engine phases
-    uint4 *xacc = reinterpret_cast<uint4 *>(smem + C::off_x);
-    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);
-    uint32_t *mpk = reinterpret_cast<uint32_t *>(smem + C::off_mpk);  // [k][o][NW]
-    uint4 *pivbuf = reinterpret_cast<uint4 *>(smem + C::off_piv);     // [2][PIVQ]
-    uint4 *rhsacc = reinterpret_cast<uint4 *>(smem + C::off_rhs);     // [W]
-    uint32_t *ypk = reinterpret_cast<uint32_t *>(smem + C::off_y);
-    uint8_t *s_key = smem + C::off_key;  // digest || salt || seed_sk || ctr
-    uint8_t *s_t = smem + C::off_t;
-    uint8_t *s_vr = smem + C::off_vr;
-    uint8_t *s_x = smem + C::off_xs;
-    int *s_flag = reinterpret_cast<int *>(smem + C::off_flag);
-    (void)masks; (void)bs; (void)acol; (void)xacc; (void)upk; (void)mpk; (void)pivbuf; (void)rhsacc; (void)ypk; (void)s_key; (void)s_t; (void)s_vr; (void)s_x; (void)s_flag;
     using WS = SignWs<SET>;
     if (CP_) {
         // compact tail: the workspace row is 16-byte aligned and padded to 16 bytes, so it comes
@@ -183,25 +228,10 @@ __device__ __forceinline__ void sign_load_ws(uint8_t *smem, int tid, const uint8
 // Queue path: the CTA hashes itself (warp 0, warp-cooperative Keccak): digest = SHAKE256(M),
 // salt = SHAKE256(digest || 0^SK || seed_sk), t = SHAKE256(digest || salt), V || r for `ctr`
 // (sign.cu:225-252).  All threads must call it.
-template <int SET, int NT_, bool CP_ = false>
+template <class C>
 __device__ __forceinline__ void sign_hash_cta(uint8_t *smem, int tid, const uint8_t *esk, const uint8_t *msg,
                                               uint32_t mlen, int ctr) {
     MAYO_SIGN_VIEWS
-    uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
-    uint4 *bs = reinterpret_cast<uint4 *>(smem + C::off_bs);
-    uint4 *acol = reinterpret_cast<uint4 *>(smem + C::off_bs);  // [NCOL][W], after the engine phases
-    uint4 *xacc = reinterpret_cast<uint4 *>(smem + C::off_x);
-    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);
-    uint32_t *mpk = reinterpret_cast<uint32_t *>(smem + C::off_mpk);  // [k][o][NW]
-    uint4 *pivbuf = reinterpret_cast<uint4 *>(smem + C::off_piv);     // [2][PIVQ]
-    uint4 *rhsacc = reinterpret_cast<uint4 *>(smem + C::off_rhs);     // [W]
-    uint32_t *ypk = reinterpret_cast<uint32_t *>(smem + C::off_y);
-    uint8_t *s_key = smem + C::off_key;  // digest || salt || seed_sk || ctr
-    uint8_t *s_t = smem + C::off_t;
-    uint8_t *s_vr = smem + C::off_vr;
-    uint8_t *s_x = smem + C::off_xs;
-    int *s_flag = reinterpret_cast<int *>(smem + C::off_flag);
-    (void)masks; (void)bs; (void)acol; (void)xacc; (void)upk; (void)mpk; (void)pivbuf; (void)rhsacc; (void)ypk; (void)s_key; (void)s_t; (void)s_vr; (void)s_x; (void)s_flag;
     uint8_t *s_salt = s_x;  // s_x is free until the attempt writes x
     if (tid < 32) {
         const int lane = tid;
@@ -225,24 +255,9 @@ __device__ __forceinline__ void sign_hash_cta(uint8_t *smem, int tid, const uint
 }
 
 // V || r for attempt `ctr` from the digest, salt and seed already in shared memory.
-template <int SET, int NT_, bool CP_ = false>
+template <class C>
 __device__ __forceinline__ void sign_next_vr(uint8_t *smem, int tid, int ctr) {
     MAYO_SIGN_VIEWS
-    uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
-    uint4 *bs = reinterpret_cast<uint4 *>(smem + C::off_bs);
-    uint4 *acol = reinterpret_cast<uint4 *>(smem + C::off_bs);  // [NCOL][W], after the engine phases
-    uint4 *xacc = reinterpret_cast<uint4 *>(smem + C::off_x);
-    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);
-    uint32_t *mpk = reinterpret_cast<uint32_t *>(smem + C::off_mpk);  // [k][o][NW]
-    uint4 *pivbuf = reinterpret_cast<uint4 *>(smem + C::off_piv);     // [2][PIVQ]
-    uint4 *rhsacc = reinterpret_cast<uint4 *>(smem + C::off_rhs);     // [W]
-    uint32_t *ypk = reinterpret_cast<uint32_t *>(smem + C::off_y);
-    uint8_t *s_key = smem + C::off_key;  // digest || salt || seed_sk || ctr
-    uint8_t *s_t = smem + C::off_t;
-    uint8_t *s_vr = smem + C::off_vr;
-    uint8_t *s_x = smem + C::off_xs;
-    int *s_flag = reinterpret_cast<int *>(smem + C::off_flag);
-    (void)masks; (void)bs; (void)acol; (void)xacc; (void)upk; (void)mpk; (void)pivbuf; (void)rhsacc; (void)ypk; (void)s_key; (void)s_t; (void)s_vr; (void)s_x; (void)s_flag;
     if (tid < 32) {
         const int lane = tid;
         WarpKeccak wk;
@@ -254,50 +269,19 @@ __device__ __forceinline__ void sign_next_vr(uint8_t *smem, int tid, int ctr) {
     __syncthreads();
 }
 
-template <int SET, int NT_, bool CP_, int G>
+template <class C, int G>
 __device__ __forceinline__ bool sign_eliminate(uint8_t *smem0, int T);
 
-// One attempt on the V || r in shared memory: x on success, x = r on a singular system.
-// Returns whether the system had full rank.  All threads of the CTA must call it.
-// `pre`, when given, holds this attempt's T_j[r] = P1[r] V_j (rows r < v) and M_j[b] = V_j L[:, b]
-// (rows v + b) as bit-plane groups [j][row][w], computed for a whole batch on the tensor cores
-// (op_shared.cu); the two engine passes over P1 and L are then skipped.
-//
-// G instances per CTA (G * NT threads; instance g's shared memory at smem0 + g * C::total): thread
-// T works on instance T / NT as thread T % NT everywhere except in the elimination, where the
-// instances' columns are interleaved -- thread T owns column KO - T / G of instance T % G -- so
-// the G pivot owners of a step sit in one warp (one publish for G instances) and the live
-// columns of a step fill whole warps.  All control flow and barriers are the same for every
-// instance (nothing depends on the data), so the instances run one shared barrier sequence.
-// With G = 1 smem0 / T are the instance's shared memory / thread index.  `esk` and `pre` are the
-// thread's own instance's (T / NT).  The result is that instance's.
-template <int SET, int NT_, bool CP_ = false, int G = 1>
-__device__ __forceinline__ bool sign_attempt(uint8_t *smem0, int T, const uint8_t *esk, const uint4 *pre = nullptr) {
-    static_assert(G == 1 || G == 2 || G == 4, "instances per CTA");
-    const int tid = G == 1 ? T : T % SignCfg<SET, NT_, CP_>::NT;
-    uint8_t *smem = smem0 + (G == 1 ? 0 : (size_t)(T / SignCfg<SET, NT_, CP_>::NT) * SignCfg<SET, NT_, CP_>::total);
+// U, y and M of one attempt from precomputed products (the shared-key path): `pre` holds
+// T_j[r] = P1[r] V_j (rows r < v) and M_j[b] = V_j L[:, b] (rows v + b) as bit-plane groups
+// [j][row][w], computed for a whole batch on the tensor cores (op_shared.cu).
+template <class C>
+__device__ __forceinline__ void sign_products_pre(uint8_t *smem, int tid, const uint4 *pre) {
     MAYO_SIGN_VIEWS
-    uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
-    uint4 *bs = reinterpret_cast<uint4 *>(smem + C::off_bs);
-    uint4 *acol = reinterpret_cast<uint4 *>(smem + C::off_bs);  // [NCOL][W], after the engine phases
+    constexpr int R = C::R, NROWS = S::v + S::o;
     uint4 *xacc = reinterpret_cast<uint4 *>(smem + C::off_x);
-    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);
-    uint32_t *mpk = reinterpret_cast<uint32_t *>(smem + C::off_mpk);  // [k][o][NW]
-    uint4 *pivbuf = reinterpret_cast<uint4 *>(smem + C::off_piv);     // [2][PIVQ]
-    uint4 *rhsacc = reinterpret_cast<uint4 *>(smem + C::off_rhs);     // [W]
-    uint32_t *ypk = reinterpret_cast<uint32_t *>(smem + C::off_y);
-    uint8_t *s_key = smem + C::off_key;  // digest || salt || seed_sk || ctr
-    uint8_t *s_t = smem + C::off_t;
-    uint8_t *s_vr = smem + C::off_vr;
-    uint8_t *s_x = smem + C::off_xs;
-    int *s_flag = reinterpret_cast<int *>(smem + C::off_flag);
-    (void)masks; (void)bs; (void)acol; (void)xacc; (void)upk; (void)mpk; (void)pivbuf; (void)rhsacc; (void)ypk; (void)s_key; (void)s_t; (void)s_vr; (void)s_x; (void)s_flag;
-    const int lane = tid & 31;
-    (void)lane;
-    const uint8_t *P1 = esk + S::sk + S::o_bytes;
-    const uint8_t *L = P1 + S::p1;
-    Engine<SET, J, R> eng;
-    eng.setup(masks, bs, tid);
+    uint32_t *yext = reinterpret_cast<uint32_t *>(smem + C::off_yext);
+    if (tid < 32) yext[tid] = 0;
     // ---- masks of V: masks[c][i] = V_i[c] ----
     for (int idx = tid; idx < S::v * J; idx += NT) {
         const int c = idx / J, i = idx - c * J;
@@ -305,53 +289,26 @@ __device__ __forceinline__ bool sign_attempt(uint8_t *smem0, int T, const uint8_
         masks[idx] = scalar_masks((s_vr[q >> 1] >> ((q & 1) * 4)) & 0xF);
     }
     __syncthreads();
-
     // ---- U = V^T P1 V: X[i][j] = sum_r V_i[r] T_j[r]; thread (j, w, rs) takes rows rs, rs + R, ... ----
+    const bool active = tid < J * W * R;
+    const int ta = active ? tid : 0, ej = ta % J, ew = (ta / J) % W, rs = ta / (J * W);
     G4 X[J];
 #pragma unroll
     for (int i = 0; i < J; i++) X[i] = g4_zero();
-    if (CP_ || pre) {  // a compact CTA has no engine staging: precomputed products only
-        constexpr int NROWS = S::v + S::o;
-        if (eng.active) {
+    if (active) {
 #pragma unroll 1
-            for (int r = eng.rs; r < S::v; r += R) {
-                const G4 T = g4_ld(pre + ((size_t)eng.j * NROWS + r) * W + eng.w);
-                const uint4 *mr = masks + (size_t)r * J;
+        for (int r = rs; r < S::v; r += R) {
+            const G4 T = g4_ld(pre + ((size_t)ej * NROWS + r) * W + ew);
+            const uint4 *mr = masks + (size_t)r * J;
 #pragma unroll
-                for (int i = 0; i < J; i++) g4_madd(X[i], T, mr[i]);
-            }
-        }
-    } else {
-        const P1Rows<SET> rows{P1};
-#pragma unroll 1
-        for (int r0 = 0; r0 < S::v; r0 += R) {
-            // the next pass's rows of P1, or after the last the first columns of L, into L2:
-            // MAYO_3/5 (MAYO_5 signWithesk 6.96 -> 6.63 ms per 1,024; MAYO_1/2 measured slower)
-            if (SET >= 3 && tid < 32) {
-                if (r0 + R < S::v)
-                    eng.prefetch(rows, r0 + R, S::v, tid);
-                else
-                    eng.prefetch(LColRows<SET>{L}, 0, S::o, tid);
-            }
-            eng.convert(rows, r0, S::v, tid, NT);
-            __syncthreads();
-            const int r = r0 + eng.rs;
-            if (eng.active && r < S::v) {
-                const G4 T = eng.row_product(rows, r);
-                const uint4 *mr = masks + (size_t)r * J;
-#pragma unroll
-                for (int i = 0; i < J; i++) g4_madd(X[i], T, mr[i]);
-            }
-            __syncthreads();
+            for (int i = 0; i < J; i++) g4_madd(X[i], T, mr[i]);
         }
     }
-    // the accumulators may share the engine staging area, whose last read is behind the loop's
-    // final barrier: zero them, then combine the threads' partial sums
     for (int i = tid; i < J * J * W * 4; i += NT) reinterpret_cast<uint32_t *>(xacc)[i] = 0;
     __syncthreads();
-    if (eng.active) {
+    if (active) {
 #pragma unroll
-        for (int i = 0; i < J; i++) g4_atomic_xor(xacc + ((size_t)i * J + eng.j) * W + eng.w, X[i]);
+        for (int i = 0; i < J; i++) g4_atomic_xor(xacc + ((size_t)i * J + ej) * W + ew, X[i]);
     }
     __syncthreads();
     for (int idx = tid; idx < S::pairs * W; idx += NT) {
@@ -366,55 +323,164 @@ __device__ __forceinline__ bool sign_attempt(uint8_t *smem0, int T, const uint8_
         if (i != j) u = g4_xor(u, g4_ld(xacc + ((size_t)j * J + i) * W + ww));
         const uint4 pk = g4_to_packed(u);
         const uint32_t wd[4] = {pk.x, pk.y, pk.z, pk.w};
+        const int l = pair_ell(i, j, J);
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            if (4 * ww + q < NW) upk[pid * NW + 4 * ww + q] = wd[q];
+            if (4 * ww + q < NW) upk[l * NW + 4 * ww + q] = wd[q];
     }
     __syncthreads();
-
-    // ---- y = sum z^l U_l + t (warp 0) while the others compute M = V L ----
-    if (tid < 32) {
-        uint32_t y = 0;
-#pragma unroll 1
-        for (int i = S::k - 1; i >= 0; i--)
-#pragma unroll 1
-            for (int j = i; j < S::k; j++) {
-                y = times_z_lane<SET>(y, lane);
-                if (lane < NW) y ^= upk[pair_index_s(i, j, S::k) * NW + lane];
-            }
-        if (lane < NW) ypk[lane] = y ^ reinterpret_cast<const uint32_t *>(s_t)[lane];
-    }
-    if (CP_ || pre) {  // a compact CTA has no engine staging: precomputed products only
-        constexpr int NROWS = S::v + S::o;
-        for (int idx = tid; idx < J * S::o * W; idx += NT) {
-            const int w = idx % W, jb = idx / W, b = jb % S::o, j = jb / S::o;
-            const uint4 pk = g4_to_packed(g4_ld(pre + ((size_t)j * NROWS + S::v + b) * W + w));
-            const uint32_t wd[4] = {pk.x, pk.y, pk.z, pk.w};
-            uint32_t *dst = mpk + ((size_t)j * S::o + b) * NW;
+    // ---- the unreduced y = sum z^l U_l, and M unpacked ----
+    y_accumulate<SET>(upk, yext, tid >> 5, NT / 32, tid & 31);
+    for (int idx = tid; idx < J * S::o * W; idx += NT) {
+        const int w = idx % W, jb = idx / W, b = jb % S::o, j = jb / S::o;
+        const uint4 pk = g4_to_packed(g4_ld(pre + ((size_t)j * NROWS + S::v + b) * W + w));
+        const uint32_t wd[4] = {pk.x, pk.y, pk.z, pk.w};
+        uint32_t *dst = mpk + ((size_t)j * S::o + b) * NW;
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (4 * w + q < NW) dst[4 * w + q] = wd[q];
+        for (int q = 0; q < 4; q++)
+            if (4 * w + q < NW) dst[4 * w + q] = wd[q];
+    }
+    __syncthreads();
+}
+
+// U, y and M of one attempt from the key (quad.cuh).  In a cluster every CTA works on its part and
+// rank 0 gathers U and M; returns false in the other ranks, which have nothing more to do.
+template <class C>
+__device__ __forceinline__ bool sign_products(uint8_t *smem, int tid, const uint8_t *esk, int rank) {
+    MAYO_SIGN_VIEWS
+    constexpr int NQ = C::NQ, MQ = C::MQ, NP = C::NP, CL = C::CL;
+    uint4 *mask2 = reinterpret_cast<uint4 *>(smem + C::off_mask2);
+    uint4 *T = reinterpret_cast<uint4 *>(smem + C::off_bs);  // [j][unit]
+    uint32_t *yext = reinterpret_cast<uint32_t *>(smem + C::off_yext);
+    const int warp = tid >> 5, lane = tid & 31;
+    auto scalar = [&](int c, int i) {  // V_i[c]
+        const int q = i * S::m + c;
+        return (uint32_t)(s_vr[q >> 1] >> ((q & 1) * 4)) & 0xFu;
+    };
+    const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(esk) & 3);
+    const uint32_t *base4 = reinterpret_cast<const uint32_t *>(esk - mis);
+    const uint32_t p1 = mis + S::sk + S::o_bytes;
+    if constexpr (CL == 1) {
+        for (int r = tid; r < S::v; r += NT) SignRows<SET>::row_ahead(base4, p1, r, r);
+        l2_prefetch_range(base4, p1 + S::p1, S::p2, tid, NT);
+    }
+    if (tid < 32) yext[tid] = 0;
+    if (tid == 0) s_flag[1] = 0;
+    build_masks9<J>(reinterpret_cast<uint32_t *>(masks), S::v, tid, NT, scalar);
+    if constexpr (C::NR > 1) {
+        for (int i = tid; i < S::pairs * NQ; i += NT) upk[i] = 0;
+    }
+    if constexpr (C::PC > 1) {
+        for (int i = tid; i < S::k * S::o * NW; i += NT) mpk[i] = 0;
+    }
+#pragma unroll 1
+    for (int round = 0; round < C::NR; round++) {
+        const int part = CL > 1 ? rank : round;
+        const int tm = part < MQ ? (MQ - part + NP - 1) / NP : 0;  // the part's quads of L come first
+        auto quad_scalar = [&](int t, int i, int j) {              // V_j at row i of the part's t-th quad
+            const int c = 4 * (part + t * NP - MQ) + i;
+            return t >= tm && c < S::v ? scalar(c, j) : 0u;
+        };
+        if constexpr (C::PC > 1) {
+            for (int i = tid; i < J * C::TU; i += NT) T[i] = make_uint4(0, 0, 0, 0);
+        }
+        if constexpr (C::NR > 1) build_quad_masks9<J>(reinterpret_cast<uint32_t *>(mask2), C::QL, tid, NT, quad_scalar);
+        __syncthreads();
+        for (;;) {
+            const int item = warp_next(s_flag + 1, lane);
+            if (item >= C::CH * C::PC) break;
+            const int chunk = item / C::PC, piece = item - chunk * C::PC;
+            const int u = chunk * 32 + lane, t = u / NQ, q = u - t * NQ;
+            const int xmin = part + (chunk * 32 / NQ) * NP, xmax = min(part + ((chunk * 32 + 31) / NQ) * NP, C::QN - 1);
+            const int x = min(part + t * NP, C::QN);  // C::QN: no quad (its rows are dropped below)
+            const int c_lo = xmin < MQ ? 0 : min(4 * (xmin - MQ), S::v), c_chk = xmax < MQ ? 0 : 4 * (xmax - MQ) + 4;
+            const int len = S::v - c_lo;
+            QuadAcc<J> acc;
+            acc.zero();
+            const int tl = chunk * 32 / NQ + (lane >> 2);
+            const SignRows<SET> rows{p1, (uint32_t)(4 * q), x,
+                                     tl <= (chunk * 32 + 31) / NQ ? 4 * (part + tl * NP - MQ) + (lane & 3) : -1};
+            quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), c_lo + len * piece / C::PC,
+                                             c_lo + len * (piece + 1) / C::PC, c_chk, masks);
+            if (x < MQ) {
+#pragma unroll
+                for (int j = 0; j < J; j++) {  // M_j[4 x + i], word q
+                    const G4 f = acc.fold(j);
+                    const G4 v = quad_planes(f.p0, f.p1, f.p2, f.p3);
+                    const uint32_t wd[4] = {v.p0, v.p1, v.p2, v.p3};
+                    const uint32_t lm = q == NQ - 1 ? QuadCfg<SET>::LAST_MASK : 0xFFFFFFFFu;
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (4 * x + i < S::o) {
+                            uint32_t *d = mpk + (j * S::o + 4 * x + i) * NW + q;
+                            if constexpr (C::PC > 1) atomicXor(d, wd[i] & lm);
+                            else *d = wd[i] & lm;
+                        }
+                }
+            } else {
+                const uint32_t rm = quad_row_mask(4 * (x - MQ), S::v);
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    const G4 v = g4_and(acc.fold(j), rm);
+                    if constexpr (C::PC > 1) g4_atomic_xor(T + j * C::TU + u, v);
+                    else g4_st(T + j * C::TU + u, v);
+                }
+            }
         }
         __syncthreads();
-    } else {
-        const LColRows<SET> rows{L};
-#pragma unroll 1
-        for (int b0 = 0; b0 < S::o; b0 += R) {
-            if (SET >= 3 && tid < 32) eng.prefetch(rows, b0 + R, S::o, tid);
-            eng.convert(rows, b0, S::o, tid, NT);
-            __syncthreads();
-            const int b = b0 + eng.rs;
-            if (eng.active && b < S::o) {
-                const G4 T = eng.row_product(rows, b);  // M_j[b], j = eng.j
-                const uint4 pk = g4_to_packed(T);
-                const uint32_t wd[4] = {pk.x, pk.y, pk.z, pk.w};
-                uint32_t *dst = mpk + ((size_t)eng.j * S::o + b) * NW;
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (4 * eng.w + q < NW) dst[4 * eng.w + q] = wd[q];
-            }
+        if (tid == 0) s_flag[1] = 0;
+        if constexpr (C::NR == 1) {
+            build_quad_masks9<J>(reinterpret_cast<uint32_t *>(mask2), C::QL, tid, NT, quad_scalar);
+            for (int i = tid; i < S::pairs * NQ; i += NT) upk[i] = 0;
             __syncthreads();
         }
+        quad_pairs<SET, C>(T, C::TU, mask2, upk, tm, warp, lane);
+        __syncthreads();
+    }
+    if constexpr (CL > 1) {
+        cluster_barrier();
+        if (rank == 0) {
+            for (int i = tid; i < S::pairs * NQ; i += NT) upk[i] = xor_cluster<CL>(upk + i);
+            for (int i = tid; i < S::k * S::o * NW; i += NT) mpk[i] = xor_cluster<CL>(mpk + i);
+        }
+        cluster_barrier();
+        if (rank != 0) return false;
+    }
+    y_accumulate<SET>(upk, yext, warp, C::CW, lane);
+    __syncthreads();
+    return true;
+}
+
+// One attempt on the V || r in shared memory: x on success, x = r on a singular system.
+// Returns whether the system had full rank.  All threads of the CTA must call it.
+// In a cluster (rank = this CTA's) every rank takes part in the key's products and rank 0 in the
+// rest; the other ranks return at once, with no result.
+//
+// G instances per CTA (compact CTAs only) (G * NT threads; instance g's shared memory at smem0 + g * C::total): thread
+// T works on instance T / NT as thread T % NT everywhere except in the elimination, where the
+// instances' columns are interleaved -- thread T owns column KO - T / G of instance T % G -- so
+// the G pivot owners of a step sit in one warp (one publish for G instances) and the live
+// columns of a step fill whole warps.  All control flow and barriers are the same for every
+// instance (nothing depends on the data), so the instances run one shared barrier sequence.
+// With G = 1 smem0 / T are the instance's shared memory / thread index.  `esk` and `pre` are the
+// thread's own instance's (T / NT).  The result is that instance's.
+template <class C, int G = 1>
+__device__ __forceinline__ bool sign_attempt(uint8_t *smem0, int T, const uint8_t *esk, const uint4 *pre = nullptr,
+                                             int rank = 0) {
+    static_assert(G == 1 || G == 2 || G == 4, "instances per CTA");
+    const int tid = G == 1 ? T : T % C::NT;
+    uint8_t *smem = smem0 + (G == 1 ? 0 : (size_t)(T / C::NT) * C::total);
+    MAYO_SIGN_VIEWS
+    if constexpr (C::CP) sign_products_pre<C>(smem, tid, pre);
+    else if (!sign_products<C>(smem, tid, esk, rank)) return false;  // a rank other than 0: the caller asks rank 0
+
+    // ---- y, by the warp whose thread takes the right-hand side below ----
+    static_assert(KO < NT, "the right-hand side has a thread in the first pass over the columns");
+    if ((tid >> 5) == KO / 32) {
+        const int lane = tid & 31;
+        const uint32_t y = y_fold<SET>(reinterpret_cast<const uint32_t *>(smem + C::off_yext), lane);
+        if (lane < NW) ypk[lane] = y ^ reinterpret_cast<const uint32_t *>(s_t)[lane];
+        __syncwarp();
     }
 
     // ---- A columns (i, b) = sum_j z^{l(i,j)} M_j[b] with one fold by f(z); RHS column = y ----
@@ -505,7 +571,7 @@ __device__ __forceinline__ bool sign_attempt(uint8_t *smem0, int T, const uint8_
     }
     for (int i = tid; i < W * 4; i += NT) reinterpret_cast<uint32_t *>(rhsacc)[i] = 0;
     __syncthreads();
-    const bool ok_mine = sign_eliminate<SET, NT_, CP_, G>(smem0, T);
+    const bool ok_mine = sign_eliminate<C, G>(smem0, T);
     (void)ok_mine;
     return reinterpret_cast<const int *>(smem + C::off_flag)[0] != 0;
 }
@@ -513,11 +579,12 @@ __device__ __forceinline__ bool sign_attempt(uint8_t *smem0, int T, const uint8_
 // The elimination of sign_attempt (sample_solution, src/sign.cu:10-145) for the G instances of a
 // CTA: [A | y] (bit-plane columns in each instance's acol area), r from V || r; writes x and the
 // rank flag of every instance.  Returns the flag of the instance whose column this thread owns.
-template <int SET, int NT_, bool CP_, int G>
+template <class C, int G>
 __device__ __forceinline__ bool sign_eliminate(uint8_t *smem0, int T) {
+    constexpr int SET = C::SET;
     using S = Set<SET>;
-    using C = SignCfg<SET, NT_, CP_>;
     constexpr int W = C::W, NT = C::NT, KO = S::ko, CPT = C::CPT;
+    (void)SET;
     // interleaved columns: thread T takes column rank u = T / G of instance T % G
     const int tid = G == 1 ? T : T / G;
     uint8_t *smem = smem0 + (G == 1 ? 0 : (size_t)(T % G) * C::total);
@@ -584,7 +651,7 @@ __device__ __forceinline__ bool sign_eliminate(uint8_t *smem0, int T) {
     //     D = a + e_p at [0, W) and the basis multiples B_s = a_p^-1 x^s at [W + 2]; a column forms
     //     e / a_p = sum_s e_s B_s by masks.  The owner's extra scalar product of the first form made
     //     these paths ~1 % slower.
-    constexpr bool PREDIV = CP_;
+    constexpr bool PREDIV = C::CP;
     auto publish = [&](int q, int pcx) {
         uint4 *buf = pivbuf + (pcx & 1) * C::PIVQ;
         uint32_t *ohw = reinterpret_cast<uint32_t *>(buf + W);  // oh[0..W)
@@ -743,25 +810,10 @@ __device__ __forceinline__ G4 o_plane_item(const uint8_t *O_g, int idx) {
 
 // s = V + O x, then salt (sign.cu:147-191, 474-477).  `opl`, when given, holds the O planes
 // (o x W items of o_plane_item) precomputed for the key.
-template <int SET, int NT_, bool CP_ = false>
+template <class C>
 __device__ __forceinline__ void sign_write(uint8_t *smem, int tid, const uint8_t *esk, uint8_t *sig,
                                            const uint4 *opl = nullptr) {
     MAYO_SIGN_VIEWS
-    uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
-    uint4 *bs = reinterpret_cast<uint4 *>(smem + C::off_bs);
-    uint4 *acol = reinterpret_cast<uint4 *>(smem + C::off_bs);  // [NCOL][W], after the engine phases
-    uint4 *xacc = reinterpret_cast<uint4 *>(smem + C::off_x);
-    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);
-    uint32_t *mpk = reinterpret_cast<uint32_t *>(smem + C::off_mpk);  // [k][o][NW]
-    uint4 *pivbuf = reinterpret_cast<uint4 *>(smem + C::off_piv);     // [2][PIVQ]
-    uint4 *rhsacc = reinterpret_cast<uint4 *>(smem + C::off_rhs);     // [W]
-    uint32_t *ypk = reinterpret_cast<uint32_t *>(smem + C::off_y);
-    uint8_t *s_key = smem + C::off_key;  // digest || salt || seed_sk || ctr
-    uint8_t *s_t = smem + C::off_t;
-    uint8_t *s_vr = smem + C::off_vr;
-    uint8_t *s_x = smem + C::off_xs;
-    int *s_flag = reinterpret_cast<int *>(smem + C::off_flag);
-    (void)masks; (void)bs; (void)acol; (void)xacc; (void)upk; (void)mpk; (void)pivbuf; (void)rhsacc; (void)ypk; (void)s_key; (void)s_t; (void)s_vr; (void)s_x; (void)s_flag;
     // s_i = V_i + O x_i on bit planes: the columns of O as planes and the k x W accumulators in
     // the engine staging area (free after the attempt); each accumulator (i, w) takes its o
     // multiply-accumulates from SPL threads (shared-memory XOR to combine); nibbles are staged
@@ -770,7 +822,7 @@ __device__ __forceinline__ void sign_write(uint8_t *smem, int tid, const uint8_t
     uint4 *ocol = reinterpret_cast<uint4 *>(smem + C::off_bs);  // [o][W]
     uint4 *sacc = ocol + S::o * W;                                 // [k][W]
     uint8_t *snib = smem + C::off_masks;                           // [k * n]
-    static_assert((size_t)(S::o + S::k) * W * 16 <= (C::sz_bs > C::sz_acol ? C::sz_bs : C::sz_acol),
+    static_assert(C::CP ? (size_t)(S::o + S::k) * W * 16 <= C::sz_acol : true,
                   "O planes and s accumulators fit");
     static_assert((size_t)S::k * S::n <= (size_t)S::v * J * 16, "nibble staging fits");
     if (opl) {

@@ -1,207 +1,175 @@
-// verify_body.cuh -- one MAYO verify on one CTA (reference src/verify.cu:9-212), shared by the
-// batched verify kernel and the persistent work-queue kernel.
+// verify_body.cuh -- one MAYO verify (reference src/verify.cu:9-212) on one CTA, or on a cluster of
+// CTAs where a batch is too small to fill the GPU; shared by the batched verify kernels and the
+// persistent work-queue kernel.
 //
-// Threads 0..NC-1 evaluate U_ij = s_i^T P s_j (+ symmetric term) over the expanded public key
-// P = [[P1, P2], [0, P3]] with the bit-sliced engine; threads NC..NC+31 (one warp) hash
-// digest = SHAKE256(M) and t = SHAKE256(digest || salt) with the warp-cooperative Keccak at the
-// same time.  Warp 0 then runs the Horner sum y = sum z^l U_l and compares it with t.
+// U_ij = s_i^T P s_j (+ symmetric term) over the expanded public key P = [[P1, P2], [0, P3]] in two
+// steps of the same product (quad.cuh): T_j[r] = sum_c P[r][c] s_j[c] for the key's quads of rows,
+// then X_ij = sum_r s_i[r] T_j[r] over the quads, both with warps that take chunks of 32 units
+// from a counter.  Warp 0 first hashes digest = SHAKE256(M) and t = SHAKE256(digest || salt).
+// y = sum z^l U_l is then collected by all warps and compared with t.
 #pragma once
 
 #include "engine.cuh"
 #include "launch_util.cuh"
+#include "quad.cuh"
 
 namespace mayo {
 
-// NC = compute threads (a multiple of 32); the CTA has NC + 32 threads.
-template <int SET, int NC_ = 0>
+template <int SET, int CL = 1>
 struct VerifyCfg {
     using S = Set<SET>;
-    static constexpr int J = S::k, W = S::W;
-    static constexpr int R_DEF = SET == 2 ? 16 : (SET == 1 ? 4 : 2);
-    static constexpr int NC = NC_ ? NC_ : (J * W * R_DEF + 31) / 32 * 32;
-    static constexpr int R = NC / (J * W) < R_DEF ? NC / (J * W) : R_DEF;  // row slots that fit
-    static constexpr int NT = NC + 32;
-    static constexpr int NW = (S::menc + 3) / 4;  // packed words per m-vector
-    static_assert(R >= 1 && J * W * R <= NC, "engine threads");
+    using A = QuadAcc<S::k>;
+    static constexpr int J = S::k, NQ = QuadCfg<SET>::NQ, ST = A::ST;
+    static constexpr int QN = (S::n + 3) / 4;  // quads of rows
+    // The quads are dealt out to NP parts, quad Q to part Q % NP (so each part has long and short
+    // rows): one part per CTA of a cluster, or NR parts one after the other on one CTA (MAYO_3: the
+    // T of half its quads and the masks then leave room for two CTAs per SM).
+    static constexpr int NR = CL > 1 ? 1 : (SET == 3 ? 2 : 1);
+    static constexpr int NP = CL * NR;
+    static constexpr int QL = (QN + NP - 1) / NP;
+    static constexpr int UL = QL * NQ;               // units of a part
+    static constexpr int CH = (UL + 31) / 32;        // chunks of 32 units
+    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 3 : SET == 3 ? 4 : 11);  // warps
+    static constexpr int NT = 32 * CW;
+    // column ranges per chunk (more items than warps where a cluster leaves few chunks per CTA)
+    static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;
+    static constexpr int CH2 = (J * NQ + 31) / 32;   // chunks of (j, word) pairs
+    static constexpr int P2 = CH2 >= CW ? (SET == 5 ? 3 : 1) : (CW + CH2 - 1) / CH2;  // quad ranges of each
+    // columns loaded ahead: two where two CTAs per SM leave the registers (MAYO_3 0.467 -> 0.427 us
+    // per instance); MAYO_1 at three CTAs of 168 registers is slower with two (0.153 -> 0.180)
+    static constexpr int D = SET == 3 ? 2 : 1;
+    static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 2 ? 6 : SET == 3 ? 2 : 1);
     static constexpr size_t off_masks = 0;
-    static constexpr size_t off_bs = off_masks + (size_t)S::n * J * 16;
-    // the U accumulators, then U's packed words, reuse the key-row staging area once the row
-    // loop is done (in place after it when they do not fit)
-    static constexpr size_t off_x = off_bs;
-    static constexpr size_t sz_bs = (size_t)R * S::n * W * 16, sz_x = (size_t)J * J * W * 16;
-    static constexpr size_t sz_upk = pad16((size_t)S::pairs * NW * 4);
-    static constexpr bool UPK_IN_BS = sz_x + sz_upk <= sz_bs;
-    static constexpr size_t off_upk = UPK_IN_BS ? off_bs + sz_x : off_bs + (sz_bs > sz_x ? sz_bs : sz_x);
-    static constexpr size_t off_sig = UPK_IN_BS ? off_bs + sz_bs : off_upk + sz_upk;
+    static constexpr size_t sz_masks = (size_t)S::n * ST * 16;
+    static constexpr size_t sz_mask2 = (size_t)QL * ST * 16, sz_upk = pad16((size_t)S::pairs * NQ * 4);
+    // the second step's masks and U take the first one's masks' place, except between rounds
+    static constexpr size_t off_mask2 = NR == 1 ? 0 : sz_masks;
+    static constexpr size_t off_upk = off_mask2 + sz_mask2;
+    static_assert(NR > 1 || sz_mask2 + sz_upk <= sz_masks, "second-step masks and U fit");
+    static constexpr size_t off_T = NR == 1 ? sz_masks : off_upk + sz_upk;
+    static constexpr size_t off_yext = off_T + (size_t)J * CH * 32 * 16;
+    static constexpr size_t off_sig = off_yext + 128;
     static constexpr size_t off_key = off_sig + pad16(S::sig);
     static constexpr size_t off_t = off_key + pad16(S::digest + S::sk);
-    static constexpr size_t total = off_t + pad16(NW * 4);
+    static constexpr size_t off_ctr = off_t + pad16(NQ * 4);
+    static constexpr size_t total = off_ctr + 16;
 };
 
-template <int SET>
-struct VerifyRows {
-    using S = Set<SET>;
-    const uint8_t *P1, *P2, *P3;
-    __device__ __forceinline__ int count(int r) const { return r < S::v ? (S::v - r) + S::o : S::n - r; }
-    __device__ __forceinline__ const uint8_t *entry(int r, int e) const {
-        if (r < S::v) {
-            const int n1 = S::v - r;
-            return e < n1 ? P1 + (size_t)tri(r, r + e, S::v) * S::menc : P2 + (size_t)(r * S::o + (e - n1)) * S::menc;
-        }
-        const int rr = r - S::v;
-        return P3 + (size_t)tri(rr, rr + e, S::o) * S::menc;
-    }
-    __device__ __forceinline__ int col(int r, int e) const { return r + e; }
-    // Ask L2 for row r's entries, one warp issuing (lane = 0..31): rows of P1 || P2 and of P3 are
-    // contiguous runs of m-vectors, so one prefetch per 128-byte line of each run.
-    __device__ __forceinline__ void prefetch(int r, int lane) const {
-        if (r < S::v) {
-            prefetch_lines(P1 + (size_t)tri(r, r, S::v) * S::menc, (S::v - r) * S::menc, lane);
-            prefetch_lines(P2 + (size_t)r * S::o * S::menc, S::o * S::menc, lane);
-        } else if (r < S::n) {
-            const int rr = r - S::v;
-            prefetch_lines(P3 + (size_t)tri(rr, rr, S::o) * S::menc, (S::o - rr) * S::menc, lane);
-        }
-    }
-    // every address issued lies in [p, p + n): the first is p, the others start 128-byte lines
-    __device__ __forceinline__ static void prefetch_lines(const uint8_t *p, int n, int lane) {
-        const uintptr_t a = reinterpret_cast<uintptr_t>(p), end = a + (uintptr_t)n;
-        for (uintptr_t l = (a & ~uintptr_t(127)) + 128u * (uintptr_t)lane; l < end; l += 128u * 32u) {
-            const uintptr_t q = l < a ? a : l;
-            asm volatile("prefetch.L2 [%0];" ::"l"(q));
-        }
-    }
-};
-
-__device__ __forceinline__ int pair_index(int i, int j, int k) { return i * k - (i * (i - 1)) / 2 + (j - i); }
-
-// Verify one instance; every thread of the CTA (NC + 32 of them) must call it.  Writes 0
-// (accept) or 1 (reject) to *res.  `smem` holds VerifyCfg<SET, NC>::total bytes.
-// `pre`, when given, holds T_j[r] = P[r] s_j for every row r < n as bit-plane groups [j][r][w],
-// computed for a whole batch on the tensor cores (op_shared.cu); the engine pass over the public
-// key is then skipped.
-template <int SET, int NC_>
+// Verify one instance; every thread of the CTA (VerifyCfg::NT of them), or of every CTA of the
+// cluster (rank = this CTA's), must call it.  Writes 0 (accept) or 1 (reject) to *res.  `smem` holds
+// VerifyCfg<SET, CL>::total bytes, at the same address in every CTA of a cluster.
+template <int SET, int CL = 1>
 __device__ __forceinline__ void verify_instance(uint8_t *smem, int tid, const uint8_t *epk, const uint8_t *msg,
-                                                uint32_t mlen, const uint8_t *sig, uint8_t *res,
-                                                const uint4 *pre = nullptr) {
+                                                uint32_t mlen, const uint8_t *sig, uint8_t *res, int rank = 0) {
     using S = Set<SET>;
-    using C = VerifyCfg<SET, NC_>;
-    constexpr int J = C::J, W = C::W, R = C::R, NC = C::NC, NW = C::NW;
+    using C = VerifyCfg<SET, CL>;
+    constexpr int J = C::J, NQ = C::NQ, NT = C::NT, CW = C::CW, ULP = C::CH * 32;
     uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
-    uint4 *bs = reinterpret_cast<uint4 *>(smem + C::off_bs);
-    uint4 *xacc = reinterpret_cast<uint4 *>(smem + C::off_x);
-    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);
+    uint4 *mask2 = reinterpret_cast<uint4 *>(smem + C::off_mask2);
+    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);  // [l][NQ]
+    uint4 *T = reinterpret_cast<uint4 *>(smem + C::off_T);            // [j][unit]
+    uint32_t *yext = reinterpret_cast<uint32_t *>(smem + C::off_yext);
     uint8_t *s_sig = smem + C::off_sig;
     uint8_t *s_key = smem + C::off_key;
     uint8_t *s_t = smem + C::off_t;
+    int *s_next = reinterpret_cast<int *>(smem + C::off_ctr);
+    const int warp = tid >> 5, lane = tid & 31;
 
-    for (int i = tid; i < S::sig; i += C::NT) s_sig[i] = sig[i];
-    for (int i = tid; i < NW * 4; i += C::NT) s_t[i] = 0;
+    for (int i = tid; i < S::sig; i += NT) s_sig[i] = sig[i];
+    for (int i = tid; i < NQ * 4; i += NT) s_t[i] = 0;
+    if (tid < 32) yext[tid] = 0;
+    if (tid == 0) *s_next = 0;
     __syncthreads();
 
-    if (tid >= NC) {
-        // ---- hashing warp: digest and target t (src/verify.cu:37-48) ----
-        const int lane = tid - NC;
-        WarpKeccak wk;
-        wk.setup(lane);
-        warp_shake<136>(s_key, S::digest, msg, (int)mlen, wk, lane);
-        for (int i = lane; i < S::sk; i += 32) s_key[S::digest + i] = s_sig[S::k * S::n / 2 + i];
-        __syncwarp();
-        warp_shake<136>(s_t, S::menc, s_key, S::digest + S::sk, wk, lane);
-    } else {
-        // ---- masks of the signature scalars: column c of s_j (src/verify.cu:62-70) ----
-        for (int idx = tid; idx < S::n * J; idx += NC) {
-            const int c = idx / J, jj = idx - c * J;
-            const int q = jj * S::n + c;
-            const uint32_t nib = (s_sig[q >> 1] >> ((q & 1) * 4)) & 0xF;
-            masks[idx] = scalar_masks(nib);
-        }
-        bar_sync(1, NC);
-
-        // MAYO_3's verify is held to 80 registers for 6 CTAs per SM: the four-partial-sum row
-        // product spills there (1.48 M against 1.51 M distinct-key verify/s), so it keeps g4_madd
-        Engine<SET, J, R, SET != 3> eng;
-        eng.setup(masks, bs, tid);
-        const VerifyRows<SET> rows{epk, epk + S::p1, epk + S::p};
-        G4 X[J];
-#pragma unroll
-        for (int i = 0; i < J; i++) X[i] = g4_zero();
-        if (pre) {
-            if (eng.active) {
-#pragma unroll 1
-                for (int r = eng.rs; r < S::n; r += R) {
-                    const G4 T = g4_ld(pre + ((size_t)eng.j * S::n + r) * W + eng.w);
-                    const uint4 *mr = masks + (size_t)r * J;
-#pragma unroll
-                    for (int i = 0; i < J; i++) g4_madd(X[i], T, mr[i]);
-                }
-            }
-        } else {
-#pragma unroll 1
-            for (int r0 = 0; r0 < S::n; r0 += R) {
-                // the next pass's key rows into L2, per entry (MAYO_1/5: distinct-key verify of
-                // MAYO_5 0.745 -> 0.780 M/s, MAYO_1 verifyWithepk 1 % faster) or per 128-byte line of
-                // each row's runs (MAYO_3, whose kernel is held to 80 registers: verifyWithepk 3 %
-                // faster); MAYO_2's measured 3 % slower with either
-                if (tid < 32) {
-                    if constexpr (SET == 1 || SET == 5) eng.prefetch(rows, r0 + R, S::n, tid);
-                    if constexpr (SET == 3)
-#pragma unroll 1
-                        for (int q = 0; q < R; q++) rows.prefetch(r0 + R + q, tid);
-                }
-                eng.convert(rows, r0, S::n, tid, NC);
-                bar_sync(1, NC);
-                const int r = r0 + eng.rs;
-                if (eng.active && r < S::n) {
-                    const G4 T = eng.row_product(rows, r);
-                    const uint4 *mr = masks + (size_t)r * J;
-#pragma unroll
-                    for (int i = 0; i < J; i++) g4_madd(X[i], T, mr[i]);
-                }
-                bar_sync(1, NC);
-            }
-        }
-        // the staging area is free now (the last row pass ended with a barrier): zero the
-        // accumulators there, then combine the threads' partial sums
-        for (int i = tid; i < J * J * W * 4; i += NC) reinterpret_cast<uint32_t *>(xacc)[i] = 0;
-        bar_sync(1, NC);
-        if (eng.active) {
-#pragma unroll
-            for (int i = 0; i < J; i++) g4_atomic_xor(xacc + ((size_t)i * J + eng.j) * W + eng.w, X[i]);
-        }
-        bar_sync(1, NC);
-        // ---- U_ij (i <= j) to packed words ----
-        for (int idx = tid; idx < S::pairs * W; idx += NC) {
-            const int pid = idx / W, ww = idx - pid * W;
-            int i = 0, rem = pid;
-            while (rem >= J - i) {
-                rem -= J - i;
-                i++;
-            }
-            const int j = i + rem;
-            G4 u = g4_ld(xacc + ((size_t)i * J + j) * W + ww);
-            if (i != j) u = g4_xor(u, g4_ld(xacc + ((size_t)j * J + i) * W + ww));
-            const uint4 pk = g4_to_packed(u);
-            const uint32_t wd[4] = {pk.x, pk.y, pk.z, pk.w};
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (4 * ww + q < NW) upk[pid * NW + 4 * ww + q] = wd[q];
-        }
+    // scalar c of s_j (src/verify.cu:62-70)
+    auto scalar = [&](int c, int j) {
+        const int q = j * S::n + c;
+        return (uint32_t)(s_sig[q >> 1] >> ((q & 1) * 4)) & 0xFu;
+    };
+    build_masks9<J>(reinterpret_cast<uint32_t *>(masks), S::n, tid, NT, scalar);
+    if constexpr (C::NR > 1) {
+        for (int i = tid; i < S::pairs * NQ; i += NT) upk[i] = 0;
     }
-    __syncthreads();
+    const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(epk) & 3);
+    const uint32_t *base4 = reinterpret_cast<const uint32_t *>(epk - mis);
+    if constexpr (CL == 1) {  // every row's first columns of P1, then P2 and P3, while the masks are built
+        for (int r = tid; r < S::v; r += NT) PubRows<SET>::row_ahead(base4, mis, r, r);
+        l2_prefetch_range(base4, mis + S::p1, S::epk - S::p1, tid, NT);
+    }
 
-    // ---- y = Horner over the pairs (i = k-1..0, j = i..k-1), compare with t (src/verify.cu:185-211) ----
-    if (tid < 32) {
-        const int lane = tid;
-        uint32_t y = 0;
 #pragma unroll 1
-        for (int i = S::k - 1; i >= 0; i--)
+    for (int round = 0; round < C::NR; round++) {
+        const int part = CL > 1 ? rank : round;
+        auto quad_scalar = [&](int t, int i, int j) {
+            const int c = 4 * (part + t * C::NP) + i;
+            return c < S::n ? scalar(c, j) : 0u;
+        };
+        if constexpr (C::PC > 1) {
+            for (int i = tid; i < J * ULP; i += NT) T[i] = make_uint4(0, 0, 0, 0);
+        }
+        if constexpr (C::NR > 1)
+            build_quad_masks9<J>(reinterpret_cast<uint32_t *>(mask2), C::QL, tid, NT, quad_scalar);
+        __syncthreads();
+        if (round == 0 && rank == 0 && warp == 0) {  // digest and target t (src/verify.cu:37-48)
+            WarpKeccak wk;
+            wk.setup(lane);
+            warp_shake<136>(s_key, S::digest, msg, (int)mlen, wk, lane);
+            for (int i = lane; i < S::sk; i += 32) s_key[S::digest + i] = s_sig[S::k * S::n / 2 + i];
+            __syncwarp();
+            warp_shake<136>(s_t, S::menc, s_key, S::digest + S::sk, wk, lane);
+        }
+        // ---- T_j[r] = sum_c P[r][c] s_j[c]: chunks of 32 units, the longest first ----
+        for (;;) {
+            const int item = warp_next(s_next, lane);
+            if (item >= C::CH * C::PC) break;
+            const int chunk = item / C::PC, piece = item - chunk * C::PC;
+            const int u = chunk * 32 + lane, t = u / NQ, q = u - t * NQ;
+            const int r0 = 4 * (part + t * C::NP);
+            const int qmin = part + (chunk * 32 / NQ) * C::NP, qmax = part + ((chunk * 32 + 31) / NQ) * C::NP;
+            const int c_lo = min(4 * qmin, S::n), c_chk = 4 * min(qmax, C::QN - 1) + 4;
+            const int len = S::n - c_lo;
+            QuadAcc<J> acc;
+            acc.zero();
+            const int tl = chunk * 32 / NQ + (lane >> 2);
+            const PubRows<SET> rows{mis, (uint32_t)(4 * q), r0,
+                                    tl <= (chunk * 32 + 31) / NQ ? 4 * (part + tl * C::NP) + (lane & 3) : S::n};
+            const int ca = c_lo + len * piece / C::PC, cb = c_lo + len * (piece + 1) / C::PC;
 #pragma unroll 1
-            for (int j = i; j < S::k; j++) {
-                y = times_z_lane<SET>(y, lane);
-                if (lane < NW) y ^= upk[pair_index(i, j, S::k) * NW + lane];
+            for (int seg = 0; seg < 2; seg++)  // P1's columns, then P2's and P3's
+                quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? max(ca, S::v) : ca,
+                                           seg ? cb : min(cb, S::v), c_chk, masks);
+            const uint32_t rm = quad_row_mask(r0, S::n);
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                const G4 v = g4_and(acc.fold(j), rm);
+                if constexpr (C::PC > 1) g4_atomic_xor(T + j * ULP + u, v);
+                else g4_st(T + j * ULP + u, v);
             }
-        const uint32_t tw = lane < NW ? reinterpret_cast<const uint32_t *>(s_t)[lane] : 0u;
+        }
+        __syncthreads();
+        if (tid == 0) *s_next = 0;
+        if constexpr (C::NR == 1) {
+            build_quad_masks9<J>(reinterpret_cast<uint32_t *>(mask2), C::QL, tid, NT, quad_scalar);
+            for (int i = tid; i < S::pairs * NQ; i += NT) upk[i] = 0;
+            __syncthreads();
+        }
+        // ---- X_ij = sum_r s_i[r] T_j[r], packed into U_l ----
+        quad_pairs<SET, C>(T, ULP, mask2, upk, 0, warp, lane);
+        __syncthreads();
+    }
+    if constexpr (CL > 1) {  // the ranks' parts of U meet in rank 0
+        cluster_barrier();
+        if (rank == 0) {
+            for (int i = tid; i < S::pairs * NQ; i += NT) upk[i] = xor_cluster<CL>(upk + i);
+        }
+        cluster_barrier();  // no CTA leaves while rank 0 reads its shared memory
+        if (rank != 0) return;
+    }
+    y_accumulate<SET>(upk, yext, warp, CW, lane);
+    __syncthreads();
+    if (warp == 0) {  // compare y with t (src/verify.cu:185-211)
+        const uint32_t y = y_fold<SET>(yext, lane);
+        const uint32_t tw = lane < NQ ? reinterpret_cast<const uint32_t *>(s_t)[lane] : 0u;
         const bool eq = __all_sync(0xffffffffu, y == tw);
         if (lane == 0) *res = eq ? 0 : 1;
     }

@@ -1,0 +1,68 @@
+"""Per-instance sign and verify at the edges of their launch rule (one CTA per instance, or a
+cluster of two, four or eight where the batch is small), with keys at every alignment, against the
+oracle byte for byte.  Instance 0 signs a message whose first attempt is singular."""
+import hashlib
+import json
+import os
+
+import numpy as np
+import pytest
+
+from cumayo_b200 import Mayo
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+GOLDEN = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden")
+N = 73
+BATCHES = (1, 12, 13, 32, 33, 72, 73)
+
+
+@pytest.fixture(scope="module", params=[1, 2, 3, 5])
+def case(request, cuda):
+    s = request.param
+    rng = np.random.default_rng(700 + s)
+    z = Mayo(s).sizes
+    seeds = rng.integers(0, 256, (N, z.sk_bytes), dtype=np.uint8)
+    sk0, _ = O.keypair(s, 0, 0)
+    seeds[0] = np.frombuffer(sk0, np.uint8)
+    esk = O.expandsk_batch(s, seeds)
+    epk = O.expandpk_batch(s, O.keypair_from_seed_batch(s, seeds))
+    g = json.load(open(os.path.join(GOLDEN, f"ref_mayo{s}.json")))["rejection"]
+    msgs = [rng.integers(0, 256, 32, dtype=np.uint8).tobytes() for _ in range(N)]
+    msgs[0] = hashlib.shake_256(f"reject-search/{s}/{g['indices'][0]}".encode()).digest(32)
+    sig, attempts = O.sign_batch(s, esk, msgs)
+    assert attempts[0] > 0
+    return s, esk, epk, np.frombuffer(b"".join(msgs), np.uint8).reshape(N, 32), sig
+
+
+def _rows(a, stride, off):
+    """Rows of `a` at `stride` bytes from byte `off` of a device buffer that ends with the last row."""
+    import torch
+    host = np.zeros(off + (len(a) - 1) * stride + a.shape[1], np.uint8)
+    for i, r in enumerate(a):
+        host[off + i * stride: off + i * stride + a.shape[1]] = r
+    return torch.from_numpy(host).cuda()[off:]
+
+
+@pytest.mark.parametrize("off", [0, 1, 2, 3])
+def test_sign_verify_launch_edges(case, off):
+    import torch
+    s, esk, epk, msgs, sig = case
+    m = Mayo(s)
+    z = m.sizes
+    es, ps = z.esk_bytes + 3 * off, z.epk_bytes + off
+    d_esk, d_epk, d_msg = _rows(esk, es, off), _rows(epk, ps, off), torch.from_numpy(msgs.copy()).cuda()
+    bad = sig.copy()
+    bad[1::3, 5] ^= 0x10
+    d_bad = torch.from_numpy(bad).cuda()
+    want = np.zeros(N, np.uint8)
+    want[1::3] = 1
+    ws = torch.zeros(N * m.sign_ws_bytes(), dtype=torch.uint8, device="cuda")
+    for b in BATCHES if off == 0 else (1, 13, 73):
+        out = torch.zeros(N, z.sig_bytes, dtype=torch.uint8, device="cuda")
+        m.sign_many(d_esk, d_msg, out, ws, b, msg_stride=32, mlen=32, esk_stride=es)
+        res = torch.full((N,), 0xEE, dtype=torch.uint8, device="cuda")
+        m.verify_many(d_epk, d_msg, d_bad, res, b, msg_stride=32, mlen=32, epk_stride=ps)
+        torch.cuda.synchronize()
+        assert (out[:b].cpu().numpy() == sig[:b]).all() and not out[b:].any(), b
+        assert (res[:b].cpu().numpy() == want[:b]).all() and (res[b:] == 0xEE).all(), b
