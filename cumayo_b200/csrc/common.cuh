@@ -76,18 +76,6 @@ __host__ __device__ __forceinline__ uint32_t lop_xand(uint32_t a, uint32_t b, ui
 #endif
 }
 
-// 4-byte little-endian load from an arbitrary byte address; bytes p..p+3 must be valid.
-// Uses aligned word loads only, so it never touches a word without a valid byte.
-__device__ __forceinline__ uint32_t ld_le32(const uint8_t *p) {
-    uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const uint32_t *q = reinterpret_cast<const uint32_t *>(a & ~uintptr_t(3));
-    uint32_t sh = (uint32_t)(a & 3) * 8;
-    uint32_t lo = __ldg(q);
-    if (sh == 0) return lo;
-    uint32_t hi = __ldg(q + 1);
-    return __funnelshift_r(lo, hi, sh);
-}
-
 // Little-endian load of n (0..8) bytes at p, zero-filled above.
 __device__ __forceinline__ uint64_t ld_le64_part(const uint8_t *p, int n) {
     if (n >= 8 && (reinterpret_cast<uintptr_t>(p) & 7) == 0) return *reinterpret_cast<const uint64_t *>(p);

@@ -1,128 +1,271 @@
 // keygen_body.cuh -- P3 of a keypair (reference src/keypair.cu:55-120) and L of an expanded
-// secret key (src/expandsk.cu:37-80) on one CTA, shared by the batched kernels and the
-// persistent work-queue kernel.
+// secret key (src/expandsk.cu:37-80) on one CTA or a cluster of CTAs, shared by the batched kernels
+// and the persistent work-queue kernel.  Both are products of the key's quads with O (quad.cuh).
 #pragma once
 
-#include "engine.cuh"
 #include "launch_util.cuh"
+#include "quad.cuh"
 
 namespace mayo {
 
-template <int SET, int NT_ = 0>
+// P3 = Upper(O^T T), T = P1 O + P2: the rows of P1 as in VerifyCfg, then T's quads with O again.
+template <int SET, int CL_ = 1>
 struct KeyCfg {
     using S = Set<SET>;
-    static constexpr int J = S::o, W = S::W;
-    static constexpr int R_DEF = SET == 1 ? 5 : (SET == 2 ? 3 : (SET == 3 ? 3 : 2));
-    static constexpr int NT = NT_ ? NT_ : (J * W * R_DEF + 31) / 32 * 32;
-    static constexpr int R = NT / (J * W) < R_DEF ? NT / (J * W) : R_DEF;
-    static_assert(R >= 1 && J * W * R <= NT, "engine threads");
+    static constexpr int CL = CL_, J = S::o, NQ = QuadCfg<SET>::NQ, ST = QuadAcc<J>::ST;
+    static constexpr int QN = (S::v + 3) / 4;
+    static constexpr int NP = CL;
+    static constexpr int QL = (QN + NP - 1) / NP;
+    static constexpr int CH = (QL * NQ + 31) / 32;
+    // Warps and CTAs per SM, keypairs at 2,072 (us per instance): MAYO_1 three CTAs of four warps 0.321
+    // against 0.330 with four CTAs (128 registers, spills); MAYO_2 (153 accumulators) two warps 0.312
+    // against 0.322 with four and 0.486 with three CTAs of three warps (spills); MAYO_3 two CTAs of
+    // six warps 0.796 against 0.809 with four warps and two columns ahead; MAYO_5 one CTA of eleven
+    // warps 1.910 against 2.003 with six.
+    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 2 : SET == 3 ? 6 : 11);
+    static constexpr int NT = 32 * CW;
+    static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;
+    static constexpr int CH2 = (J * NQ + 31) / 32;
+    static constexpr int P2 = CH2 >= CW ? (SET == 5 ? 3 : 1) : (CW + CH2 - 1) / CH2;
+    static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 5 ? 1 : 2);
+    static constexpr int TRI = S::o * (S::o + 1) / 2;
     static constexpr size_t off_masks = 0;
-    static constexpr size_t off_bs = off_masks + (size_t)S::n * J * 16;
-    static constexpr size_t off_x = off_bs + (size_t)R * S::n * W * 16;
-    static constexpr size_t off_o = off_x + (size_t)J * J * W * 16;
-    static constexpr size_t total = off_o + pad16(S::o_bytes);
+    static constexpr size_t sz_masks = (size_t)S::v * ST * 16;
+    static constexpr size_t sz_mask2 = (size_t)QL * ST * 16, sz_upk = pad16((size_t)TRI * NQ * 4);
+    static_assert(sz_mask2 + sz_upk <= sz_masks, "second-step masks and P3 fit");
+    static constexpr size_t off_mask2 = 0, off_upk = sz_mask2;
+    static constexpr size_t off_T = sz_masks;
+    static constexpr size_t off_o = off_T + (size_t)J * CH * 32 * 16;
+    static constexpr size_t off_ctr = off_o + pad16(S::o_bytes);
+    static constexpr size_t total = off_ctr + 16;
 };
 
-// masks[c][b]: c < v -> O[c][b]; c >= v -> identity (adds P2 entries unscaled)
+// Rows r0 .. r0 + 3 of the upper-triangular P1, p1 bytes from base4; word q.
 template <int SET>
-__device__ __forceinline__ void build_o_masks(uint4 *masks, const uint8_t *s_O, int tid, int nthreads) {
+struct TriRows {
     using S = Set<SET>;
-    for (int idx = tid; idx < S::n * S::o; idx += nthreads) {
-        const int c = idx / S::o, b = idx - c * S::o;
-        uint32_t s;
-        if (c < S::v) {
-            const int q = c * S::o + b;
-            s = (s_O[q >> 1] >> ((q & 1) * 4)) & 0xF;
-        } else {
-            s = (c - S::v == b) ? 1u : 0u;
-        }
-        masks[idx] = scalar_masks(s);
+    uint32_t p1, q4;
+    int r0, row_l;
+    __device__ __forceinline__ void start(uint32_t (&bit)[4], int c) const {
+#pragma unroll
+        for (int i = 0; i < 4; i++) bit[i] = 8u * (p1 + (uint32_t)(tri(min(r0 + i, S::v - 1), c, S::v) * S::menc) + q4);
+    }
+    __device__ __forceinline__ void next(uint32_t (&bit)[4], int) const {
+#pragma unroll
+        for (int i = 0; i < 4; i++) bit[i] += 8 * S::menc;
+    }
+    __device__ __forceinline__ void next_all(uint32_t (&bit)[4], int c) const { next(bit, c); }
+    __device__ __forceinline__ bool keep(int i, int c) const { return c >= r0 + i; }
+    __device__ __forceinline__ void ahead(const uint32_t *base4, int c) const { row_ahead(base4, p1, row_l, c); }
+    __device__ static __forceinline__ void row_ahead(const uint32_t *base4, uint32_t p1, int r, int c) {
+        if (r < S::v && c >= r && c < S::v)
+            l2_prefetch(base4, p1 + (uint32_t)(tri(r, c, S::v) * S::menc), (uint32_t)(min(S::v - c, QUAD_AHEAD) * S::menc));
+    }
+};
+
+// O[c][j] from the packed O in shared memory.
+template <int SET>
+__device__ __forceinline__ uint32_t o_nibble(const uint8_t *s_O, int c, int j) {
+    const int q = c * Set<SET>::o + j;
+    return (uint32_t)(s_O[q >> 1] >> ((q & 1) * 4)) & 0xFu;
+}
+
+// The quad of entries (r0 + i, j) of P2 (v x o), word q, as packed words (rows past v: any value).
+template <int SET, bool RO>
+__device__ __forceinline__ void p2_words(const uint32_t *base4, uint32_t p2, int r0, int j, int q, uint32_t (&w)[4]) {
+    using S = Set<SET>;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t bit = 8u * (p2 + (uint32_t)((min(r0 + i, S::v - 1) * S::o + j) * S::menc) + 4u * q);
+        w[i] = raw_value(ld_raw<RO, true>(base4, bit, QuadCfg<SET>::bytes(q)), bit);
     }
 }
 
-template <int SET, bool RO = true>
-struct P3Rows {  // rows r < v of [P1 | P2] (src/keypair.cu:67-92)
-    using S = Set<SET>;
-    static constexpr bool read_only = RO;
-    const uint8_t *P1, *P2;
-    __device__ __forceinline__ int count(int r) const { return (S::v - r) + S::o; }
-    __device__ __forceinline__ const uint8_t *entry(int r, int e) const {
-        const int n1 = S::v - r;
-        return e < n1 ? P1 + (size_t)tri(r, r + e, S::v) * S::menc : P2 + (size_t)(r * S::o + (e - n1)) * S::menc;
+// n (1..4) bytes of a packed word to any address.
+__device__ __forceinline__ void store_word(uint8_t *p, uint32_t w, int n) {
+    if (n == 4 && (reinterpret_cast<uintptr_t>(p) & 3) == 0) {
+        *reinterpret_cast<uint32_t *>(p) = w;
+    } else if ((reinterpret_cast<uintptr_t>(p) & 1) == 0 && (n & 1) == 0) {
+        *reinterpret_cast<uint16_t *>(p) = (uint16_t)w;
+        if (n == 4) *reinterpret_cast<uint16_t *>(p + 2) = (uint16_t)(w >> 16);
+    } else {
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+            if (b < n) p[b] = (uint8_t)(w >> (8 * b));
     }
-    __device__ __forceinline__ int col(int r, int e) const { return r + e; }
-};
+}
 
-template <int SET>
-struct LRows {  // row r of P1 + P1^T without the diagonal, then P2 row r (src/expandsk.cu:162-199)
+// P3 of one instance: P1 || P2 at P1, O (o_bytes) already in shared memory at off_o (of every CTA of a
+// cluster); writes the packed upper triangle to P3out (rank 0).  All NT threads must call it.  RO:
+// P1 and P2 are not written in this kernel.
+template <int SET, int CL, bool RO>
+__device__ __forceinline__ void p3_instance(uint8_t *smem, int tid, const uint8_t *P1, uint8_t *P3out, int rank = 0) {
     using S = Set<SET>;
-    static constexpr bool read_only = false;  // L overwrites P2 in the same kernel
-    const uint8_t *P1, *P2;
-    __device__ __forceinline__ int count(int) const { return S::n; }
-    __device__ __forceinline__ const uint8_t *entry(int r, int e) const {
-        if (e < S::v) {
-            if (e == r) return nullptr;
-            return P1 + (size_t)(e > r ? tri(r, e, S::v) : tri(e, r, S::v)) * S::menc;
-        }
-        return P2 + (size_t)(r * S::o + (e - S::v)) * S::menc;
-    }
-    __device__ __forceinline__ int col(int, int e) const { return e; }
-};
-
-// P3 = Upper(O^T (P1 O + P2)) for one instance: O (o_bytes) already in smem at off_o; writes the
-// packed upper triangle to P3out.  All NT threads must call it.  RO: P1/P2 read-only in this kernel.
-template <int SET, int NT_, bool RO, int CU = 1>
-__device__ __forceinline__ void p3_instance(uint8_t *smem, int tid, const uint8_t *P1, const uint8_t *P2,
-                                            uint8_t *P3out) {
-    using S = Set<SET>;
-    using C = KeyCfg<SET, NT_>;
-    constexpr int J = C::J, W = C::W, R = C::R, NT = C::NT;
+    using C = KeyCfg<SET, CL>;
+    constexpr int J = C::J, NQ = C::NQ, NT = C::NT, NP = C::NP, ULP = C::CH * 32;
     uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
-    uint4 *bs = reinterpret_cast<uint4 *>(smem + C::off_bs);
-    uint4 *xacc = reinterpret_cast<uint4 *>(smem + C::off_x);
+    uint4 *mask2 = reinterpret_cast<uint4 *>(smem + C::off_mask2);
+    uint32_t *upk = reinterpret_cast<uint32_t *>(smem + C::off_upk);  // [pair][NQ]
+    uint4 *T = reinterpret_cast<uint4 *>(smem + C::off_T);            // [j][unit]
     const uint8_t *s_O = smem + C::off_o;
-    for (int i = tid; i < J * J * W * 4; i += NT) reinterpret_cast<uint32_t *>(xacc)[i] = 0;
-    build_o_masks<SET>(masks, s_O, tid, NT);
+    int *s_next = reinterpret_cast<int *>(smem + C::off_ctr);
+    const int warp = tid >> 5, lane = tid & 31;
+    const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(P1) & 3);
+    const uint32_t *base4 = reinterpret_cast<const uint32_t *>(P1 - mis);
+    if constexpr (CL == 1 && RO) {
+        for (int r = tid; r < S::v; r += NT) TriRows<SET>::row_ahead(base4, mis, r, r);
+        l2_prefetch_range(base4, mis + S::p1, S::p2, tid, NT);
+    }
+    auto scalar = [&](int c, int j) { return o_nibble<SET>(s_O, c, j); };
+    auto quad_scalar = [&](int t, int i, int j) {
+        const int c = 4 * (rank + t * NP) + i;
+        return c < S::v ? scalar(c, j) : 0u;
+    };
+    if (tid == 0) *s_next = 0;
+    build_masks9<J>(reinterpret_cast<uint32_t *>(masks), S::v, tid, NT, scalar);
+    if constexpr (C::PC > 1) {
+        for (int i = tid; i < J * ULP; i += NT) T[i] = make_uint4(0, 0, 0, 0);
+    }
     __syncthreads();
+    for (;;) {
+        const int item = warp_next(s_next, lane);
+        if (item >= C::CH * C::PC) break;
+        const int chunk = item / C::PC, piece = item - chunk * C::PC;
+        const int u = chunk * 32 + lane, t = u / NQ, q = u - t * NQ;
+        const int r0 = 4 * (rank + t * NP);
+        const int qmin = rank + (chunk * 32 / NQ) * NP, qmax = min(rank + ((chunk * 32 + 31) / NQ) * NP, C::QN - 1);
+        const int c_lo = min(4 * qmin, S::v), len = S::v - c_lo;
+        const int tl = chunk * 32 / NQ + (lane >> 2);
+        QuadAcc<J> acc;
+        acc.zero();
+        const TriRows<SET> rows{mis, (uint32_t)(4 * q), r0,
+                                RO && tl <= (chunk * 32 + 31) / NQ ? 4 * (rank + tl * NP) + (lane & 3) : S::v};
+        quad_columns<SET, J, RO, 1>(acc, rows, base4, QuadCfg<SET>::bytes(q), c_lo + len * piece / C::PC,
+                                    c_lo + len * (piece + 1) / C::PC, 4 * qmax + 4, masks);
+        const uint32_t rm = quad_row_mask(r0, S::v);
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            G4 v = acc.fold(j);
+            if (C::PC == 1 || piece == 0) {  // + P2[r][j]
+                uint32_t w[4];
+                p2_words<SET, RO>(base4, mis + S::p1, r0, j, q, w);
+                v = g4_xor(v, quad_planes(w[0], w[1], w[2], w[3]));
+            }
+            v = g4_and(v, rm);
+            if constexpr (C::PC > 1) g4_atomic_xor(T + j * ULP + u, v);
+            else g4_st(T + j * ULP + u, v);
+        }
+    }
+    __syncthreads();
+    build_quad_masks9<J>(reinterpret_cast<uint32_t *>(mask2), C::QL, tid, NT, quad_scalar);
+    for (int i = tid; i < C::TRI * NQ; i += NT) upk[i] = 0;
+    __syncthreads();
+    quad_pairs<SET, C>(T, ULP, mask2, upk, 0, warp, lane, [](int a, int b) { return tri(a, b, J); });
+    __syncthreads();
+    if constexpr (CL > 1) {
+        cluster_barrier();
+        if (rank == 0)
+            for (int i = tid; i < C::TRI * NQ; i += NT) upk[i] = xor_cluster<CL>(upk + i);
+        cluster_barrier();
+        if (rank != 0) return;
+        __syncthreads();
+    }
+    for (int i = tid; i < C::TRI * NQ; i += NT) {
+        const int p = i / NQ, q = i - p * NQ;
+        store_word(P3out + p * S::menc + 4 * q, upk[i], QuadCfg<SET>::bytes(q));
+    }
+}
 
-    Engine<SET, J, R, true, CU> eng;
-    eng.setup(masks, bs, tid);
-    const P3Rows<SET, RO> rows{P1, P2};
-    G4 X[J];
+// L = (P1 + P1^T) O + P2, in place over P2.
+template <int SET, int CL_ = 1>
+struct LCfg {
+    using S = Set<SET>;
+    static constexpr int CL = CL_, J = S::o, NQ = QuadCfg<SET>::NQ, ST = QuadAcc<J>::ST;
+    static constexpr int QN = (S::v + 3) / 4, CH = (QN * NQ + 31) / 32;  // chunks, every one v columns long
+    // expand-sk at 2,072 (us per instance): MAYO_1 0.410 with three CTAs per SM, 0.424 with four (128
+    // registers); MAYO_2 0.327 with four warps, 0.344 with two; MAYO_5 2.61 with eleven warps, 2.76
+    // with two CTAs of six, 2.83 with seven warps
+    static constexpr int CW = CL > 1 ? (CH + CL - 1) / CL : (SET == 1 ? 4 : SET == 2 ? 4 : SET == 3 ? 6 : 11);
+    static constexpr int NT = 32 * CW;
+    static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 5 ? 1 : 2);
+    static constexpr size_t off_masks = 0;
+    static constexpr size_t off_o = (size_t)S::v * ST * 16;
+    static constexpr size_t off_ctr = off_o + pad16(S::o_bytes);
+    static constexpr size_t total = off_ctr + 16;
+};
+
+// Rows r0 .. r0 + 3 of P1 + P1^T without the diagonal: entry (r, c) is P1's (c, r) left of the
+// diagonal.  lower: every row of the warp is there for all columns asked for (next_all's step).
+template <int SET>
+struct SymRows {
+    using S = Set<SET>;
+    uint32_t p1, q4;
+    int r0;
+    bool lower;
+    __device__ __forceinline__ void start(uint32_t (&bit)[4], int c) const {
 #pragma unroll
-    for (int i = 0; i < J; i++) X[i] = g4_zero();
-#pragma unroll 1
-    for (int r0 = 0; r0 < S::v; r0 += R) {
-        // the next pass's rows into L2 (MAYO_1/3/5 keypairs 1-5 % faster, MAYO_2's 4 % slower)
-        if (SET != 2 && tid < 32) eng.prefetch(rows, r0 + R, S::v, tid);
-        eng.convert(rows, r0, S::v, tid, NT);
-        __syncthreads();
-        const int r = r0 + eng.rs;
-        if (eng.active && r < S::v) {
-            const G4 T = eng.row_product(rows, r);  // B[r][j] = (P1 O + P2)[r][j]
-            const uint4 *mr = masks + (size_t)r * J;  // O[r][a]
-#pragma unroll
-            for (int a = 0; a < J; a++) g4_madd(X[a], T, mr[a]);
+        for (int i = 0; i < 4; i++) {
+            const int r = min(r0 + i, S::v - 1);
+            bit[i] = 8u * (p1 + (uint32_t)((c < r ? tri(c, r, S::v) : tri(r, c, S::v)) * S::menc) + q4);
         }
-        __syncthreads();
     }
-    if (eng.active) {
+    // tri(c, r) - tri(c - 1, r) = v - c for c <= r
+    __device__ __forceinline__ void next(uint32_t (&bit)[4], int c) const {
+        const uint32_t lo = 8u * S::menc * (uint32_t)(S::v - c);
 #pragma unroll
-        for (int a = 0; a < J; a++) g4_atomic_xor(xacc + ((size_t)a * J + eng.j) * W + eng.w, X[a]);
+        for (int i = 0; i < 4; i++) bit[i] += c <= min(r0 + i, S::v - 1) ? lo : 8u * S::menc;
     }
+    __device__ __forceinline__ void next_all(uint32_t (&bit)[4], int c) const {
+        const uint32_t d = lower ? 8u * S::menc * (uint32_t)(S::v - c) : 8u * S::menc;
+#pragma unroll
+        for (int i = 0; i < 4; i++) bit[i] += d;
+    }
+    __device__ __forceinline__ bool keep(int i, int c) const { return c != r0 + i; }
+    __device__ __forceinline__ void ahead(const uint32_t *, int) const {}
+};
+
+// L of one instance: P1 at P1 (then P2, which becomes L); O in shared memory at LCfg::off_o.
+template <int SET, int CL>
+__device__ __forceinline__ void l_instance(uint8_t *smem, int tid, const uint8_t *P1, uint8_t *P2, int rank) {
+    using S = Set<SET>;
+    using C = LCfg<SET, CL>;
+    constexpr int J = C::J, NQ = C::NQ, NT = C::NT;
+    uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
+    const uint8_t *s_O = smem + C::off_o;
+    int *s_next = reinterpret_cast<int *>(smem + C::off_ctr);
+    const int lane = tid & 31;
+    const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(P1) & 3);
+    const uint32_t *base4 = reinterpret_cast<const uint32_t *>(P1 - mis);
+    if (tid == 0) *s_next = 0;
+    build_masks9<J>(reinterpret_cast<uint32_t *>(masks), S::v, tid, NT,
+                    [&](int c, int j) { return o_nibble<SET>(s_O, c, j); });
     __syncthreads();
-    // P3[a][b] = X_ab + X_ba (a < b), X_aa; upper triangle row-major
-    for (int idx = tid; idx < S::o * (S::o + 1) / 2 * W; idx += NT) {
-        const int pid = idx / W, ww = idx - pid * W;
-        int a = 0, rem = pid;
-        while (rem >= J - a) {
-            rem -= J - a;
-            a++;
+    for (;;) {
+        const int chunk = rank + CL * warp_next(s_next, lane);
+        if (chunk >= C::CH) break;
+        const int u = chunk * 32 + lane, t = u / NQ, q = u - t * NQ, r0 = 4 * t;
+        const int qmin = chunk * 32 / NQ, qmax = min((chunk * 32 + 31) / NQ, C::QN - 1);
+        QuadAcc<J> acc;
+        acc.zero();
+        SymRows<SET> rows{mis, (uint32_t)(4 * q), r0, false};
+#pragma unroll 1
+        for (int seg = 0; seg < 2; seg++) {  // from the diagonal on, then the columns left of every row
+            rows.lower = seg == 1;
+            quad_columns<SET, J, true, 1>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? 0 : 4 * qmin,
+                                          seg ? 4 * qmin : S::v, seg ? 0 : 4 * qmax + 4, masks);
         }
-        const int b = a + rem;
-        G4 u = g4_ld(xacc + ((size_t)a * J + b) * W + ww);
-        if (a != b) u = g4_xor(u, g4_ld(xacc + ((size_t)b * J + a) * W + ww));
-        store_group<SET>(P3out + (size_t)tri(a, b, S::o) * S::menc, ww, u);
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            const G4 f = acc.fold(j);
+            const G4 v = quad_planes(f.p0, f.p1, f.p2, f.p3);
+            const uint32_t wd[4] = {v.p0, v.p1, v.p2, v.p3};
+            uint32_t w[4];
+            p2_words<SET, false>(base4, mis + S::p1, r0, j, q, w);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (r0 + i < S::v)
+                    store_word(P2 + (size_t)((r0 + i) * S::o + j) * S::menc + 4 * q, wd[i] ^ w[i], QuadCfg<SET>::bytes(q));
+        }
     }
 }
 

@@ -60,62 +60,34 @@ __global__ void expandsk_hash_kernel(uint8_t *pool, size_t pitch, uint32_t batch
 }
 
 // ---------------------------------------------------------------------------------------------
-// P3 (keypair) and L (expandsk) engine kernels: one CTA per instance.
+// P3 (keypair) and L (expandsk) kernels: one CTA per instance, or a cluster where the batch is small.
 // ---------------------------------------------------------------------------------------------
-template <int SET>
-__global__ void __launch_bounds__(KeyCfg<SET>::NT) p3_kernel(uint8_t *pool, size_t pitch) {
+template <int SET, int CL>
+__global__ void __launch_bounds__(KeyCfg<SET, CL>::NT, KeyCfg<SET, CL>::MINB) p3_kernel(uint8_t *pool, size_t pitch) {
     using S = Set<SET>;
-    using C = KeyCfg<SET>;
+    using C = KeyCfg<SET, CL>;
     extern __shared__ __align__(16) uint8_t smem[];
     const int tid = threadIdx.x;
-    uint8_t *row = pool + (size_t)blockIdx.x * pitch;
+    uint8_t *row = pool + (size_t)(blockIdx.x / CL) * pitch;
     uint8_t *pk = row + align128(S::sk);
     const uint8_t *P1 = pk + align128(S::pk);
     // O is parked in pk[16:]: copy it to shared memory before P3 overwrites that region
     for (int i = tid; i < S::o_bytes; i += C::NT) smem[C::off_o + i] = pk[16 + i];
     __syncthreads();
-    // batched row loads (CU = 4) measured faster for MAYO_2's P3 only (MAYO_1/3/5: 0.494 -> 0.502,
-    // 1.18 -> 1.20, 2.89 -> 3.04 ms per 1,024 keypairs; MAYO_2 0.475 -> 0.462)
-    p3_instance<SET, C::NT, true, SET == 2 ? 4 : 1>(smem, tid, P1, P1 + S::p1, pk + 16);
+    p3_instance<SET, CL, true>(smem, tid, P1, pk + 16, CL > 1 ? (int)cluster_rank() : 0);
 }
 
-template <int SET>
-__global__ void __launch_bounds__(KeyCfg<SET>::NT) l_kernel(uint8_t *pool, size_t pitch) {
+template <int SET, int CL>
+__global__ void __launch_bounds__(LCfg<SET, CL>::NT, LCfg<SET, CL>::MINB) l_kernel(uint8_t *pool, size_t pitch) {
     using S = Set<SET>;
-    using C = KeyCfg<SET>;
-    constexpr int J = C::J, R = C::R, NT = C::NT;
+    using C = LCfg<SET, CL>;
     extern __shared__ __align__(16) uint8_t smem[];
-    uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
-    uint4 *bs = reinterpret_cast<uint4 *>(smem + C::off_bs);
-    uint8_t *s_O = smem + C::off_o;
     const int tid = threadIdx.x;
-    uint8_t *row = pool + (size_t)blockIdx.x * pitch;
-    const uint8_t *P1 = row + S::sk + S::o_bytes;
-    uint8_t *P2 = row + S::sk + S::o_bytes + S::p1;
-
-    for (int i = tid; i < S::o_bytes; i += NT) s_O[i] = row[S::sk + i];
+    uint8_t *row = pool + (size_t)(blockIdx.x / CL) * pitch;
+    uint8_t *P1 = row + S::sk + S::o_bytes;
+    for (int i = tid; i < S::o_bytes; i += C::NT) smem[C::off_o + i] = row[S::sk + i];
     __syncthreads();
-    build_o_masks<SET>(masks, s_O, tid, NT);
-    __syncthreads();
-
-    // four row groups' loads in flight per thread: L reads P1 twice (rows and columns) with
-    // little else to hide the latency (MAYO_1 signWithesk 1.10 -> 1.07 ms per 1,024, MAYO_5
-    // 7.13 -> 6.97)
-    Engine<SET, J, R, true, 4> eng;
-    eng.setup(masks, bs, tid);
-    const LRows<SET> rows{P1, P2};
-#pragma unroll 1
-    for (int r0 = 0; r0 < S::v; r0 += R) {
-        if (SET >= 3 && tid < 32) eng.prefetch(rows, r0 + R, S::v, tid);  // next pass into L2
-        eng.convert(rows, r0, S::v, tid, NT);
-        __syncthreads();
-        const int r = r0 + eng.rs;
-        if (eng.active && r < S::v) {
-            const G4 T = eng.row_product(rows, r);  // L[r][j]
-            store_group<SET>(P2 + (size_t)(r * S::o + eng.j) * S::menc, eng.w, T);
-        }
-        __syncthreads();
-    }
+    l_instance<SET, CL>(smem, tid, P1, P1 + S::p1, (int)(blockIdx.x % CL));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -145,31 +117,52 @@ static int aes_expand(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st
     return cudaPeekAtLastError() == cudaSuccess ? ST_OK : ST_CUDA;
 }
 
+template <int SET, int CL>
+static int p3_cl(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st) {
+    using C = KeyCfg<SET, CL>;
+    if (!set_smem_attr(p3_kernel<SET, CL>, C::total)) return ST_CUDA;
+    return launch_cluster(p3_kernel<SET, CL>, (unsigned)(batch * CL), C::NT, C::total, CL, st, pool, pitch) == cudaSuccess
+               ? ST_OK
+               : ST_CUDA;
+}
+// The CTAs of an instance share no shared memory here: a plain grid.
+template <int SET, int CL>
+static int l_cl(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st) {
+    using C = LCfg<SET, CL>;
+    if (!set_smem_attr(l_kernel<SET, CL>, C::total)) return ST_CUDA;
+    l_kernel<SET, CL><<<(unsigned)(batch * CL), C::NT, C::total, st>>>(pool, pitch);
+    return cudaPeekAtLastError() == cudaSuccess ? ST_OK : ST_CUDA;
+}
+
 template <int SET>
 static int keypair_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, uint64_t rand_index, bool seeded) {
     using S = Set<SET>;
-    using C = KeyCfg<SET>;
     keypair_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch, rand_index,
                                                                                  seeded ? 1 : 0);
     const size_t pk_off = align128(S::sk);
     int rc = aes_expand(pool, pitch, batch, st, pk_off, pk_off + align128(S::pk), S::p, false);
     if (rc) return rc;
-    if (!set_smem_attr(p3_kernel<SET>, C::total)) return ST_CUDA;
-    p3_kernel<SET><<<(unsigned)batch, C::NT, C::total, st>>>(pool, pitch);
-    return cudaPeekAtLastError() == cudaSuccess ? ST_OK : ST_CUDA;
+    switch (cluster_ctas(batch)) {
+        case 8: return p3_cl<SET, 8>(pool, pitch, batch, st);
+        case 4: return p3_cl<SET, 4>(pool, pitch, batch, st);
+        case 2: return p3_cl<SET, 2>(pool, pitch, batch, st);
+        default: return p3_cl<SET, 1>(pool, pitch, batch, st);
+    }
 }
 
 template <int SET>
 static int expandsk_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st) {
     using S = Set<SET>;
-    using C = KeyCfg<SET>;
     expandsk_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch);
     const size_t out_off = S::sk + S::o_bytes;
     int rc = aes_expand(pool, pitch, batch, st, out_off + S::p - 16, out_off, S::p, true);
     if (rc) return rc;
-    if (!set_smem_attr(l_kernel<SET>, C::total)) return ST_CUDA;
-    l_kernel<SET><<<(unsigned)batch, C::NT, C::total, st>>>(pool, pitch);
-    return cudaPeekAtLastError() == cudaSuccess ? ST_OK : ST_CUDA;
+    switch (cluster_ctas(batch)) {
+        case 8: return l_cl<SET, 8>(pool, pitch, batch, st);
+        case 4: return l_cl<SET, 4>(pool, pitch, batch, st);
+        case 2: return l_cl<SET, 2>(pool, pitch, batch, st);
+        default: return l_cl<SET, 1>(pool, pitch, batch, st);
+    }
 }
 
 template <int SET>

@@ -6,9 +6,9 @@
 //   2. partitions the caller's mixed item array into 12 buckets, one per (set, op), keeping the
 //      order within a bucket,
 //   3. forks streams and launches one persistent kernel per bucket whose operands are set.
-// Each (set, op) has its own kernel because their CTAs need 35-81 KB of shared memory and 56-128
-// registers per thread: one kernel shaped for the largest would run MAYO_1 at two CTAs per SM
-// instead of five, and MAYO_5's keypair and verify at two instead of three.  Each kernel has the
+// Each (set, op) has its own kernel because their CTAs need 23-205 KB of shared memory and 96-255
+// registers per thread: one kernel shaped for the largest would run every set at one CTA per SM
+// (MAYO_1 runs three, MAYO_2's sign and verify six).  Each kernel has the
 // shape of the batched kernel for its (set, op).  On forked streams the kernels share the SMs,
 // and the CTAs of a kernel launched later take the SMs of one whose bucket has drained, so one
 // bucket's tail overlaps another's work.
@@ -35,8 +35,6 @@ constexpr uint32_t Q_EMPTY = 0xFFFFFFFFu;
 constexpr uint32_t Q_STOP = 0xFFFFFFFEu;
 constexpr int Q_BUCKETS = 12;             // (set index) * 3 + op
 constexpr int Q_CTRL_WORDS = 16;          // control words per bucket; block 12 counts invalid ops
-constexpr size_t Q_SM_SMEM = 228 * 1024;  // shared memory per SM (sm_100)
-constexpr size_t Q_CTA_RESERVED = 1024;   // shared memory the runtime reserves per CTA
 
 template <int SET, int OP>
 struct QueueCfg;
@@ -45,10 +43,11 @@ template <int SET>
 struct QueueCfg<SET, MAYO_B200_OP_KEYPAIR> {
     using S = Set<SET>;
     using KC = KeyCfg<SET>;
-    static constexpr int NT = KC::NT;
-    // replicated T0 (and ror16(T0) where the P3 engine's area below O holds both: MAYO_5) and the
-    // round keys; the tables are dead once the keystream is written
-    static constexpr int NTAB = KC::off_o >= 2 * 256 * 32 * 4 + 44 * 4 ? 2 : 1;
+    static constexpr int NT = KC::NT, MINB = KC::MINB;
+    // as many replicated round tables as the P3 area below O holds (MAYO_1: T0; MAYO_2: T0 and
+    // ror16(T0); MAYO_3/5: all three) and the round keys; dead once the keystream is written
+    static constexpr int ntab(int n) { return KC::off_o >= (size_t)n * 256 * 32 * 4 + 44 * 4; }
+    static constexpr int NTAB = ntab(3) ? 3 : ntab(2) ? 2 : 1;
     static constexpr size_t aes_end = NTAB * 256 * 32 * 4 + 44 * 4;
     static_assert(KC::off_o >= aes_end, "O must not overlap the AES tables");
     static constexpr size_t seedpk = KC::off_o + pad16(S::o_bytes);
@@ -58,24 +57,16 @@ struct QueueCfg<SET, MAYO_B200_OP_KEYPAIR> {
 
 template <int SET>
 struct QueueCfg<SET, MAYO_B200_OP_SIGN> {
-    static constexpr int NT = SignCfg<SET>::NT;
+    static constexpr int NT = SignCfg<SET>::NT, MINB = SignCfg<SET>::MINB;
     static constexpr size_t smem = SignCfg<SET>::total;
     static constexpr size_t scratch = 0;
 };
 
 template <int SET>
 struct QueueCfg<SET, MAYO_B200_OP_VERIFY> {
-    static constexpr int NT = VerifyCfg<SET>::NT;
+    static constexpr int NT = VerifyCfg<SET>::NT, MINB = VerifyCfg<SET>::MINB;
     static constexpr size_t smem = VerifyCfg<SET>::total;
     static constexpr size_t scratch = 0;
-};
-
-// CTAs of a bucket's kernel that fit in one SM's shared memory: the register budget per thread
-// is set so that registers do not lower the residency further.
-template <int SET, int OP>
-struct QueueFit {
-    static constexpr int fit = (int)(Q_SM_SMEM / (QueueCfg<SET, OP>::smem + Q_CTA_RESERVED));
-    static constexpr int MINB = fit > 8 ? 8 : (fit < 1 ? 1 : fit);
 };
 
 using QueueOps = mayo_b200_queue_ops;
@@ -221,6 +212,10 @@ __device__ void queue_keypair(uint8_t *smem, int tid, const QueueOps &ops, uint3
         const uint32_t v = c_aes.te0[i >> 5];
         T[i] = v;
         if (NTAB == 2) T[256 * 32 + i] = ror16(v);
+        if (NTAB == 3) {
+            T[256 * 32 + i] = ror8(v);
+            T[2 * 256 * 32 + i] = ror16(v);
+        }
     }
     __syncthreads();
     {
@@ -237,7 +232,7 @@ __device__ void queue_keypair(uint8_t *smem, int tid, const QueueOps &ops, uint3
     }
     __syncthreads();  // scratch writes visible to the whole CTA; AES tables no longer needed
     for (int i = tid; i < 16; i += NT) pk[i] = s_seedpk[i];
-    p3_instance<SET, NT, false>(smem, tid, scratch, scratch + S::p1, pk + 16);
+    p3_instance<SET, 1, false>(smem, tid, scratch, pk + 16);
 }
 
 template <int SET>
@@ -256,7 +251,7 @@ __device__ void queue_sign(uint8_t *smem, int tid, const QueueArgs &q, const Ite
 }
 
 template <int SET, int OP>
-__global__ void __launch_bounds__(QueueCfg<SET, OP>::NT, QueueFit<SET, OP>::MINB) queue_kernel(const QueueArgs q) {
+__global__ void __launch_bounds__(QueueCfg<SET, OP>::NT, QueueCfg<SET, OP>::MINB) queue_kernel(const QueueArgs q) {
     using S = Set<SET>;
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint32_t s_item;

@@ -1,7 +1,7 @@
 // op_shared.cu -- sign / verify of a batch under ONE key, with the key's heavy products on the
 // tensor cores (tcgen05.mma, kind::i8).
 //
-// The per-instance engine (engine.cuh) spends most of a signature on T_j[r] = sum_c P1[r][c] V_j[c]
+// The per-instance kernels (quad.cuh) spend most of a signature on T_j[r] = sum_c P1[r][c] V_j[c]
 // (U = V^T P1 V) and M_j[b] = sum_a V_j[a] L[a][b] (src/sign.cu:254-330, 396-437), and most of a
 // verification on T_j[r] = sum_c P[r][c] s_j[c] (src/verify.cu:72-182).  When every instance of a
 // batch uses the same key these are one matrix product over the whole batch: GF(16) is GF(2)^4,
@@ -28,7 +28,7 @@
 //   SHAKE256 block count, and the hash kernels take them in that order.
 //   sign: sign_hash_kernel (thread per instance) -> product -> sign_shared_tail_kernel (first
 //         attempt from the planes in a compact CTA) -> sign_shared_fix_kernel (retries of the
-//         rare singular first attempts with the engine).
+//         rare singular first attempts per instance).
 //   verify: verify_hash_kernel (thread per instance: digest, t) -> product ->
 //         verify_shared_tail_kernel (U from the planes, Horner, compare; a small CTA).
 //   If the status word shows a failed product, the tails do nothing and the fix-up kernels run
@@ -899,7 +899,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SH_GEMM_NT, 1)
 
 // ---- sign ----
 // First attempt from the planes, in a CTA without engine staging (more CTAs per SM).  A singular
-// first attempt goes to the retry list; the fix-up kernel finishes it with the engine.
+// first attempt goes to the retry list; the fix-up kernel finishes it per instance.
 // SH_TAIL_G instances per CTA (sign_attempt's interleaved elimination: the G pivot owners of a
 // step share one publish and the live columns fill whole warps); a CTA's last instances past the
 // batch repeat the batch's last instance and write nothing.
@@ -908,7 +908,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SH_GEMM_NT, 1)
 template <int SET, int G>
 struct TailShape {
     // threads per signature: three warps where the elimination's ko + 1 columns fit (MAYO_1: 81,
-    // MAYO_2: 69); the engine's row slots shrink with them (R = 3 / 12).  More signatures per SM
+    // MAYO_2: 69); the row slots shrink with them (R = 3 / 12).  More signatures per SM
     // at the same registers: MAYO_2 G = 4, 4 CTAs of 384 threads at 40 registers (16 signatures
     // per SM against 12 with 128 threads), 1.643 -> 1.494 ms at 65,536.
     static constexpr int TNT = (SET == 1 || SET == 2) ? 96 : (SET == 5 ? 160 : 128);
@@ -944,7 +944,7 @@ __global__ void __launch_bounds__(TailShape<SET, G>::NT, TailShape<SET, G>::MINB
     if (!ok && live && tid == 0) retry[atomicAdd(&ctl[1], 1u)] = inst;
 }
 
-// Retries (attempts ctr >= 1 of the listed instances) with the engine, or every instance from
+// Retries (attempts ctr >= 1 of the listed instances) per instance, or every instance from
 // ctr = 0 if the product gave up.  A grid-stride loop over a count read on the device.
 template <int SET>
 __global__ void __launch_bounds__(SignCfg<SET>::NT, SignCfg<SET>::MINB)
@@ -1087,7 +1087,7 @@ __global__ void __launch_bounds__(VTailCfg<SET>::NT)
     }
 }
 
-// Every instance with the engine, only if the product gave up.
+// Every instance on its own, only if the product gave up.
 template <int SET>
 __global__ void __launch_bounds__(VerifyCfg<SET>::NT, VerifyCfg<SET>::MINB)
     verify_shared_fix_kernel(const VerifyIO io, const uint32_t *ctl, uint32_t batch) {

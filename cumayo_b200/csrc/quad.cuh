@@ -22,13 +22,26 @@
 //     (9 JB / 4 loads) and the key words (8 loads, two clocks each) keep the load pipe about as busy
 //     as the products keep the logic pipe (MAYO_1: 62 and 57 clocks per column; measured 89).
 // Verify at 3,552 / 3,552 / 2,072 / 1,036 instances with keys of their own (MAYO_1, 2, 3, 5): 0.33,
-// 0.17, 0.66, 1.46 us per instance with the plane products of engine.cuh, 0.153, 0.067, 0.43, 0.85 here.
+// 0.17, 0.66, 1.46 us per instance with the plane products (16 LOP3, rows staged
+// in shared memory between barriers), 0.153, 0.067, 0.43, 0.85 here.
 // Scalars enter only as masks and no address depends on them: constant time.
 #pragma once
 
 #include "common.cuh"
 
 namespace mayo {
+
+// XOR-accumulate a G4 into shared memory (atomic).
+__device__ __forceinline__ void g4_atomic_xor(uint4 *dst, const G4 &g) {
+    uint32_t *d = reinterpret_cast<uint32_t *>(dst);
+    atomicXor(d + 0, g.p0);
+    atomicXor(d + 1, g.p1);
+    atomicXor(d + 2, g.p2);
+    atomicXor(d + 3, g.p3);
+}
+
+// Named barrier over the first `n` threads (n a multiple of 32).
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 constexpr int NFORM = 9;
 
@@ -173,9 +186,9 @@ __device__ __forceinline__ void l2_prefetch_range(const uint32_t *base4, uint32_
 
 // Columns [c0, c1) of one unit: acc += S[c] * (the quad's entries of column c).  `rows` gives the
 // addresses: bit[4] (bit offsets from base4, the unit's word included), rows.start(bit, c) for
-// column c, rows.next(bit, c) from column c - 1 to c, rows.keep(i, c) whether row i has an entry in
-// column c (asked for c < c_chk only; a row's offset is in bounds for every c), rows.ahead(base4, c)
-// to ask L2 for the warp's rows from column c on.  The loads of column c + D are issued before the
+// column c, rows.next(bit, c) from column c - 1 to c (next_all: the same where c - 1 >= c_chk),
+// rows.keep(i, c) whether row i has an entry in column c (asked for c < c_chk only; a row's offset is
+// in bounds for every c), rows.ahead(base4, c) to ask L2 for the warp's rows from column c on.  The loads of column c + D are issued before the
 // products of column c.  All lanes of a warp must pass the same c0, c1 and c_chk.
 // Three loops, so that the long one (every row has an entry, no column is the last) has no tests.
 constexpr int QUAD_AHEAD = 16;  // columns per L2 request
@@ -204,13 +217,11 @@ __device__ __forceinline__ void quad_columns(QuadAcc<JB> &acc, const Rows &rows,
 #pragma unroll
             for (int i = 0; i < 4; i++) raw[d][i] = raw[d + 1][i];
     };
-    auto load_next = [&](int c) {  // column c, not the last
-        rows.next(bl, c);
+    auto load_last = [&] {  // column c + D, not the last of the range
 #pragma unroll
         for (int i = 0; i < 4; i++) raw[D - 1][i] = ld_raw<RO, false>(base4, bl[i], n);
     };
-    auto products = [&](int c) {
-        rows.next(bit, c + 1);
+    auto products = [&] {
         uint32_t f[NFORM];
         forms_of(quad_planes(w[0], w[1], w[2], w[3], two, four), f);
         acc.madd(mp, f);
@@ -227,14 +238,18 @@ __device__ __forceinline__ void quad_columns(QuadAcc<JB> &acc, const Rows &rows,
             take();
 #pragma unroll
             for (int i = 0; i < 4; i++) w[i] = rows.keep(i, c) ? w[i] : 0u;
-            load_next(c + D);
-            products(c);
+            rows.next(bl, c + D);
+            load_last();
+            rows.next(bit, c + 1);
+            products();
         }
 #pragma unroll D
         for (; c < b2; c++) {
             take();
-            load_next(c + D);
-            products(c);
+            rows.next_all(bl, c + D);
+            load_last();
+            rows.next_all(bit, c + 1);
+            products();
         }
     }
 #pragma unroll 1
@@ -247,7 +262,8 @@ __device__ __forceinline__ void quad_columns(QuadAcc<JB> &acc, const Rows &rows,
 #pragma unroll
             for (int i = 0; i < 4; i++) raw[D - 1][i] = ld_raw<RO, true>(base4, bl[i], n);
         }
-        products(c);
+        rows.next(bit, c + 1);
+        products();
     }
 }
 
@@ -276,6 +292,7 @@ struct PubRows {
 #pragma unroll
         for (int i = 0; i < 4; i++) bit[i] += 8 * S::menc;
     }
+    __device__ __forceinline__ void next_all(uint32_t (&bit)[4], int c) const { next(bit, c); }
     __device__ __forceinline__ bool keep(int i, int c) const { return c >= r0 + i; }
     __device__ __forceinline__ void ahead(const uint32_t *base4, int c) const { row_ahead(base4, p, row_l, c); }
     // columns c .. c + QUAD_AHEAD - 1 of row r, up to the end of its run
@@ -356,10 +373,10 @@ __device__ __forceinline__ uint32_t xor_cluster(const uint32_t *p) {
 __device__ __forceinline__ int pair_ell(int a, int b, int k) { return a * k - (a * (a - 1)) / 2 + (k - 1 - b); }
 
 // The second step: X_ij = sum_r S[r][i] T_j[r] over the quads t0 <= t < C::QL of T ([j][ulp units]),
-// packed and added to U (upk[l][NQ]).  A unit is (j, word); masks2: the quads' scalars.
-template <int SET, class C>
-__device__ __forceinline__ void quad_pairs(const uint4 *T, int ulp, const uint4 *mask2, uint32_t *upk, int t0, int warp,
-                                           int lane) {
+// packed and added to out[index(i <= j)][NQ].  A unit is (j, word); masks2: the quads' scalars.
+template <int SET, class C, class F>
+__device__ __forceinline__ void quad_pairs(const uint4 *T, int ulp, const uint4 *mask2, uint32_t *out, int t0, int warp,
+                                           int lane, F index) {
     constexpr int J = C::J, NQ = C::NQ;
 #pragma unroll 1
     for (int task = warp; task < C::CH2 * C::P2; task += C::CW) {
@@ -378,7 +395,7 @@ __device__ __forceinline__ void quad_pairs(const uint4 *T, int ulp, const uint4 
             const uint32_t lm = q == NQ - 1 ? QuadCfg<SET>::LAST_MASK : 0xFFFFFFFFu;
 #pragma unroll
             for (int i = 0; i < J; i++)
-                atomicXor(upk + pair_ell(min(i, j), max(i, j), J) * NQ + q, quad_row_sum(acc.fold(i)) & lm);
+                atomicXor(out + index(min(i, j), max(i, j)) * NQ + q, quad_row_sum(acc.fold(i)) & lm);
         }
     }
 }

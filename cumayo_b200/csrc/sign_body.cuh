@@ -18,7 +18,6 @@
 // same z.  Rank < m is detected by both (the reference: last echelon row zero).
 #pragma once
 
-#include "engine.cuh"
 #include "launch_util.cuh"
 #include "ops.h"
 #include "quad.cuh"
@@ -134,6 +133,7 @@ struct SignRows {
 #pragma unroll
         for (int i = 0; i < 4; i++) bit[i] += d;
     }
+    __device__ __forceinline__ void next_all(uint32_t (&bit)[4], int c) const { next(bit, c); }
     __device__ __forceinline__ bool keep(int i, int c) const { return x < MQ || c >= 4 * (x - MQ) + i; }
     __device__ __forceinline__ void ahead(const uint32_t *base4, int c) const { row_ahead(base4, p1, row_l, c); }
     // columns c .. of row r of P1
@@ -434,7 +434,7 @@ __device__ __forceinline__ bool sign_products(uint8_t *smem, int tid, const uint
             for (int i = tid; i < S::pairs * NQ; i += NT) upk[i] = 0;
             __syncthreads();
         }
-        quad_pairs<SET, C>(T, C::TU, mask2, upk, tm, warp, lane);
+        quad_pairs<SET, C>(T, C::TU, mask2, upk, tm, warp, lane, [](int a, int b) { return pair_ell(a, b, J); });
         __syncthreads();
     }
     if constexpr (CL > 1) {
@@ -815,7 +815,7 @@ __device__ __forceinline__ void sign_write(uint8_t *smem, int tid, const uint8_t
                                            const uint4 *opl = nullptr) {
     MAYO_SIGN_VIEWS
     // s_i = V_i + O x_i on bit planes: the columns of O as planes and the k x W accumulators in
-    // the engine staging area (free after the attempt); each accumulator (i, w) takes its o
+    // the area of T and the columns of A (free after the attempt); each accumulator (i, w) takes its o
     // multiply-accumulates from SPL threads (shared-memory XOR to combine); nibbles are staged
     // one per byte (the mask area, also free) because s_i starts mid-byte when n is odd.
     constexpr int SPL = 4;

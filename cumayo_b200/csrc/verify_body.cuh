@@ -9,7 +9,6 @@
 // y = sum z^l U_l is then collected by all warps and compared with t.
 #pragma once
 
-#include "engine.cuh"
 #include "launch_util.cuh"
 #include "quad.cuh"
 
@@ -154,7 +153,7 @@ __device__ __forceinline__ void verify_instance(uint8_t *smem, int tid, const ui
             __syncthreads();
         }
         // ---- X_ij = sum_r s_i[r] T_j[r], packed into U_l ----
-        quad_pairs<SET, C>(T, ULP, mask2, upk, 0, warp, lane);
+        quad_pairs<SET, C>(T, ULP, mask2, upk, 0, warp, lane, [](int a, int b) { return pair_ell(a, b, J); });
         __syncthreads();
     }
     if constexpr (CL > 1) {  // the ranks' parts of U meet in rank 0

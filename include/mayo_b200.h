@@ -215,7 +215,7 @@ MAYO_B200_API int mayo_b200_verify_shared(int set, const uint8_t *epk, const uin
  * A device queue of keypair / sign / verify items of all four parameter sets.  The mixed item
  * array is partitioned on the device (stably) into 12 buckets, one per (set, op), each drained by
  * its own persistent kernel shaped like the batched kernel for that (set, op) (their CTAs need
- * 35-81 KB of shared memory, so one kernel for all would hold every set to the residency of the
+ * 23-205 KB of shared memory, so one kernel for all would hold every set to the residency of the
  * largest).  The kernels are launched on forked streams, so they share the SMs and fill each
  * other's tails.  A sign attempt with a singular system is re-enqueued with the next attempt
  * counter instead of being retried in place.  Every wait inside the kernels is bounded; an

@@ -1,4 +1,4 @@
-"""Per-instance sign and verify at the edges of their launch rule (one CTA per instance, or a
+"""Per-instance keypair, expand-sk, sign and verify at the edges of their launch rule (one CTA per instance, or a
 cluster of two, four or eight where the batch is small), with keys at every alignment, against the
 oracle byte for byte.  Instance 0 signs a message whose first attempt is singular."""
 import hashlib
@@ -26,13 +26,14 @@ def case(request, cuda):
     sk0, _ = O.keypair(s, 0, 0)
     seeds[0] = np.frombuffer(sk0, np.uint8)
     esk = O.expandsk_batch(s, seeds)
-    epk = O.expandpk_batch(s, O.keypair_from_seed_batch(s, seeds))
+    cpk = O.keypair_from_seed_batch(s, seeds)
+    epk = O.expandpk_batch(s, cpk)
     g = json.load(open(os.path.join(GOLDEN, f"ref_mayo{s}.json")))["rejection"]
     msgs = [rng.integers(0, 256, 32, dtype=np.uint8).tobytes() for _ in range(N)]
     msgs[0] = hashlib.shake_256(f"reject-search/{s}/{g['indices'][0]}".encode()).digest(32)
     sig, attempts = O.sign_batch(s, esk, msgs)
     assert attempts[0] > 0
-    return s, esk, epk, np.frombuffer(b"".join(msgs), np.uint8).reshape(N, 32), sig
+    return s, seeds, esk, epk, np.frombuffer(b"".join(msgs), np.uint8).reshape(N, 32), sig, cpk
 
 
 def _rows(a, stride, off):
@@ -47,7 +48,7 @@ def _rows(a, stride, off):
 @pytest.mark.parametrize("off", [0, 1, 2, 3])
 def test_sign_verify_launch_edges(case, off):
     import torch
-    s, esk, epk, msgs, sig = case
+    s, _, esk, epk, msgs, sig, _ = case
     m = Mayo(s)
     z = m.sizes
     es, ps = z.esk_bytes + 3 * off, z.epk_bytes + off
@@ -66,3 +67,26 @@ def test_sign_verify_launch_edges(case, off):
         torch.cuda.synchronize()
         assert (out[:b].cpu().numpy() == sig[:b]).all() and not out[b:].any(), b
         assert (res[:b].cpu().numpy() == want[:b]).all() and (res[b:] == 0xEE).all(), b
+
+
+@pytest.mark.parametrize("off", [0, 1, 2, 3])
+def test_keypair_expandsk_launch_edges(case, off):
+    import torch
+    s, seeds, esk, _, _, _, cpk = case
+    m = Mayo(s)
+    z = m.sizes
+    kp, ep = z.pitch_keypair + off, z.esk_bytes + off
+    at = (z.sk_bytes + 127) // 128 * 128
+    for b in BATCHES if off == 0 else (1, 13, 73):
+        pool = torch.zeros(off + N * kp, dtype=torch.uint8, device="cuda")[off:]  # ends with the last row
+        rows = pool.view(N, kp)
+        rows[:, : z.sk_bytes] = torch.from_numpy(seeds).cuda()
+        m.crypto_sign_keypair_from_seed(pool, kp, b)
+        epool = torch.zeros(off + N * ep, dtype=torch.uint8, device="cuda")[off:]
+        erows = epool.view(N, ep)
+        erows[:, : z.sk_bytes] = torch.from_numpy(seeds).cuda()
+        m.crypto_sign_expandsk(epool, ep, b)
+        torch.cuda.synchronize()
+        assert (rows[:b, at: at + z.pk_bytes].cpu().numpy() == cpk[:b]).all() and not rows[b:, at:].any(), b
+        assert (erows[:b, : z.esk_bytes].cpu().numpy() == esk[:b]).all() and not erows[b:, z.sk_bytes:].any(), b
+        assert not erows[:, z.esk_bytes:].any(), b
