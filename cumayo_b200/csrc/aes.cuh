@@ -99,11 +99,12 @@ struct AesOut {
 // launch argument for it: a constant-bank operand keeps the address arithmetic an IMAD.
 __constant__ uint32_t c_aes_stride = 128;
 
-// Encrypt counter block `blk` with NTAB replicated round tables in shared memory, 32 KB apart
-// from `base` (the shared-memory address of T0 with this lane's column added):
-//   NTAB = 3: T0, ror8(T0), ror16(T0)   (the expansion kernel, 96 KB)
-//   NTAB = 2: T0, ror16(T0)             (the work queue's keypair where its P3 area holds both)
-//   NTAB = 1: T0                        (the work queue's keypair otherwise)
+// NTAB replicated round tables in shared memory, 32 KB apart from `base` (the shared-memory address
+// of T0 with this lane's column added):
+//   NTAB = 4: T0, ror8(T0), ror16(T0), ror24(T0)   (the expansion kernel, 128 KB)
+//   NTAB = 3: T0, ror8(T0), ror16(T0)   (the work queue's keypair, as many as its P3 area holds)
+//   NTAB = 2: T0, ror16(T0)
+//   NTAB = 1: T0
 // the other round tables by PRMT rotations.  A lookup is a byte extraction, one IMAD for the
 // address (the multiplier `k128` = 128 is a kernel argument or a constant-bank value, so the
 // address arithmetic stays on the IMAD pipe instead of joining the extractions, rotations and
@@ -111,60 +112,96 @@ __constant__ uint32_t c_aes_stride = 128;
 // MAYO_1's 1,024 x 9,031 blocks: one table with PRMT rotations and shifted-index addresses
 // 0.250 ms, IMAD addresses 0.234, two tables 0.222, three tables in two CTAs of 384 threads per
 // SM 0.203 (byte-exact).
-template <int NTAB, class RK>
-__device__ __forceinline__ AesOut aes128_ctr_block_t(uint32_t base, const RK &rk, uint32_t blk, uint32_t k128) {
-    static_assert(NTAB >= 1 && NTAB <= 3, "one to three tables");
-    auto ld = [&](uint32_t x, auto tab) {
-        constexpr int T = decltype(tab)::value;
+template <int NTAB>
+struct AesLut {
+    static_assert(NTAB >= 1 && NTAB <= 4, "one to four tables");
+    uint32_t base, k128;
+    template <int T>
+    __device__ __forceinline__ uint32_t ld(uint32_t x) const {
         uint32_t v;
         if constexpr (T == 0)
             asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(x * k128 + base));
         else if constexpr (T == 1)
             asm volatile("ld.shared.u32 %0, [%1+32768];" : "=r"(v) : "r"(x * k128 + base));
-        else
+        else if constexpr (T == 2)
             asm volatile("ld.shared.u32 %0, [%1+65536];" : "=r"(v) : "r"(x * k128 + base));
+        else
+            asm volatile("ld.shared.u32 %0, [%1+98304];" : "=r"(v) : "r"(x * k128 + base));
         return v;
-    };
-    using I0 = std::integral_constant<int, 0>;
-    using I1 = std::integral_constant<int, 1>;
-    using I2 = std::integral_constant<int, 2>;
-    auto r0 = [&](uint32_t x) { return ld(x, I0{}); };  // T0[x]
-    auto r8 = [&](uint32_t x) {                          // ror8(T0[x])
-        if constexpr (NTAB == 3) return ld(x, I1{});
-        else return ror8(ld(x, I0{}));
-    };
-    auto r16 = [&](uint32_t x) {  // ror16(T0[x])
-        if constexpr (NTAB == 3) return ld(x, I2{});
-        else if constexpr (NTAB == 2) return ld(x, I1{});
-        else return ror16(ld(x, I0{}));
-    };
-    auto r24 = [&](uint32_t x) {  // ror24(T0[x])
-        if constexpr (NTAB == 1) return ror24(ld(x, I0{}));
+    }
+    __device__ __forceinline__ uint32_t r0(uint32_t x) const { return ld<0>(x); }  // T0[x]
+    __device__ __forceinline__ uint32_t r8(uint32_t x) const {                      // ror8(T0[x])
+        if constexpr (NTAB >= 3) return ld<1>(x);
+        else return ror8(ld<0>(x));
+    }
+    __device__ __forceinline__ uint32_t r16(uint32_t x) const {  // ror16(T0[x])
+        if constexpr (NTAB >= 3) return ld<2>(x);
+        else if constexpr (NTAB == 2) return ld<1>(x);
+        else return ror16(ld<0>(x));
+    }
+    __device__ __forceinline__ uint32_t r24(uint32_t x) const {  // ror24(T0[x])
+        if constexpr (NTAB == 4) return ld<3>(x);
+        else if constexpr (NTAB == 1) return ror24(ld<0>(x));
         else return ror8(r16(x));
-    };
-    uint32_t s0 = rk[0], s1 = rk[1], s2 = rk[2], s3 = blk ^ rk[3];
+    }
+    // one output word of a round (without its round key)
+    __device__ __forceinline__ uint32_t mix(uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
+        return r0(a >> 24) ^ r8(byte_of(b, 2)) ^ r16(byte_of(c, 1)) ^ r24(byte_of(d, 0));
+    }
+    // the same of the last round: S-box = byte 1 of T0[x]
+    __device__ __forceinline__ uint32_t last(uint32_t a, uint32_t b, uint32_t c, uint32_t d) const {
+        return __byte_perm(__byte_perm(r0(a >> 24), r0(byte_of(b, 2)), 0x1500),
+                           __byte_perm(r0(byte_of(c, 1)), r0(byte_of(d, 0)), 0x0015), 0x3254);
+    }
+};
+
+// What the first two rounds of 256 consecutive counter blocks share (blk >> 8 the same).  Only byte 15
+// of the input differs between them, so of round 1 only output word a changes, by one lookup, and of
+// round 2 each output word by the one lookup that takes a byte of a: five lookups instead of 32.
+struct AesRun {
+    uint32_t ka, kb, kc, kd;  // round 2 without the bytes of a
+};
+// rk: the round keys (rk[0 .. 11] are read).  a0: word a of round 1 without byte 15's lookup, the same
+// for every run of a key.
+template <int NTAB, class RK>
+__device__ __forceinline__ uint32_t aes_run_a0(const AesLut<NTAB> &t, const RK &rk) {
+    return t.r0(rk[0] >> 24) ^ t.r8(byte_of(rk[1], 2)) ^ t.r16(byte_of(rk[2], 1)) ^ rk[4];
+}
+template <int NTAB, class RK>
+__device__ __forceinline__ AesRun aes_run(const AesLut<NTAB> &t, const RK &rk, uint32_t blk_hi) {
+    const uint32_t s0 = rk[0], s1 = rk[1], s2 = rk[2], s3 = (blk_hi << 8) ^ rk[3];
+    const uint32_t b = t.mix(s1, s2, s3, s0) ^ rk[5], c = t.mix(s2, s3, s0, s1) ^ rk[6], d = t.mix(s3, s0, s1, s2) ^ rk[7];
+    AesRun r;
+    r.ka = t.r8(byte_of(b, 2)) ^ t.r16(byte_of(c, 1)) ^ t.r24(byte_of(d, 0)) ^ rk[8];
+    r.kb = t.r0(b >> 24) ^ t.r8(byte_of(c, 2)) ^ t.r16(byte_of(d, 1)) ^ rk[9];
+    r.kc = t.r0(c >> 24) ^ t.r8(byte_of(d, 2)) ^ t.r24(byte_of(b, 0)) ^ rk[10];
+    r.kd = t.r0(d >> 24) ^ t.r16(byte_of(b, 1)) ^ t.r24(byte_of(c, 0)) ^ rk[11];
+    return r;
+}
+
+// Encrypt counter block `blk` of run `run`: k3 = the low byte of rk[3], rk[i] = round key word 12 + i.
+template <int NTAB, class RK>
+__device__ __forceinline__ AesOut aes128_ctr_block_t(const AesLut<NTAB> &t, uint32_t a0, uint32_t k3, const AesRun &run,
+                                                     const RK &rk, uint32_t blk) {
+    const uint32_t a1 = a0 ^ t.r24(byte_of(blk ^ k3, 0));
+    uint32_t s0 = run.ka ^ t.r0(a1 >> 24), s1 = run.kb ^ t.r24(byte_of(a1, 0)), s2 = run.kc ^ t.r16(byte_of(a1, 1)),
+             s3 = run.kd ^ t.r8(byte_of(a1, 2));
 #pragma unroll
-    for (int r = 1; r < 10; r++) {
-        const uint32_t a = r0(s0 >> 24) ^ r8(byte_of(s1, 2)) ^ r16(byte_of(s2, 1)) ^ r24(byte_of(s3, 0)) ^ rk[4 * r];
-        const uint32_t b = r0(s1 >> 24) ^ r8(byte_of(s2, 2)) ^ r16(byte_of(s3, 1)) ^ r24(byte_of(s0, 0)) ^ rk[4 * r + 1];
-        const uint32_t c = r0(s2 >> 24) ^ r8(byte_of(s3, 2)) ^ r16(byte_of(s0, 1)) ^ r24(byte_of(s1, 0)) ^ rk[4 * r + 2];
-        const uint32_t d = r0(s3 >> 24) ^ r8(byte_of(s0, 2)) ^ r16(byte_of(s1, 1)) ^ r24(byte_of(s2, 0)) ^ rk[4 * r + 3];
+    for (int r = 0; r < 7; r++) {  // rounds 3 .. 9
+        const uint32_t a = t.mix(s0, s1, s2, s3) ^ rk[4 * r];
+        const uint32_t b = t.mix(s1, s2, s3, s0) ^ rk[4 * r + 1];
+        const uint32_t c = t.mix(s2, s3, s0, s1) ^ rk[4 * r + 2];
+        const uint32_t d = t.mix(s3, s0, s1, s2) ^ rk[4 * r + 3];
         s0 = a;
         s1 = b;
         s2 = c;
         s3 = d;
     }
-    // last round: S-box = byte 1 of T0[x]
-#define LASTW(a, b, c, d, k)                                                                   \
-    (__byte_perm(__byte_perm(r0((a) >> 24), r0(byte_of(b, 2)), 0x1500),                         \
-                 __byte_perm(r0(byte_of(c, 1)), r0(byte_of(d, 0)), 0x0015), 0x3254) ^            \
-     rk[k])
     AesOut o;
-    o.w0 = LASTW(s0, s1, s2, s3, 40);
-    o.w1 = LASTW(s1, s2, s3, s0, 41);
-    o.w2 = LASTW(s2, s3, s0, s1, 42);
-    o.w3 = LASTW(s3, s0, s1, s2, 43);
-#undef LASTW
+    o.w0 = t.last(s0, s1, s2, s3) ^ rk[28];
+    o.w1 = t.last(s1, s2, s3, s0) ^ rk[29];
+    o.w2 = t.last(s2, s3, s0, s1) ^ rk[30];
+    o.w3 = t.last(s3, s0, s1, s2) ^ rk[31];
     return o;
 }
 
@@ -193,43 +230,85 @@ __device__ __forceinline__ void st16(uint8_t *p, uint32_t a, uint32_t b, uint32_
 }
 
 // ---------------------------------------------------------------------------------------------
-// Kernel: AES-CTR keystream into a pitched pool.  grid = (chunks, batch); chunk x of instance
-// blockIdx.y takes blocks [x * bpc, min((x + 1) * bpc, nblk_main)) to row + out_off, keyed by 16
-// bytes at row + key_off.  The launcher splits an instance's blocks into near-equal chunks of at
-// most AES_BLOCKS_PER_CTA.  When the key overlaps the output (expand-pk, expand-sk keep seed_pk
-// in the last 16 output bytes until expansion), nblk_main excludes the blocks that overlap the
-// key and aes_ctr_tail_kernel finishes them afterwards, one thread per instance.
+// Kernel: AES-CTR keystream into a pitched pool.  An item is (instance, chunk): chunk x of an instance
+// takes blocks [x * bpc, min((x + 1) * bpc, nblk_main)) to row + out_off, keyed by 16 bytes at row +
+// key_off.  A CTA builds the tables once and takes items blockIdx.x, + gridDim.x, ...; while its
+// worker warps run one item, the last warp prepares the next one (key schedule, the chunk's AesRuns).
+// The workers take the item's blocks 64 at a time from a counter (32 where an item has few).  When the key overlaps the output
+// (expand-pk, expand-sk keep seed_pk in the last 16 output bytes until expansion), nblk_main
+// excludes the blocks that overlap the key and aes_ctr_tail_kernel finishes them afterwards, one
+// thread per instance.
 // ---------------------------------------------------------------------------------------------
-constexpr int AES_THREADS = 384;
-constexpr int AES_BLOCKS_PER_CTA = 3072;
-constexpr size_t AES_SMEM = 3 * 256 * 32 * 4;  // T0, ror8(T0), ror16(T0), each replicated 32 times
+constexpr int AES_WORKERS = 768, AES_THREADS = AES_WORKERS + 32;  // and the warp that prepares
+constexpr int AES_BLOCKS_PER_ITEM = 12288;  // at most
+constexpr int AES_ITEM_COST = 700;          // what an item costs besides its blocks, in blocks (its workers drain)
+constexpr int AES_RUNS = AES_BLOCKS_PER_ITEM / 256 + 2;
+constexpr size_t AES_SMEM = 4 * 256 * 32 * 4;  // T0 and its rotations by 8, 16, 24, each replicated 32 times
 
-static __global__ void __launch_bounds__(AES_THREADS, 2)
+static __global__ void __launch_bounds__(AES_THREADS, 1)
     aes_ctr_kernel(uint8_t *pool, size_t pitch, size_t key_off, size_t out_off, uint32_t nblk_main, uint32_t bpc,
-                   uint32_t k128) {
-    extern __shared__ uint32_t aes_smem[];  // [3][256 * 32] words
-    __shared__ uint32_t rk_s[44];
-    uint8_t *row = pool + (size_t)blockIdx.y * pitch;
-    // warp 0's lane 0 runs the (serial) key schedule while the other warps build the tables
-    if (threadIdx.x == 0) aes128_key_schedule(row + key_off, rk_s);
-    for (int i = (int)threadIdx.x - 32; i < 256 * 32; i += AES_THREADS - 32) {
-        if (i < 0) break;
+                   uint32_t chunks, uint32_t items, uint32_t k128) {
+    extern __shared__ uint32_t aes_smem[];  // [4][256 * 32] words
+    __shared__ uint32_t s_rk[2][44];
+    __shared__ uint4 s_run[2][AES_RUNS];
+    __shared__ uint32_t s_a0[2];
+    __shared__ int s_next[2];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < 256 * 32; i += AES_THREADS) {
         const uint32_t v = c_aes.te0[i >> 5];
         aes_smem[i] = v;
         aes_smem[256 * 32 + i] = ror8(v);
         aes_smem[2 * 256 * 32 + i] = ror16(v);
+        aes_smem[3 * 256 * 32 + i] = ror24(v);
     }
     __syncthreads();
-    uint32_t rk[44];
+    const AesLut<4> lut{(uint32_t)__cvta_generic_to_shared(aes_smem + lane), k128};
+    auto prepare = [&](int buf, uint32_t item) {  // the last warp
+        const uint32_t inst = item / chunks, b0 = (item - inst * chunks) * bpc;
+        if (lane == 0) {
+            aes128_key_schedule(pool + (size_t)inst * pitch + key_off, s_rk[buf]);
+            s_next[buf] = 0;
+        }
+        __syncwarp();
+        const uint32_t *rk = s_rk[buf];
+        const uint32_t runs = ((b0 & 255u) + bpc + 255u) / 256u;
+        for (uint32_t h = (uint32_t)lane; h < runs; h += 32) {
+            const AesRun r = aes_run(lut, rk, (b0 >> 8) + h);
+            s_run[buf][h] = make_uint4(r.ka, r.kb, r.kc, r.kd);
+        }
+        if (lane == 0) s_a0[buf] = aes_run_a0(lut, rk);
+    };
+    constexpr int PREP = AES_WORKERS / 32;
+    if (warp == PREP) prepare(0, blockIdx.x);  // gridDim.x <= items
+    __syncthreads();
+    const uint32_t grab = bpc < 2 * AES_WORKERS ? 32u : 64u;
+    int buf = 0;
+#pragma unroll 1
+    for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, buf ^= 1) {
+        if (warp == PREP) {
+            if (item + gridDim.x < items) prepare(buf ^ 1, item + gridDim.x);
+            __syncthreads();
+            continue;
+        }
+        uint32_t rk[32];
 #pragma unroll
-    for (int i = 0; i < 44; i++) rk[i] = rk_s[i];
-    const uint32_t base = (uint32_t)__cvta_generic_to_shared(aes_smem + (threadIdx.x & 31));
-    uint8_t *out = row + out_off;
-    const uint32_t b0 = blockIdx.x * bpc;
-    const uint32_t b1 = min(b0 + bpc, nblk_main);
-    for (uint32_t blk = b0 + threadIdx.x; blk < b1; blk += AES_THREADS) {
-        AesOut o = aes128_ctr_block_t<3>(base, rk, blk, k128);
-        st16(out + (size_t)blk * 16, bswap32(o.w0), bswap32(o.w1), bswap32(o.w2), bswap32(o.w3));
+        for (int i = 0; i < 32; i++) rk[i] = s_rk[buf][12 + i];
+        const uint32_t a0 = s_a0[buf], k3 = s_rk[buf][3];
+        const uint32_t inst = item / chunks, b0 = (item - inst * chunks) * bpc, b1 = min(b0 + bpc, nblk_main);
+        uint8_t *out = pool + (size_t)inst * pitch + out_off;
+        for (;;) {
+            uint32_t g = 0;
+            if (lane == 0) g = (uint32_t)atomicAdd(&s_next[buf], (int)grab);
+            g = b0 + __shfl_sync(0xffffffffu, g, 0);
+            if (g >= b1) break;
+#pragma unroll 1
+            for (uint32_t blk = g + lane; blk < min(g + grab, b1); blk += 32) {
+                const uint4 r = s_run[buf][(blk >> 8) - (b0 >> 8)];
+                const AesOut o = aes128_ctr_block_t<4>(lut, a0, k3, AesRun{r.x, r.y, r.z, r.w}, rk, blk);
+                st16(out + (size_t)blk * 16, bswap32(o.w0), bswap32(o.w1), bswap32(o.w2), bswap32(o.w3));
+            }
+        }
+        __syncthreads();
     }
 }
 

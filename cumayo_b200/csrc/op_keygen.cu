@@ -93,6 +93,25 @@ __global__ void __launch_bounds__(LCfg<SET, CL>::NT, LCfg<SET, CL>::MINB) l_kern
 // ---------------------------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------------------------
+// Near-equal chunks per instance: the split whose busiest CTA has the least to do, an item counting
+// its blocks and AES_ITEM_COST.  MAYO_1 (9,031 blocks) at 1,024: 207, 185, 181, 177 us with items of
+// at most 1,536, 3,072, 6,400 and 12,288 blocks; MAYO_5 (52,616) at 128: 140 us with 6,400, 150 with
+// 12,288 (640 items on 148 CTAs).
+static uint32_t aes_chunks(uint32_t nblk, size_t batch, uint32_t ctas, uint32_t *bpc) {
+    uint32_t best = 0;
+    uint64_t least = ~0ull;
+    for (uint32_t c = (nblk + AES_BLOCKS_PER_ITEM - 1) / AES_BLOCKS_PER_ITEM; c <= (nblk + AES_WORKERS / 2 - 1) / (AES_WORKERS / 2); c++) {
+        const uint32_t n = (nblk + c - 1) / c;
+        const uint64_t cost = ((uint64_t)batch * c + ctas - 1) / ctas * (n + AES_ITEM_COST);
+        if (cost < least) {
+            least = cost;
+            best = c;
+        }
+    }
+    *bpc = (nblk + best - 1) / best;
+    return best;
+}
+
 static int aes_expand(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, size_t key_off, size_t out_off,
                       uint32_t nbytes, bool key_in_output) {
     // the main kernel writes whole blocks that neither run past nbytes nor touch the key
@@ -101,14 +120,19 @@ static int aes_expand(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st
     const uint32_t nblk = (nbytes + 15) / 16;
     if (nblk_main > 0) {
         if (!set_smem_attr(aes_ctr_kernel, AES_SMEM)) return ST_CUDA;
-        // near-equal chunks of at most AES_BLOCKS_PER_CTA blocks per instance
-        const uint32_t chunks = (nblk_main + AES_BLOCKS_PER_CTA - 1) / AES_BLOCKS_PER_CTA;
-        const uint32_t bpc = (nblk_main + chunks - 1) / chunks;
-        // instances on the grid's y dimension, at most 65,535 per launch
-        for (size_t b0 = 0; b0 < batch; b0 += 65535) {
-            const unsigned nb = (unsigned)(batch - b0 < 65535 ? batch - b0 : 65535);
-            aes_ctr_kernel<<<dim3(chunks, nb), AES_THREADS, AES_SMEM, st>>>(pool + b0 * pitch, pitch, key_off, out_off,
-                                                                             nblk_main, bpc, 128u);
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return ST_CUDA;
+        const uint32_t ctas = (uint32_t)sms;
+        uint32_t bpc = 0;
+        const uint32_t chunks = aes_chunks(nblk_main, batch, ctas, &bpc);
+        // 32-bit item numbers: at most 2^24 instances per launch
+        for (size_t b0 = 0; b0 < batch; b0 += size_t(1) << 24) {
+            const uint32_t nb = (uint32_t)(batch - b0 < (size_t(1) << 24) ? batch - b0 : size_t(1) << 24);
+            const uint32_t items = nb * chunks;
+            aes_ctr_kernel<<<items < ctas ? items : ctas, AES_THREADS, AES_SMEM, st>>>(
+                pool + b0 * pitch, pitch, key_off, out_off, nblk_main, bpc, chunks, items, 128u);
         }
     }
     if (nblk_main < nblk)

@@ -45,10 +45,12 @@ struct QueueCfg<SET, MAYO_B200_OP_KEYPAIR> {
     using KC = KeyCfg<SET>;
     static constexpr int NT = KC::NT, MINB = KC::MINB;
     // as many replicated round tables as the P3 area below O holds (MAYO_1: T0; MAYO_2: T0 and
-    // ror16(T0); MAYO_3/5: all three) and the round keys; dead once the keystream is written
-    static constexpr int ntab(int n) { return KC::off_o >= (size_t)n * 256 * 32 * 4 + 44 * 4; }
-    static constexpr int NTAB = ntab(3) ? 3 : ntab(2) ? 2 : 1;
-    static constexpr size_t aes_end = NTAB * 256 * 32 * 4 + 44 * 4;
+    // ror16(T0); MAYO_3: three; MAYO_5: all four) and the round keys; dead once the keystream is written
+    static constexpr size_t runs = ((size_t)S::p / 16 + 256) / 256 + 1;  // AesRuns of an instance
+    static constexpr size_t aes_bytes(int n) { return (size_t)n * 256 * 32 * 4 + 44 * 4 + 16 * runs; }
+    static constexpr int NTAB = KC::off_o >= aes_bytes(4) ? 4 : KC::off_o >= aes_bytes(3) ? 3 : KC::off_o >= aes_bytes(2) ? 2 : 1;
+    static constexpr size_t run = (size_t)NTAB * 256 * 32 * 4 + 44 * 4;  // after the round keys (16-byte aligned)
+    static constexpr size_t aes_end = aes_bytes(NTAB);
     static_assert(KC::off_o >= aes_end, "O must not overlap the AES tables");
     static constexpr size_t seedpk = KC::off_o + pad16(S::o_bytes);
     static constexpr size_t smem = seedpk + 16;
@@ -212,21 +214,30 @@ __device__ void queue_keypair(uint8_t *smem, int tid, const QueueOps &ops, uint3
         const uint32_t v = c_aes.te0[i >> 5];
         T[i] = v;
         if (NTAB == 2) T[256 * 32 + i] = ror16(v);
-        if (NTAB == 3) {
+        if (NTAB >= 3) {
             T[256 * 32 + i] = ror8(v);
             T[2 * 256 * 32 + i] = ror16(v);
         }
+        if (NTAB == 4) T[3 * 256 * 32 + i] = ror24(v);
     }
     __syncthreads();
     {
-        uint32_t rk[44];
+        const AesLut<NTAB> lut{(uint32_t)__cvta_generic_to_shared(T + (tid & 31)), c_aes_stride};
+        uint4 *s_run = reinterpret_cast<uint4 *>(smem + QC::run);
+        constexpr uint32_t nblk = (S::p + 15) / 16;  // the scratch has room for the whole last block
+        const uint32_t *rks = rk_s;
+        for (uint32_t h = tid; h < (nblk + 255) / 256; h += NT) {
+            const AesRun r = aes_run(lut, rks, h);
+            s_run[h] = make_uint4(r.ka, r.kb, r.kc, r.kd);
+        }
+        const uint32_t a0 = aes_run_a0(lut, rks), k3 = rks[3];
+        uint32_t rk[32];
 #pragma unroll
-        for (int i = 0; i < 44; i++) rk[i] = rk_s[i];
-        const uint32_t base = (uint32_t)__cvta_generic_to_shared(T + (tid & 31));
-        const uint32_t k128 = c_aes_stride;
-        const uint32_t nblk = (S::p + 15) / 16;  // the scratch has room for the whole last block
+        for (int i = 0; i < 32; i++) rk[i] = rk_s[12 + i];
+        __syncthreads();
         for (uint32_t blk = tid; blk < nblk; blk += NT) {
-            const AesOut o = aes128_ctr_block_t<NTAB>(base, rk, blk, k128);
+            const uint4 r = s_run[blk >> 8];
+            const AesOut o = aes128_ctr_block_t<NTAB>(lut, a0, k3, AesRun{r.x, r.y, r.z, r.w}, rk, blk);
             st16(scratch + (size_t)blk * 16, bswap32(o.w0), bswap32(o.w1), bswap32(o.w2), bswap32(o.w3));
         }
     }
