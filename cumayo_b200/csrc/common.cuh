@@ -350,9 +350,11 @@ struct Sponge {
 };
 
 // Warp-cooperative Keccak-f[1600]: lane L < 25 holds lane word A[x + 5y] (x = L % 5, y = L / 5).
-// All 32 lanes must call it (lanes 25..31 carry junk and are ignored).
+// All 32 lanes must call it (lanes 25..31 carry junk and are ignored).  A round is three shuffle
+// stages: the column sums, theta's two neighbours, and chi's three inputs fetched from where pi finds
+// them.
 struct WarpKeccak {
-    int x, src_c0, src_c1, src_pi, src_chi1, src_chi2, rho;
+    int x, src_c0, src_c1, src_b0, src_b1, src_b2, rho;
     __device__ __forceinline__ void setup(int lane) {
         int L = lane < 25 ? lane : 0;
         x = L % 5;
@@ -360,13 +362,20 @@ struct WarpKeccak {
         src_c0 = (x + 4) % 5;  // D[x] = C[x-1] ^ rot(C[x+1], 1)
         src_c1 = (x + 1) % 5;
         // pi: destination (X, Y) = (y, 2x + 3y) pulls from source lane ((X + 3Y) % 5) + 5X
-        src_pi = ((x + 3 * y) % 5) + 5 * x;
-        src_chi1 = (x + 1) % 5 + 5 * y;
-        src_chi2 = (x + 2) % 5 + 5 * y;
+        src_b0 = ((x + 3 * y) % 5) + 5 * x;
+        const int x1 = (x + 1) % 5, x2 = (x + 2) % 5;
+        src_b1 = ((x1 + 3 * y) % 5) + 5 * x1;
+        src_b2 = ((x2 + 3 * y) % 5) + 5 * x2;
         rho = c_keccak_rho[L];
     }
     __device__ __forceinline__ uint64_t rotl_var(uint64_t a, int r) const {
-        return r == 0 ? a : ((a << r) | (a >> (64 - r)));
+        uint32_t lo = (uint32_t)a, hi = (uint32_t)(a >> 32);
+        if (r & 32) {
+            const uint32_t t = lo;
+            lo = hi;
+            hi = t;
+        }
+        return ((uint64_t)__funnelshift_l(lo, hi, r) << 32) | __funnelshift_l(hi, lo, r);
     }
     __device__ uint64_t permute(uint64_t a, int lane) const {
         const unsigned FULL = 0xffffffffu;
@@ -374,38 +383,46 @@ struct WarpKeccak {
         for (int round = 0; round < 24; round++) {
             uint64_t c = __shfl_sync(FULL, a, x) ^ __shfl_sync(FULL, a, x + 5) ^ __shfl_sync(FULL, a, x + 10) ^
                          __shfl_sync(FULL, a, x + 15) ^ __shfl_sync(FULL, a, x + 20);
-            uint64_t d = __shfl_sync(FULL, c, src_c0) ^ rotl64c<1>(__shfl_sync(FULL, c, src_c1));
-            a ^= d;
-            uint64_t b = __shfl_sync(FULL, rotl_var(a, rho), src_pi);
-            a = b ^ (~__shfl_sync(FULL, b, src_chi1) & __shfl_sync(FULL, b, src_chi2));
+            a ^= __shfl_sync(FULL, c, src_c0) ^ rotl64c<1>(__shfl_sync(FULL, c, src_c1));
+            a = rotl_var(a, rho);
+            const uint64_t b0 = __shfl_sync(FULL, a, src_b0), b1 = __shfl_sync(FULL, a, src_b1),
+                           b2 = __shfl_sync(FULL, a, src_b2);
+            a = b0 ^ (~b1 & b2);
             if (lane == 0) a ^= c_keccak_rc[round];
         }
         return a;
     }
 };
 
-// SHAKE over a shared-memory input with the warp-cooperative permutation; output to shared.
-// in_len/out_len in bytes; `in` and `out` must not overlap.
+// Bytes p .. p + n - 1 (n <= 8; none for n <= 0) as a little-endian word, from the aligned 8-byte
+// words that hold them.
+__device__ __forceinline__ uint64_t ld_bytes(const uint8_t *p, int n) {
+    if (n <= 0) return 0;
+    const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 7u);
+    const uint64_t *q = reinterpret_cast<const uint64_t *>(p - off);
+    uint64_t w = q[0] >> (8u * off);
+    if ((int)off + n > 8) w |= q[1] << (64u - 8u * off);
+    return n < 8 ? w & (~0ull >> (64 - 8 * n)) : w;
+}
+
+// A warp's SHAKE sponge over byte strings in any memory space: lane l < RATE / 8 absorbs and squeezes
+// word l of a block.  in_len / out_len in bytes; `in` and `out` must not overlap.
 template <int RATE>
 __device__ void warp_shake(uint8_t *out, int out_len, const uint8_t *in, int in_len, const WarpKeccak &wk,
                            int lane) {
     uint64_t a = 0;
     int off = 0;
     for (;;) {
-        int blk = min(in_len - off, RATE);
-        bool last = (in_len - off) < RATE;
-        uint64_t w = 0;
+        const bool last = (in_len - off) < RATE;
         if (lane < RATE / 8) {
-#pragma unroll
-            for (int b = 0; b < 8; b++) {
-                int pos = lane * 8 + b;
-                uint8_t byte = pos < blk ? in[off + pos] : 0;
-                if (last && pos == blk) byte ^= 0x1F;
-                if (last && pos == RATE - 1) byte ^= 0x80;
-                w |= (uint64_t)byte << (8 * b);
+            const int at = off + lane * 8, n = min(in_len - at, 8);
+            uint64_t w = ld_bytes(in + at, n);
+            if (last) {
+                if (n >= 0 && n < 8) w ^= (uint64_t)0x1F << (8 * n);
+                if (lane == RATE / 8 - 1) w ^= 0x8000000000000000ull;
             }
+            a ^= w;
         }
-        a ^= w;
         if (last) break;
         a = wk.permute(a, lane);
         off += RATE;
@@ -414,10 +431,14 @@ __device__ void warp_shake(uint8_t *out, int out_len, const uint8_t *in, int in_
         a = wk.permute(a, lane);
         __syncwarp();
         if (lane < RATE / 8) {
+            uint8_t *p = out + o + lane * 8;
+            const int n = min(out_len - (o + lane * 8), 8);
+            if (n == 8 && (reinterpret_cast<uintptr_t>(p) & 7) == 0) {
+                *reinterpret_cast<uint64_t *>(p) = a;
+            } else {
 #pragma unroll
-            for (int b = 0; b < 8; b++) {
-                int pos = o + lane * 8 + b;
-                if (pos < out_len) out[pos] = (uint8_t)(a >> (8 * b));
+                for (int b = 0; b < 8; b++)
+                    if (b < n) p[b] = (uint8_t)(a >> (8 * b));
             }
         }
     }

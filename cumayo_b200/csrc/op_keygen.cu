@@ -11,7 +11,8 @@
 namespace mayo {
 
 // ---------------------------------------------------------------------------------------------
-// Hash kernels: one thread per instance, Keccak state in registers.
+// Hash kernels: one thread per instance, Keccak state in registers; or, for batches up to
+// HASH_WARP_MAX, one warp per instance.
 // ---------------------------------------------------------------------------------------------
 // keypair: seed_sk = SHAKE128(LE64(rand_index + 2*inst + 1), SK) (src/keypair.cu:35-45) unless
 // `seeded`; then seed_pk || O = SHAKE256(seed_sk) (src/keypair.cu:47-50).  seed_pk goes to pk[0:16];
@@ -57,6 +58,47 @@ __global__ void expandsk_hash_kernel(uint8_t *pool, size_t pitch, uint32_t batch
     sp.finalize();
     sp.squeeze(row + S::sk + S::o_bytes + S::p - 16, 16);
     sp.squeeze(row + S::sk, S::o_bytes);
+}
+
+// The same with a warp per instance.
+constexpr int HASH_WARPS = 4;
+template <int SET>
+__global__ void __launch_bounds__(32 * HASH_WARPS)
+    keypair_hash_warp_kernel(uint8_t *pool, size_t pitch, uint32_t batch, uint64_t rand_index, int seeded) {
+    using S = Set<SET>;
+    __shared__ uint64_t s_buf[HASH_WARPS][8];  // the counter, the seed
+    const int lane = threadIdx.x & 31;
+    const uint32_t inst = blockIdx.x * HASH_WARPS + (threadIdx.x >> 5);
+    if (inst >= batch) return;
+    uint8_t *row = pool + (size_t)inst * pitch, *pk = row + align128(S::sk);
+    uint64_t *buf = s_buf[threadIdx.x >> 5];
+    const uint8_t *sk = row;
+    WarpKeccak wk;
+    wk.setup(lane);
+    if (!seeded) {
+        if (lane == 0) buf[0] = rand_index + (uint64_t)(uint32_t)(2u * inst) + 1;
+        __syncwarp();
+        uint8_t *seed = reinterpret_cast<uint8_t *>(buf + 1);
+        warp_shake<168>(seed, S::sk, reinterpret_cast<const uint8_t *>(buf), 8, wk, lane);
+        for (int i = lane; i < S::sk; i += 32) row[i] = seed[i];
+        sk = seed;
+    }
+    warp_shake<136>(pk, 16 + S::o_bytes, sk, S::sk, wk, lane);
+}
+
+template <int SET>
+__global__ void __launch_bounds__(32 * HASH_WARPS) expandsk_hash_warp_kernel(uint8_t *pool, size_t pitch, uint32_t batch) {
+    using S = Set<SET>;
+    __shared__ uint64_t s_out[HASH_WARPS][(16 + S::o_bytes + 7) / 8];
+    const int lane = threadIdx.x & 31;
+    const uint32_t inst = blockIdx.x * HASH_WARPS + (threadIdx.x >> 5);
+    if (inst >= batch) return;
+    uint8_t *row = pool + (size_t)inst * pitch, *out = reinterpret_cast<uint8_t *>(s_out[threadIdx.x >> 5]);
+    WarpKeccak wk;
+    wk.setup(lane);
+    warp_shake<136>(out, 16 + S::o_bytes, row, S::sk, wk, lane);
+    if (lane < 16) row[S::sk + S::o_bytes + S::p - 16 + lane] = out[lane];
+    for (int i = lane; i < S::o_bytes; i += 32) row[S::sk + i] = out[16 + i];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -161,8 +203,12 @@ static int l_cl(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st) {
 template <int SET>
 static int keypair_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, uint64_t rand_index, bool seeded) {
     using S = Set<SET>;
-    keypair_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch, rand_index,
-                                                                                 seeded ? 1 : 0);
+    if (batch <= HASH_WARP_MAX)
+        keypair_hash_warp_kernel<SET><<<(unsigned)((batch + HASH_WARPS - 1) / HASH_WARPS), 32 * HASH_WARPS, 0, st>>>(
+            pool, pitch, (uint32_t)batch, rand_index, seeded ? 1 : 0);
+    else
+        keypair_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch,
+                                                                                     rand_index, seeded ? 1 : 0);
     const size_t pk_off = align128(S::sk);
     int rc = aes_expand(pool, pitch, batch, st, pk_off, pk_off + align128(S::pk), S::p, false);
     if (rc) return rc;
@@ -177,7 +223,11 @@ static int keypair_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st,
 template <int SET>
 static int expandsk_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st) {
     using S = Set<SET>;
-    expandsk_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch);
+    if (batch <= HASH_WARP_MAX)
+        expandsk_hash_warp_kernel<SET><<<(unsigned)((batch + HASH_WARPS - 1) / HASH_WARPS), 32 * HASH_WARPS, 0, st>>>(
+            pool, pitch, (uint32_t)batch);
+    else
+        expandsk_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch);
     const size_t out_off = S::sk + S::o_bytes;
     int rc = aes_expand(pool, pitch, batch, st, out_off + S::p - 16, out_off, S::p, true);
     if (rc) return rc;

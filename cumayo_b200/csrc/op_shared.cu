@@ -223,11 +223,12 @@ __global__ void __launch_bounds__(ORD_NT)
     ord_chunk(batch, b0, b1);
     for (uint32_t i = b0 + threadIdx.x; i < b1; i += ORD_NT) order[atomicAdd(&cur[msg_bin(m, i)], 1u)] = i;
 }
-// The order for a call, or nullptr when every message has the same length (nothing to group).
+// The order for a call, or nullptr when every message has the same length (nothing to group) or a
+// warp hashes each instance.
 template <int SET, bool VERIFY>
 static const uint32_t *launch_hash_order(const MsgIO &m, uint8_t *ws, size_t batch, cudaStream_t st) {
     using WSL = SharedWs<SET, VERIFY>;
-    if (!m.msg_len || batch < 2 * (size_t)HASH_NT) return nullptr;
+    if (!m.msg_len || batch <= HASH_WARP_MAX) return nullptr;
     const size_t want = (batch + ORD_NT - 1) / ORD_NT;
     const unsigned g = (unsigned)(want < (size_t)ORD_CTAS ? want : (size_t)ORD_CTAS);
     uint32_t *hist = reinterpret_cast<uint32_t *>(ws + WSL::hist_off());
@@ -994,6 +995,27 @@ __global__ void verify_hash_kernel(const VerifyIO io, uint8_t *tws, size_t tws_s
     for (int i = S::menc; i < (S::menc + 3) / 4 * 4; i++) t[i] = 0;
 }
 
+// The same with a warp per instance.
+constexpr int VERIFY_HASH_WARPS = 4;
+template <int SET>
+__global__ void __launch_bounds__(32 * VERIFY_HASH_WARPS)
+    verify_hash_warp_kernel(const VerifyIO io, uint8_t *tws, size_t tws_stride, uint32_t batch) {
+    using S = Set<SET>;
+    __shared__ uint64_t s_key[VERIFY_HASH_WARPS][(S::digest + S::sk) / 8];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t inst = blockIdx.x * VERIFY_HASH_WARPS + w;
+    if (inst >= batch) return;
+    uint8_t *key = reinterpret_cast<uint8_t *>(s_key[w]), *t = tws + (size_t)inst * tws_stride;
+    WarpKeccak wk;
+    wk.setup(lane);
+    warp_shake<136>(key, S::digest, io.m.ptr(inst), (int)io.m.len(inst), wk, lane);
+    const uint8_t *salt = io.sig + (size_t)inst * io.sig_stride + S::k * S::n / 2;
+    for (int i = lane; i < S::sk; i += 32) key[S::digest + i] = salt[i];
+    for (int i = S::menc + lane; i < (S::menc + 3) / 4 * 4; i += 32) t[i] = 0;
+    __syncwarp();
+    warp_shake<136>(t, S::menc, key, S::digest + S::sk, wk, lane);
+}
+
 // U_ij = s_i^T T_j from the planes, y = Horner over the pairs, compare with t.  No engine
 // staging, no hashing: a small CTA.
 template <int SET>
@@ -1229,8 +1251,12 @@ static int verify_shared_t(const VerifyIO &io0, uint8_t *ws, size_t batch, cudaS
     tmark(st);
     const uint32_t *order = launch_hash_order<SET, true>(io.m, ws, batch, st);
     const int hnt = g_shape[shape_index(SET)].hash_nt.load(std::memory_order_relaxed);
-    verify_hash_kernel<SET><<<(unsigned)((batch + hnt - 1) / hnt), hnt, 0, st>>>(io, tws, WSL::inst, (uint32_t)batch,
-                                                                             order);
+    if (batch <= HASH_WARP_MAX)
+        verify_hash_warp_kernel<SET><<<(unsigned)((batch + VERIFY_HASH_WARPS - 1) / VERIFY_HASH_WARPS),
+                                       32 * VERIFY_HASH_WARPS, 0, st>>>(io, tws, WSL::inst, (uint32_t)batch);
+    else
+        verify_hash_kernel<SET><<<(unsigned)((batch + hnt - 1) / hnt), hnt, 0, st>>>(io, tws, WSL::inst,
+                                                                                 (uint32_t)batch, order);
     tmark(st);
     int rc = launch_product<SET, true>(io.epk, io.sig, io.sig_stride, ws, batch, st);
     if (rc != ST_OK) return rc;

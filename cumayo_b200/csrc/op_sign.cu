@@ -65,6 +65,37 @@ __global__ void sign_hash_kernel(const SignIO io, uint32_t batch, const uint32_t
     }
 }
 
+// The same with a warp per instance.
+constexpr int SIGN_HASH_WARPS = 4;
+template <int SET>
+__global__ void __launch_bounds__(32 * SIGN_HASH_WARPS) sign_hash_warp_kernel(const SignIO io, uint32_t batch) {
+    using S = Set<SET>;
+    using WS = SignWs<SET>;
+    constexpr int KEY = S::digest + 2 * S::sk + 1;  // digest || salt (0 at first) || seed_sk || ctr = 0
+    __shared__ uint64_t s_key[SIGN_HASH_WARPS][(KEY + 7) / 8], s_salt[SIGN_HASH_WARPS][S::sk / 8];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t inst = blockIdx.x * SIGN_HASH_WARPS + w;
+    if (inst >= batch) return;
+    const uint8_t *seed_sk = io.esk + (size_t)inst * io.esk_stride;
+    uint8_t *ws = io.ws + (size_t)inst * io.ws_stride;
+    uint8_t *key = reinterpret_cast<uint8_t *>(s_key[w]), *salt = reinterpret_cast<uint8_t *>(s_salt[w]);
+    WarpKeccak wk;
+    wk.setup(lane);
+    for (int i = lane; i < S::sk; i += 32) {
+        key[S::digest + i] = 0;
+        key[S::digest + S::sk + i] = seed_sk[i];
+    }
+    if (lane == 0) key[KEY - 1] = 0;
+    warp_shake<136>(key, S::digest, io.m.ptr(inst), (int)io.m.len(inst), wk, lane);  // sign.cu:225
+    warp_shake<136>(salt, S::sk, key, S::digest + 2 * S::sk, wk, lane);              // sign.cu:230-238
+    for (int i = lane; i < S::sk; i += 32) key[S::digest + i] = salt[i];
+    __syncwarp();
+    warp_shake<136>(ws + WS::t, S::menc, key, S::digest + S::sk, wk, lane);  // sign.cu:240-243
+    warp_shake<136>(ws + WS::vr, S::vr, key, KEY, wk, lane);                 // sign.cu:250-252
+    static_assert(WS::dig == 0 && WS::salt == S::digest, "digest and salt lie as in the key");
+    for (int i = lane; i < S::digest + S::sk; i += 32) ws[i] = key[i];
+}
+
 template <int SET, int CL>
 __global__ void __launch_bounds__(SignCfg<SET, CL>::NT, SignCfg<SET, CL>::MINB) sign_kernel(const SignIO io) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -98,8 +129,8 @@ static int sign_cl(const SignIO &io, size_t batch, cudaStream_t st) {
 
 template <int SET>
 static int sign_t(const SignIO &io, size_t batch, cudaStream_t st) {
-    sign_hash_kernel<SET><<<(unsigned)((batch + HASH_NT - 1) / HASH_NT), HASH_NT, 0, st>>>(io, (uint32_t)batch, nullptr);
-    if (cudaPeekAtLastError() != cudaSuccess) return ST_CUDA;
+    const int rc = launch_sign_hash(SET, io, batch, st);
+    if (rc != ST_OK) return rc;
     switch (cluster_ctas(batch)) {
         case 8: return sign_cl<SET, 8>(io, batch, st);
         case 4: return sign_cl<SET, 4>(io, batch, st);
@@ -108,15 +139,22 @@ static int sign_t(const SignIO &io, size_t batch, cudaStream_t st) {
     }
 }
 
+template <int SET>
+static void sign_hash_t(const SignIO &io, size_t batch, cudaStream_t st, const uint32_t *order, int nt) {
+    if (batch <= HASH_WARP_MAX)
+        sign_hash_warp_kernel<SET><<<(unsigned)((batch + SIGN_HASH_WARPS - 1) / SIGN_HASH_WARPS), 32 * SIGN_HASH_WARPS,
+                                     0, st>>>(io, (uint32_t)batch);
+    else
+        sign_hash_kernel<SET><<<(unsigned)((batch + nt - 1) / nt), nt, 0, st>>>(io, (uint32_t)batch, order);
+}
+
 int launch_sign_hash(int set, const SignIO &io, size_t batch, cudaStream_t st, const uint32_t *order, int nt) {
     if (batch == 0) return ST_OK;
-    const unsigned g = (unsigned)((batch + nt - 1) / nt);
-    const uint32_t b = (uint32_t)batch;
     switch (set) {
-        case 1: sign_hash_kernel<1><<<g, nt, 0, st>>>(io, b, order); break;
-        case 2: sign_hash_kernel<2><<<g, nt, 0, st>>>(io, b, order); break;
-        case 3: sign_hash_kernel<3><<<g, nt, 0, st>>>(io, b, order); break;
-        case 5: sign_hash_kernel<5><<<g, nt, 0, st>>>(io, b, order); break;
+        case 1: sign_hash_t<1>(io, batch, st, order, nt); break;
+        case 2: sign_hash_t<2>(io, batch, st, order, nt); break;
+        case 3: sign_hash_t<3>(io, batch, st, order, nt); break;
+        case 5: sign_hash_t<5>(io, batch, st, order, nt); break;
         default: return ST_BAD_SET;
     }
     return cudaPeekAtLastError() == cudaSuccess ? ST_OK : ST_CUDA;

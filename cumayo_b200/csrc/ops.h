@@ -12,6 +12,11 @@ namespace mayo {
 // Threads per CTA of the thread-per-instance hash kernels: their registers allow 8 such CTAs per
 // SM, so small CTAs spread a batch evenly over the 148 SMs (whole waves).
 constexpr int HASH_NT = 64;
+// Batches up to this are hashed by a warp per instance: a thread's Keccak-f takes about 5 us however
+// few there are, a warp's 2.4 us, and a batch of a few thousand warps still fits the GPU.  Sign hash,
+// us, warp against thread per instance (MAYO_1 / 5): one instance 29 / 45 against 51 / 90, 1,024
+// 38 / 57 against 86 / 150, 2,048 51 / 79 against 87 / 152, 4,096 78 / 122 against 88 / 150.
+constexpr size_t HASH_WARP_MAX = 2048;
 
 // Status codes shared with include/mayo_b200.h.
 enum : int {
