@@ -141,7 +141,7 @@ __device__ __forceinline__ void p3_instance(uint8_t *smem, int tid, const uint8_
         const TriRows<SET> rows{mis, (uint32_t)(4 * q), r0,
                                 RO && tl <= (chunk * 32 + 31) / NQ ? 4 * (rank + tl * NP) + (lane & 3) : S::v};
         quad_columns<SET, J, RO, 1>(acc, rows, base4, QuadCfg<SET>::bytes(q), c_lo + len * piece / C::PC,
-                                    c_lo + len * (piece + 1) / C::PC, 4 * qmax + 4, masks);
+                                    c_lo + len * (piece + 1) / C::PC, 4 * qmax + 4, masks, mis == 0);
         const uint32_t rm = quad_row_mask(r0, S::v);
 #pragma unroll
         for (int j = 0; j < J; j++) {
@@ -237,6 +237,7 @@ __device__ __forceinline__ void l_instance(uint8_t *smem, int tid, const uint8_t
     const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(P1) & 3);
     const uint32_t *base4 = reinterpret_cast<const uint32_t *>(P1 - mis);
     if (tid == 0) *s_next = 0;
+    if constexpr (CL == 1) l2_prefetch_range(base4, mis, S::p1, tid, NT);  // read by rows and by columns
     build_masks9<J>(reinterpret_cast<uint32_t *>(masks), S::v, tid, NT,
                     [&](int c, int j) { return o_nibble<SET>(s_O, c, j); });
     __syncthreads();
@@ -252,7 +253,7 @@ __device__ __forceinline__ void l_instance(uint8_t *smem, int tid, const uint8_t
         for (int seg = 0; seg < 2; seg++) {  // from the diagonal on, then the columns left of every row
             rows.lower = seg == 1;
             quad_columns<SET, J, true, 1>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? 0 : 4 * qmin,
-                                          seg ? 4 * qmin : S::v, seg ? 0 : 4 * qmax + 4, masks);
+                                          seg ? 4 * qmin : S::v, seg ? 0 : 4 * qmax + 4, masks, mis == 0);
         }
 #pragma unroll
         for (int j = 0; j < J; j++) {

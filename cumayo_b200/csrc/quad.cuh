@@ -125,16 +125,18 @@ template <bool RO>
 __device__ __forceinline__ uint32_t ld_word(const uint32_t *p) {
     return RO ? __ldg(p) : __ldca(p);
 }
-template <bool RO, bool SAFE>
+// AL: every word is 4-byte aligned (whole words: n is 4).
+template <bool RO, bool SAFE, bool AL = false>
 __device__ __forceinline__ RawWord ld_raw(const uint32_t *base4, uint32_t bit, int n) {
     const uint32_t *p = base4 + (bit >> 5);
     RawWord r;
     r.lo = ld_word<RO>(p);
-    r.hi = !SAFE || (int)((bit >> 3) & 3u) + n > 4 ? ld_word<RO>(p + 1) : 0u;
+    r.hi = AL ? 0u : !SAFE || (int)((bit >> 3) & 3u) + n > 4 ? ld_word<RO>(p + 1) : 0u;
     return r;
 }
+template <bool AL = false>
 __device__ __forceinline__ uint32_t raw_value(const RawWord &r, uint32_t bit) {
-    return __funnelshift_r(r.lo, r.hi, bit);
+    return AL ? r.lo : __funnelshift_r(r.lo, r.hi, bit);
 }
 
 // Ask L2 for bytes [at, at + n) from base4 (n > 0), rounded out to 16-byte units, each of which
@@ -192,8 +194,8 @@ __device__ __forceinline__ void l2_prefetch_range(const uint32_t *base4, uint32_
 // products of column c.  All lanes of a warp must pass the same c0, c1 and c_chk.
 // Three loops, so that the long one (every row has an entry, no column is the last) has no tests.
 constexpr int QUAD_AHEAD = 16;  // columns per L2 request
-template <int SET, int JB, bool RO, int D, class Rows>
-__device__ __forceinline__ void quad_columns(QuadAcc<JB> &acc, const Rows &rows, const uint32_t *base4, int n, int c0,
+template <int SET, int JB, bool RO, int D, bool AL, class Rows>
+__device__ __forceinline__ void quad_columns_t(QuadAcc<JB> &acc, const Rows &rows, const uint32_t *base4, int n, int c0,
                                              int c1, int c_chk, const uint4 *masks) {
     if (c0 >= c1) return;
     const uint32_t two = c_quad_mul[0], four = c_quad_mul[1];
@@ -206,12 +208,12 @@ __device__ __forceinline__ void quad_columns(QuadAcc<JB> &acc, const Rows &rows,
     for (int d = 0; d < D; d++) {
         if (d > 0 && c0 + d < c1) rows.next(bl, c0 + d);
 #pragma unroll
-        for (int i = 0; i < 4; i++) raw[d][i] = ld_raw<RO, true>(base4, bl[i], n);
+        for (int i = 0; i < 4; i++) raw[d][i] = ld_raw<RO, true, AL>(base4, bl[i], n);
     }
     const uint4 *mp = masks + (size_t)c0 * QuadAcc<JB>::ST;
     auto take = [&] {
 #pragma unroll
-        for (int i = 0; i < 4; i++) w[i] = raw_value(raw[0][i], bit[i]);
+        for (int i = 0; i < 4; i++) w[i] = raw_value<AL>(raw[0][i], bit[i]);
 #pragma unroll
         for (int d = 0; d + 1 < D; d++)
 #pragma unroll
@@ -219,7 +221,7 @@ __device__ __forceinline__ void quad_columns(QuadAcc<JB> &acc, const Rows &rows,
     };
     auto load_last = [&] {  // column c + D, not the last of the range
 #pragma unroll
-        for (int i = 0; i < 4; i++) raw[D - 1][i] = ld_raw<RO, false>(base4, bl[i], n);
+        for (int i = 0; i < 4; i++) raw[D - 1][i] = ld_raw<RO, false, AL>(base4, bl[i], n);
     };
     auto products = [&] {
         uint32_t f[NFORM];
@@ -260,11 +262,22 @@ __device__ __forceinline__ void quad_columns(QuadAcc<JB> &acc, const Rows &rows,
         if (c + D < c1) {
             rows.next(bl, c + D);
 #pragma unroll
-            for (int i = 0; i < 4; i++) raw[D - 1][i] = ld_raw<RO, true>(base4, bl[i], n);
+            for (int i = 0; i < 4; i++) raw[D - 1][i] = ld_raw<RO, true, AL>(base4, bl[i], n);
         }
         rows.next(bit, c + 1);
         products();
     }
+}
+
+// m-vectors of whole words (MAYO_2: 32 bytes) from a 4-byte aligned key need one load per word and no
+// shift.
+template <int SET, int JB, bool RO, int D, class Rows>
+__device__ __forceinline__ void quad_columns(QuadAcc<JB> &acc, const Rows &rows, const uint32_t *base4, int n, int c0,
+                                             int c1, int c_chk, const uint4 *masks, bool aligned) {
+    if (Set<SET>::menc % 4 == 0 && aligned)
+        quad_columns_t<SET, JB, RO, D, Set<SET>::menc % 4 == 0>(acc, rows, base4, n, c0, c1, c_chk, masks);
+    else
+        quad_columns_t<SET, JB, RO, D, false>(acc, rows, base4, n, c0, c1, c_chk, masks);
 }
 
 // Rows r0 .. r0 + 3 of [[P1, P2], [0, P3]] (n x n), the matrix p bytes from base4; word q.  row_l:

@@ -92,7 +92,7 @@ struct SignCfg {
     static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;
     static constexpr int CH2 = (J * NQ + 31) / 32;
     static constexpr int P2 = CH2 >= CW ? (SET == 5 ? 3 : 1) : (CW + CH2 - 1) / CH2;
-    static constexpr int D = SET == 3 ? 2 : 1;
+    static constexpr int D = SET == 3 || SET == 2 ? 2 : 1;
     static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 2 ? 6 : SET == 3 ? 2 : 1);
     // slots of T a part needs: its quads of P1 (a chunk's last lanes write past them)
     static constexpr int TU = CH * 32;
@@ -401,7 +401,7 @@ __device__ __forceinline__ bool sign_products(uint8_t *smem, int tid, const uint
             const SignRows<SET> rows{p1, (uint32_t)(4 * q), x,
                                      tl <= (chunk * 32 + 31) / NQ ? 4 * (part + tl * NP - MQ) + (lane & 3) : -1};
             quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), c_lo + len * piece / C::PC,
-                                             c_lo + len * (piece + 1) / C::PC, c_chk, masks);
+                                             c_lo + len * (piece + 1) / C::PC, c_chk, masks, p1 % 4 == 0);
             if (x < MQ) {
 #pragma unroll
                 for (int j = 0; j < J; j++) {  // M_j[4 x + i], word q

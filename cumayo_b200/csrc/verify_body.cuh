@@ -34,9 +34,9 @@ struct VerifyCfg {
     static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;
     static constexpr int CH2 = (J * NQ + 31) / 32;   // chunks of (j, word) pairs
     static constexpr int P2 = CH2 >= CW ? (SET == 5 ? 3 : 1) : (CW + CH2 - 1) / CH2;  // quad ranges of each
-    // columns loaded ahead: two where two CTAs per SM leave the registers (MAYO_3 0.467 -> 0.427 us
-    // per instance); MAYO_1 at three CTAs of 168 registers is slower with two (0.153 -> 0.180)
-    static constexpr int D = SET == 3 ? 2 : 1;
+    // columns loaded ahead: two where the registers are there (MAYO_3 0.467 -> 0.427 us per instance,
+    // MAYO_2 0.067 -> 0.064); MAYO_1 at three CTAs of 168 registers is slower with two (0.153 -> 0.180)
+    static constexpr int D = SET == 3 || SET == 2 ? 2 : 1;
     static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 2 ? 6 : SET == 3 ? 2 : 1);
     static constexpr size_t off_masks = 0;
     static constexpr size_t sz_masks = (size_t)S::n * ST * 16;
@@ -136,7 +136,7 @@ __device__ __forceinline__ void verify_instance(uint8_t *smem, int tid, const ui
 #pragma unroll 1
             for (int seg = 0; seg < 2; seg++)  // P1's columns, then P2's and P3's
                 quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? max(ca, S::v) : ca,
-                                           seg ? cb : min(cb, S::v), c_chk, masks);
+                                           seg ? cb : min(cb, S::v), c_chk, masks, mis == 0);
             const uint32_t rm = quad_row_mask(r0, S::n);
 #pragma unroll
             for (int j = 0; j < J; j++) {
