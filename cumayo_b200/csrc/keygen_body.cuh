@@ -20,13 +20,14 @@ struct KeyCfg {
     // Warps and CTAs per SM, keypairs at 2,072 (us per instance): MAYO_1 three CTAs of four warps 0.321
     // against 0.330 with four CTAs (128 registers, spills); MAYO_2 (153 accumulators) two warps 0.312
     // against 0.322 with four and 0.486 with three CTAs of three warps (spills); MAYO_3 two CTAs of
-    // six warps 0.796 against 0.809 with four warps and two columns ahead; MAYO_5 one CTA of eleven
-    // warps 1.910 against 2.003 with six.
-    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 2 : SET == 3 ? 6 : 11);
+    // six warps 0.796 against 0.809 with four warps and two columns ahead (then 0.698; eight warps in one CTA 0.729);
+    // MAYO_5 one CTA of eight warps, two columns ahead, 1.55 against 1.69 with eleven, one ahead.
+    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 2 : SET == 3 ? 6 : 8);
     static constexpr int NT = 32 * CW;
     static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;
     static constexpr int CH2 = (J * NQ + 31) / 32;
-    static constexpr int P2 = CH2 >= CW ? (SET == 5 ? 3 : 1) : (CW + CH2 - 1) / CH2;
+    static constexpr int P2 = CH2 >= CW || (CL == 1 && SET == 5) ? 1 : (CW + CH2 - 1) / CH2;
+    static constexpr int D = SET == 5 ? 2 : 1;  // columns loaded ahead
     static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 5 ? 1 : 2);
     static constexpr int TRI = S::o * (S::o + 1) / 2;
     static constexpr size_t off_masks = 0;
@@ -140,7 +141,7 @@ __device__ __forceinline__ void p3_instance(uint8_t *smem, int tid, const uint8_
         acc.zero();
         const TriRows<SET> rows{mis, (uint32_t)(4 * q), r0,
                                 RO && tl <= (chunk * 32 + 31) / NQ ? 4 * (rank + tl * NP) + (lane & 3) : S::v};
-        quad_columns<SET, J, RO, 1>(acc, rows, base4, QuadCfg<SET>::bytes(q), c_lo + len * piece / C::PC,
+        quad_columns<SET, J, RO, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), c_lo + len * piece / C::PC,
                                     c_lo + len * (piece + 1) / C::PC, 4 * qmax + 4, masks, mis == 0);
         const uint32_t rm = quad_row_mask(r0, S::v);
 #pragma unroll
@@ -183,10 +184,12 @@ struct LCfg {
     static constexpr int CL = CL_, J = S::o, NQ = QuadCfg<SET>::NQ, ST = QuadAcc<J>::ST;
     static constexpr int QN = (S::v + 3) / 4, CH = (QN * NQ + 31) / 32;  // chunks, every one v columns long
     // expand-sk at 2,072 (us per instance): MAYO_1 0.410 with three CTAs per SM, 0.424 with four (128
-    // registers); MAYO_2 0.327 with four warps, 0.344 with two; MAYO_5 2.61 with eleven warps, 2.76
-    // with two CTAs of six, 2.83 with seven warps
-    static constexpr int CW = CL > 1 ? (CH + CL - 1) / CL : (SET == 1 ? 4 : SET == 2 ? 4 : SET == 3 ? 6 : 11);
+    // registers); MAYO_2 0.327 with four warps, 0.344 with two; MAYO_3 0.901 with two CTAs of six warps,
+    // 1.02 with eight warps, two columns ahead; MAYO_5 2.27 with eight warps, two ahead, 2.40 with
+    // eleven, one ahead
+    static constexpr int CW = CL > 1 ? (CH + CL - 1) / CL : (SET == 1 ? 4 : SET == 2 ? 4 : SET == 3 ? 6 : 8);
     static constexpr int NT = 32 * CW;
+    static constexpr int D = SET == 5 ? 2 : 1;  // columns loaded ahead
     static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 5 ? 1 : 2);
     static constexpr size_t off_masks = 0;
     static constexpr size_t off_o = (size_t)S::v * ST * 16;
@@ -252,7 +255,7 @@ __device__ __forceinline__ void l_instance(uint8_t *smem, int tid, const uint8_t
 #pragma unroll 1
         for (int seg = 0; seg < 2; seg++) {  // from the diagonal on, then the columns left of every row
             rows.lower = seg == 1;
-            quad_columns<SET, J, true, 1>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? 0 : 4 * qmin,
+            quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? 0 : 4 * qmin,
                                           seg ? 4 * qmin : S::v, seg ? 0 : 4 * qmax + 4, masks, mis == 0);
         }
 #pragma unroll

@@ -319,6 +319,7 @@ struct PubRows {
 
 // The next work item of a CTA's counter, for a whole warp (a uniform value).
 __device__ __forceinline__ int warp_next(int *counter, int lane) {
+    __syncwarp();
     return (int)__reduce_or_sync(0xffffffffu, lane == 0 ? (uint32_t)atomicAdd(counter, 1) : 0u);
 }
 

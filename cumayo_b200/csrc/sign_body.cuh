@@ -75,7 +75,8 @@ struct SignTailCfg {
 };
 
 // The CTA, or cluster of CL CTAs, of a signature under its own key.  The quads -- MQ of columns of L,
-// then UQ of rows of P1 -- are dealt out to NP parts as in VerifyCfg.
+// then UQ of rows of P1 -- are dealt out to NP parts, quad x to part x % NP: the
+// CTAs of a cluster, or NR rounds of one CTA.
 template <int SET_, int CL_ = 1>
 struct SignCfg {
     static constexpr int SET = SET_;
@@ -83,16 +84,20 @@ struct SignCfg {
     static constexpr bool CP = false;
     static constexpr int J = S::k, W = S::W, NQ = QuadCfg<SET>::NQ, ST = QuadAcc<J>::ST, CL = CL_;
     static constexpr int MQ = (S::o + 3) / 4, UQ = (S::v + 3) / 4, QN = MQ + UQ;
+    // MAYO_3 on one CTA: two parts one after the other, so that T leaves room for two CTAs per SM and one
+    // CTA's tail runs beside the other's products (sign at 2,072: 1.39 ms against 1.58 with one CTA
+    // of 8 warps; MAYO_5, whose CTA fills the SM either way: 8 warps and two columns ahead 2.63 ms,
+    // 11 and one ahead 3.15)
     static constexpr int NR = CL > 1 ? 1 : (SET == 3 ? 2 : 1);
     static constexpr int NP = CL * NR;
     static constexpr int QL = (QN + NP - 1) / NP;
     static constexpr int CH = (QL * NQ + 31) / 32;
-    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 3 : SET == 3 ? 4 : 11);
+    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 3 : SET == 3 ? 4 : 8);
     static constexpr int NT = 32 * CW;
     static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;
     static constexpr int CH2 = (J * NQ + 31) / 32;
-    static constexpr int P2 = CH2 >= CW ? (SET == 5 ? 3 : 1) : (CW + CH2 - 1) / CH2;
-    static constexpr int D = SET == 3 || SET == 2 ? 2 : 1;
+    static constexpr int P2 = CH2 >= CW || (CL == 1 && SET == 5) ? 1 : (CW + CH2 - 1) / CH2;
+    static constexpr int D = SET == 1 ? 1 : 2;
     static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 2 ? 6 : SET == 3 ? 2 : 1);
     // slots of T a part needs: its quads of P1 (a chunk's last lanes write past them)
     static constexpr int TU = CH * 32;

@@ -32,7 +32,7 @@ def case(request, cuda):
     msgs = [rng.integers(0, 256, 32, dtype=np.uint8).tobytes() for _ in range(N)]
     msgs[0] = hashlib.shake_256(f"reject-search/{s}/{g['indices'][0]}".encode()).digest(32)
     sig, attempts = O.sign_batch(s, esk, msgs)
-    assert attempts[0] > 0
+    assert attempts[0] > 1
     return s, seeds, esk, epk, np.frombuffer(b"".join(msgs), np.uint8).reshape(N, 32), sig, cpk
 
 
@@ -67,6 +67,26 @@ def test_sign_verify_launch_edges(case, off):
         torch.cuda.synchronize()
         assert (out[:b].cpu().numpy() == sig[:b]).all() and not out[b:].any(), b
         assert (res[:b].cpu().numpy() == want[:b]).all() and (res[b:] == 0xEE).all(), b
+
+
+def test_sign_more_than_a_wave(case):
+    """More signatures than CTAs fit the GPU at once; singular first attempts at the start, in the
+    middle and at the end of the batch."""
+    import torch
+    s, _, esk, _, msgs, sig, _ = case
+    m = Mayo(s)
+    z = m.sizes
+    n = 148 * {1: 3, 2: 6, 3: 2, 5: 1}[s] + 37
+    pick = np.arange(n) % N  # 0: singular
+    pick[[1, 149, n - 1, n - 2]] = 0
+    d_esk = torch.from_numpy(esk[pick]).cuda()
+    d_msg = torch.from_numpy(msgs[pick]).cuda()
+    ws = torch.zeros(n * m.sign_ws_bytes(), dtype=torch.uint8, device="cuda")
+    for b in (n, n - 1, 149):
+        out = torch.zeros(n, z.sig_bytes, dtype=torch.uint8, device="cuda")
+        m.sign_many(d_esk, d_msg, out, ws, b, msg_stride=32, mlen=32, esk_stride=z.esk_bytes)
+        torch.cuda.synchronize()
+        assert (out[:b].cpu().numpy() == sig[pick[:b]]).all() and not out[b:].any(), b
 
 
 @pytest.mark.parametrize("off", [0, 1, 2, 3])
