@@ -15,9 +15,9 @@
 //
 // Inside a kernel each CTA takes the next item (see queue_pop), runs it with the same device
 // functions as the batched kernels, and takes the next; a CTA that finds its bucket empty exits
-// at once and frees its SM for the other buckets' kernels.  A sign attempt whose linear system is singular is not retried in place: the CTA
-// pushes (sign, ctr + 1) to the tail of its bucket and goes on popping, so the item is served
-// either by that CTA or by another one still running.  No CTA waits for another kernel, so the
+// at once and frees its SM for the other buckets' kernels.  A sign attempt whose linear system is
+// singular is not retried in place: the CTA pushes (sign, ctr + 1) to the tail of its bucket and goes
+// on popping, so the item is served either by that CTA or by another one still running.  No CTA waits for another kernel, so the
 // kernels need not be co-resident.  Every wait is bounded: past `spin_limit` it sets an error
 // code and ends the CTA.
 #include <cuda_runtime.h>
@@ -33,6 +33,7 @@ namespace mayo {
 
 constexpr uint32_t Q_EMPTY = 0xFFFFFFFFu;
 constexpr uint32_t Q_STOP = 0xFFFFFFFEu;
+constexpr uint32_t Q_ABANDONED = 0xFFFFFFFDu;  // a slot past the tail whose ticket was given up (no item has op 3)
 constexpr int Q_BUCKETS = 12;             // (set index) * 3 + op
 constexpr int Q_CTRL_WORDS = 16;          // control words per bucket; block 12 counts invalid ops
 
@@ -77,7 +78,7 @@ struct QueueArgs {
     QueueOps ops;
     uint32_t *slots;
     uint32_t capacity;
-    uint32_t *ctrl;  // [0] head, [1] tail, [2] done, [3] error, [4] pushes
+    uint32_t *ctrl;  // [0] taken, [1] tail, [2] done, [3] error, [4] pushes, [5] tickets
     uint8_t *scratch;
     size_t scratch_stride;
     uint32_t spin_limit;
@@ -87,26 +88,26 @@ __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) { return *rei
 
 __device__ __forceinline__ void queue_error(uint32_t *ctrl, uint32_t code) { atomicCAS(&ctrl[3], 0u, code); }
 
-// Take the next item.  Near the end of a bucket head moves by compare-and-swap and only while
-// head < tail, so no ticket is handed out past the published items and a CTA that finds its
-// bucket empty leaves at once, freeing its SM for the other buckets' kernels.  A sign re-enqueued
-// later is still served: the CTA that pushed it keeps popping, and it either takes the item
-// itself or finds it taken by another CTA.  While at least gridDim items remain, head moves by
-// atomicAdd (no retries under contention); such a ticket can overshoot the tail only if other
-// CTAs popped several times in between, and then it waits, as every ticket past the tail must,
-// for a push into its slot or for the bucket to drain (done == tail: `done` is read first, so a
-// push from an unfinished item cannot be missed).  Every wait is bounded by spin_limit.
-__device__ uint32_t queue_wait_slot(const QueueArgs &q, uint32_t h, uint32_t &it) {
-    for (;; it++) {
-        const uint32_t v = ld_volatile(&q.slots[h]);
+// Take the next item: a ticket by one atomicAdd, whose slot holds an item, or is about to (its number is
+// below the tail, so the wait is for another CTA's store; bounded by spin_limit), or lies past the
+// tail: then the CTA marks it abandoned and leaves, freeing its SM for the other buckets' kernels.  A
+// sign re-enqueued into an abandoned slot stays with the CTA that pushed it; one pushed into a slot
+// whose ticket is still to come is served by that CTA, which goes on popping, or by another.
+// (Tickets by compare-and-swap, so that none passes the tail, made a bucket with fewer items than
+// CTAs spend up to 0.3 ms in failed exchanges: MAYO_2 verify, 1,365 items, 483 us.)
+__device__ uint32_t queue_pop(const QueueArgs &q) {
+    const uint32_t h = atomicAdd(&q.ctrl[5], 1u);
+    if (h >= q.capacity) return Q_STOP;
+    for (uint32_t it = 0;; it++) {
+        uint32_t v = ld_volatile(&q.slots[h]);
+        if (v == Q_EMPTY && h >= ld_volatile(&q.ctrl[1])) {
+            v = atomicCAS(&q.slots[h], Q_EMPTY, Q_ABANDONED);
+            if (v == Q_EMPTY) return Q_STOP;
+        }
         if (v != Q_EMPTY) {
             __threadfence();
             return v;
         }
-        const uint32_t done = ld_volatile(&q.ctrl[2]);
-        __threadfence();
-        const uint32_t tail = ld_volatile(&q.ctrl[1]);
-        if (h >= tail && done == tail) return Q_STOP;  // drained: no unfinished item can push
         if (it >= q.spin_limit) {
             queue_error(q.ctrl, MAYO_B200_QUEUE_ERR_TIMEOUT);
             return Q_STOP;
@@ -115,35 +116,17 @@ __device__ uint32_t queue_wait_slot(const QueueArgs &q, uint32_t h, uint32_t &it
     }
 }
 
-__device__ uint32_t queue_pop(const QueueArgs &q) {
-    uint32_t it = 0;
-    for (;;) {
-        const uint32_t h = ld_volatile(&q.ctrl[0]);
-        const uint32_t t = ld_volatile(&q.ctrl[1]);
-        const uint32_t lim = t < q.capacity ? t : q.capacity;
-        if (h >= lim) return Q_STOP;
-        if (lim - h >= gridDim.x) {
-            const uint32_t h2 = atomicAdd(&q.ctrl[0], 1u);
-            return h2 < q.capacity ? queue_wait_slot(q, h2, it) : Q_STOP;
-        }
-        if (atomicCAS(&q.ctrl[0], h, h + 1) == h) return queue_wait_slot(q, h, it);
-        if (++it >= q.spin_limit) {  // lost the race that many times
-            queue_error(q.ctrl, MAYO_B200_QUEUE_ERR_TIMEOUT);
-            return Q_STOP;
-        }
-    }
-}
-
-__device__ void queue_push(const QueueArgs &q, uint32_t item) {
+// Publish an item; returns it if its slot has been abandoned (the caller runs it), else Q_EMPTY.
+__device__ uint32_t queue_push(const QueueArgs &q, uint32_t item) {
     const uint32_t slot = atomicAdd(&q.ctrl[1], 1u);
     if (slot >= q.capacity) {
         queue_error(q.ctrl, MAYO_B200_QUEUE_ERR_FULL);
         atomicAdd(&q.ctrl[2], 1u);  // the item is dropped: count it as finished
-        return;
+        return Q_EMPTY;
     }
     atomicAdd(&q.ctrl[4], 1u);
     __threadfence();
-    *reinterpret_cast<volatile uint32_t *>(&q.slots[slot]) = item;
+    return atomicCAS(&q.slots[slot], Q_EMPTY, item) == Q_ABANDONED ? item : Q_EMPTY;
 }
 
 // Operands of one instance, checked against the counts and key tables the caller declared.
@@ -248,7 +231,7 @@ __device__ void queue_keypair(uint8_t *smem, int tid, const QueueOps &ops, uint3
 
 template <int SET>
 __device__ void queue_sign(uint8_t *smem, int tid, const QueueArgs &q, const ItemRefs &r, uint32_t inst, int ctr,
-                           uint32_t item) {
+                           uint32_t item, uint32_t *kept) {
     using S = Set<SET>;
     using C = SignCfg<SET>;
     sign_hash_cta<C>(smem, tid, r.key, r.msg, r.mlen, ctr);
@@ -257,7 +240,7 @@ __device__ void queue_sign(uint8_t *smem, int tid, const QueueArgs &q, const Ite
         // success, or the 255th rejection: the reference emits the last attempt (x = r)
         sign_write<C>(smem, tid, r.key, q.ops.sg_sig + (size_t)inst * S::sig);
     } else if (tid == 0) {
-        queue_push(q, (item & ~(0xFFu << 20)) | ((uint32_t)(ctr + 1) << 20));
+        *kept = queue_push(q, (item & ~(0xFFu << 20)) | ((uint32_t)(ctr + 1) << 20));
     }
 }
 
@@ -265,14 +248,20 @@ template <int SET, int OP>
 __global__ void __launch_bounds__(QueueCfg<SET, OP>::NT, QueueCfg<SET, OP>::MINB) queue_kernel(const QueueArgs q) {
     using S = Set<SET>;
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint32_t s_item;
+    __shared__ uint32_t s_item, s_kept;
     const int tid = threadIdx.x;
+    uint32_t taken = 0;
+    if (tid == 0) s_kept = Q_EMPTY;
     for (;;) {
-        if (tid == 0) s_item = queue_pop(q);
+        if (tid == 0) {
+            s_item = s_kept != Q_EMPTY ? s_kept : queue_pop(q);
+            s_kept = Q_EMPTY;
+        }
         __syncthreads();
         const uint32_t item = s_item;
         __syncthreads();
         if (item == Q_STOP) break;
+        taken++;
         const uint32_t inst = item & 0xFFFFF;
         const ItemRefs r = queue_refs<SET, OP>(q.ops, inst);
         if (!r.ok) {
@@ -280,9 +269,10 @@ __global__ void __launch_bounds__(QueueCfg<SET, OP>::NT, QueueCfg<SET, OP>::MINB
         } else if constexpr (OP == MAYO_B200_OP_KEYPAIR) {
             queue_keypair<SET>(smem, tid, q.ops, inst, q.scratch + (size_t)blockIdx.x * q.scratch_stride);
         } else if constexpr (OP == MAYO_B200_OP_SIGN) {
-            queue_sign<SET>(smem, tid, q, r, inst, (int)((item >> 20) & 0xFF), item);
+            queue_sign<SET>(smem, tid, q, r, inst, (int)((item >> 20) & 0xFF), item, &s_kept);
         } else {
-            verify_instance<SET>(smem, tid, r.key, r.msg, r.mlen, q.ops.vf_sig + (size_t)inst * S::sig, q.ops.vf_res + inst);
+            verify_instance<SET>(smem, tid, r.key, r.msg, r.mlen, q.ops.vf_sig + (size_t)inst * S::sig,
+                                 q.ops.vf_res + inst);
         }
         __syncthreads();
         if (tid == 0) {
@@ -290,6 +280,7 @@ __global__ void __launch_bounds__(QueueCfg<SET, OP>::NT, QueueCfg<SET, OP>::MINB
             atomicAdd(&q.ctrl[2], 1u);
         }
     }
+    if (tid == 0 && taken) atomicAdd(&q.ctrl[0], taken);
 }
 
 // Every bucket's slots <- empty, control words <- 0.
