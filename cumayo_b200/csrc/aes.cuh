@@ -179,30 +179,41 @@ __device__ __forceinline__ AesRun aes_run(const AesLut<NTAB> &t, const RK &rk, u
     return r;
 }
 
-// Encrypt counter block `blk` of run `run`: k3 = the low byte of rk[3], rk[i] = round key word 12 + i.
-template <int NTAB, class RK>
-__device__ __forceinline__ AesOut aes128_ctr_block_t(const AesLut<NTAB> &t, uint32_t a0, uint32_t k3, const AesRun &run,
-                                                     const RK &rk, uint32_t blk) {
-    const uint32_t a1 = a0 ^ t.r24(byte_of(blk ^ k3, 0));
-    uint32_t s0 = run.ka ^ t.r0(a1 >> 24), s1 = run.kb ^ t.r24(byte_of(a1, 0)), s2 = run.kc ^ t.r16(byte_of(a1, 1)),
-             s3 = run.kd ^ t.r8(byte_of(a1, 2));
+// Encrypt N counter blocks side by side, block blk[i] of run run[i] (i < N): k3 = the low byte of rk[3],
+// rk[i] = round key word 12 + i.
+template <int NTAB, int N, class RK>
+__device__ __forceinline__ void aes128_ctr_blocks(const AesLut<NTAB> &t, uint32_t a0, uint32_t k3, const AesRun (&run)[N],
+                                                  const RK &rk, const uint32_t (&blk)[N], AesOut (&o)[N]) {
+    uint32_t s[N][4];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const uint32_t a1 = a0 ^ t.r24(byte_of(blk[i] ^ k3, 0));
+        s[i][0] = run[i].ka ^ t.r0(a1 >> 24);
+        s[i][1] = run[i].kb ^ t.r24(byte_of(a1, 0));
+        s[i][2] = run[i].kc ^ t.r16(byte_of(a1, 1));
+        s[i][3] = run[i].kd ^ t.r8(byte_of(a1, 2));
+    }
 #pragma unroll
     for (int r = 0; r < 7; r++) {  // rounds 3 .. 9
-        const uint32_t a = t.mix(s0, s1, s2, s3) ^ rk[4 * r];
-        const uint32_t b = t.mix(s1, s2, s3, s0) ^ rk[4 * r + 1];
-        const uint32_t c = t.mix(s2, s3, s0, s1) ^ rk[4 * r + 2];
-        const uint32_t d = t.mix(s3, s0, s1, s2) ^ rk[4 * r + 3];
-        s0 = a;
-        s1 = b;
-        s2 = c;
-        s3 = d;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const uint32_t a = t.mix(s[i][0], s[i][1], s[i][2], s[i][3]) ^ rk[4 * r];
+            const uint32_t b = t.mix(s[i][1], s[i][2], s[i][3], s[i][0]) ^ rk[4 * r + 1];
+            const uint32_t c = t.mix(s[i][2], s[i][3], s[i][0], s[i][1]) ^ rk[4 * r + 2];
+            const uint32_t d = t.mix(s[i][3], s[i][0], s[i][1], s[i][2]) ^ rk[4 * r + 3];
+            s[i][0] = a;
+            s[i][1] = b;
+            s[i][2] = c;
+            s[i][3] = d;
+        }
     }
-    AesOut o;
-    o.w0 = t.last(s0, s1, s2, s3) ^ rk[28];
-    o.w1 = t.last(s1, s2, s3, s0) ^ rk[29];
-    o.w2 = t.last(s2, s3, s0, s1) ^ rk[30];
-    o.w3 = t.last(s3, s0, s1, s2) ^ rk[31];
-    return o;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        o[i].w0 = t.last(s[i][0], s[i][1], s[i][2], s[i][3]) ^ rk[28];
+        o[i].w1 = t.last(s[i][1], s[i][2], s[i][3], s[i][0]) ^ rk[29];
+        o[i].w2 = t.last(s[i][2], s[i][3], s[i][0], s[i][1]) ^ rk[30];
+        o[i].w3 = t.last(s[i][3], s[i][0], s[i][1], s[i][2]) ^ rk[31];
+    }
 }
 
 // Big-endian words -> little-endian words of the byte stream.
@@ -227,6 +238,11 @@ __device__ __forceinline__ void st16(uint8_t *p, uint32_t a, uint32_t b, uint32_
 #pragma unroll
         for (int i = 0; i < 16; i++) p[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
     }
+}
+
+// Counter block blk's 16 stream bytes.
+__device__ __forceinline__ void aes_store(uint8_t *out, uint32_t blk, const AesOut &o) {
+    st16(out + (size_t)blk * 16, bswap32(o.w0), bswap32(o.w1), bswap32(o.w2), bswap32(o.w3));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -304,8 +320,11 @@ static __global__ void __launch_bounds__(AES_THREADS, 1)
 #pragma unroll 1
             for (uint32_t blk = g + lane; blk < min(g + grab, b1); blk += 32) {
                 const uint4 r = s_run[buf][(blk >> 8) - (b0 >> 8)];
-                const AesOut o = aes128_ctr_block_t<4>(lut, a0, k3, AesRun{r.x, r.y, r.z, r.w}, rk, blk);
-                st16(out + (size_t)blk * 16, bswap32(o.w0), bswap32(o.w1), bswap32(o.w2), bswap32(o.w3));
+                const AesRun run[1] = {{r.x, r.y, r.z, r.w}};
+                const uint32_t n[1] = {blk};
+                AesOut o[1];
+                aes128_ctr_blocks(lut, a0, k3, run, rk, n, o);
+                aes_store(out, blk, o[0]);
             }
         }
         __syncthreads();

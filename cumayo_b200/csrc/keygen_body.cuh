@@ -9,7 +9,7 @@
 namespace mayo {
 
 // P3 = Upper(O^T T), T = P1 O + P2: the rows of P1 as in VerifyCfg, then T's quads with O again.
-template <int SET, int CL_ = 1>
+template <int SET, int CL_ = 1, int CW_ = 0>
 struct KeyCfg {
     using S = Set<SET>;
     static constexpr int CL = CL_, J = S::o, NQ = QuadCfg<SET>::NQ, ST = QuadAcc<J>::ST;
@@ -22,7 +22,7 @@ struct KeyCfg {
     // against 0.322 with four and 0.486 with three CTAs of three warps (spills); MAYO_3 two CTAs of
     // six warps 0.796 against 0.809 with four warps and two columns ahead (then 0.698; eight warps in one CTA 0.729);
     // MAYO_5 one CTA of eight warps, two columns ahead, 1.55 against 1.69 with eleven, one ahead.
-    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 2 : SET == 3 ? 6 : 8);
+    static constexpr int CW = CW_ ? CW_ : CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 2 : SET == 3 ? 6 : 8);
     static constexpr int NT = 32 * CW;
     static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;
     static constexpr int CH2 = (J * NQ + 31) / 32;
@@ -99,10 +99,9 @@ __device__ __forceinline__ void store_word(uint8_t *p, uint32_t w, int n) {
 // P3 of one instance: P1 || P2 at P1, O (o_bytes) already in shared memory at off_o (of every CTA of a
 // cluster); writes the packed upper triangle to P3out (rank 0).  All NT threads must call it.  RO:
 // P1 and P2 are not written in this kernel.
-template <int SET, int CL, bool RO>
+template <int SET, int CL, bool RO, class C = KeyCfg<SET, CL>>
 __device__ __forceinline__ void p3_instance(uint8_t *smem, int tid, const uint8_t *P1, uint8_t *P3out, int rank = 0) {
     using S = Set<SET>;
-    using C = KeyCfg<SET, CL>;
     constexpr int J = C::J, NQ = C::NQ, NT = C::NT, NP = C::NP, ULP = C::CH * 32;
     uint4 *masks = reinterpret_cast<uint4 *>(smem + C::off_masks);
     uint4 *mask2 = reinterpret_cast<uint4 *>(smem + C::off_mask2);

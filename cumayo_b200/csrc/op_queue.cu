@@ -43,7 +43,8 @@ struct QueueCfg;
 template <int SET>
 struct QueueCfg<SET, MAYO_B200_OP_KEYPAIR> {
     using S = Set<SET>;
-    using KC = KeyCfg<SET>;
+    // MAYO_2: four warps instead of the batched kernel's two, for the expansion's sake
+    using KC = KeyCfg<SET, 1, SET == 2 ? 4 : 0>;
     static constexpr int NT = KC::NT, MINB = KC::MINB;
     // as many replicated round tables as the P3 area below O holds (MAYO_1: T0; MAYO_2: T0 and
     // ror16(T0); MAYO_3: three; MAYO_5: all four) and the round keys; dead once the keystream is written
@@ -218,15 +219,28 @@ __device__ void queue_keypair(uint8_t *smem, int tid, const QueueOps &ops, uint3
 #pragma unroll
         for (int i = 0; i < 32; i++) rk[i] = rk_s[12 + i];
         __syncthreads();
-        for (uint32_t blk = tid; blk < nblk; blk += NT) {
-            const uint4 r = s_run[blk >> 8];
-            const AesOut o = aes128_ctr_block_t<NTAB>(lut, a0, k3, AesRun{r.x, r.y, r.z, r.w}, rk, blk);
-            st16(scratch + (size_t)blk * 16, bswap32(o.w0), bswap32(o.w1), bswap32(o.w2), bswap32(o.w3));
+        // NB blocks per thread side by side: a CTA has too few warps to hide the table reads (MAYO_5,
+        // 1,365 keypairs: one 2.92 ms, two 2.78, three 2.72)
+        constexpr int NB = 3;
+        for (uint32_t b0 = tid; b0 < nblk; b0 += NB * NT) {
+            AesRun run[NB];
+            uint32_t blk[NB];
+            AesOut o[NB];
+#pragma unroll
+            for (int i = 0; i < NB; i++) {
+                blk[i] = min(b0 + (uint32_t)(i * NT), nblk - 1);
+                const uint4 r = s_run[blk[i] >> 8];
+                run[i] = AesRun{r.x, r.y, r.z, r.w};
+            }
+            aes128_ctr_blocks(lut, a0, k3, run, rk, blk, o);
+#pragma unroll
+            for (int i = 0; i < NB; i++)
+                if (b0 + i * NT < nblk) aes_store(scratch, blk[i], o[i]);
         }
     }
     __syncthreads();  // scratch writes visible to the whole CTA; AES tables no longer needed
     for (int i = tid; i < 16; i += NT) pk[i] = s_seedpk[i];
-    p3_instance<SET, 1, false>(smem, tid, scratch, pk + 16);
+    p3_instance<SET, 1, false, typename QC::KC>(smem, tid, scratch, pk + 16);
 }
 
 template <int SET>
