@@ -186,12 +186,19 @@ struct LCfg {
     // registers); MAYO_2 0.327 with four warps, 0.344 with two; MAYO_3 0.901 with two CTAs of six warps,
     // 1.02 with eight warps, two columns ahead; MAYO_5 2.27 with eight warps, two ahead, 2.40 with
     // eleven, one ahead
-    static constexpr int CW = CL > 1 ? (CH + CL - 1) / CL : (SET == 1 ? 4 : SET == 2 ? 4 : SET == 3 ? 6 : 8);
+    // With several CTAs per instance a chunk's columns are split over eight warps, whose sums meet in
+    // shared memory: a lone warp ran a chunk's 78 to 142 columns one after another.  expand-sk for one
+    // secret, MAYO_1 57 -> 38 us, MAYO_2 64 -> 45, MAYO_3 72 -> 50, MAYO_5 83 -> 74; at 72 secrets MAYO_1
+    // 71 -> 64, MAYO_5 210 -> 212.
+    static constexpr int CHC = (CH + CL - 1) / CL;  // chunks of a CTA
+    static constexpr int CW = CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 4 : SET == 3 ? 6 : 8);
     static constexpr int NT = 32 * CW;
     static constexpr int D = SET == 5 ? 2 : 1;  // columns loaded ahead
     static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 5 ? 1 : 2);
+    static constexpr int PC = CL > 1 ? (2 * CW + CHC - 1) / CHC : 1;
     static constexpr size_t off_masks = 0;
-    static constexpr size_t off_o = (size_t)S::v * ST * 16;
+    static constexpr size_t off_T = (size_t)S::v * ST * 16;
+    static constexpr size_t off_o = off_T + (PC > 1 ? (size_t)J * CHC * 32 * 16 : 0);
     static constexpr size_t off_ctr = off_o + pad16(S::o_bytes);
     static constexpr size_t total = off_ctr + 16;
 };
@@ -238,36 +245,54 @@ __device__ __forceinline__ void l_instance(uint8_t *smem, int tid, const uint8_t
     const int lane = tid & 31;
     const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(P1) & 3);
     const uint32_t *base4 = reinterpret_cast<const uint32_t *>(P1 - mis);
+    uint4 *T = reinterpret_cast<uint4 *>(smem + C::off_T);  // [j][unit of this CTA]
     if (tid == 0) *s_next = 0;
     if constexpr (CL == 1) l2_prefetch_range(base4, mis, S::p1, tid, NT);  // read by rows and by columns
     build_masks9<J>(reinterpret_cast<uint32_t *>(masks), S::v, tid, NT,
                     [&](int c, int j) { return o_nibble<SET>(s_O, c, j); });
+    if constexpr (C::PC > 1) {
+        for (int i = tid; i < J * C::CHC * 32; i += NT) T[i] = make_uint4(0, 0, 0, 0);
+    }
     __syncthreads();
+    // words q of L[r0 + i][j] from the sum's planes
+    auto store = [&](const G4 &f, int r0, int j, int q) {
+        const G4 v = quad_planes(f.p0, f.p1, f.p2, f.p3);
+        const uint32_t wd[4] = {v.p0, v.p1, v.p2, v.p3};
+        uint32_t w[4];
+        p2_words<SET, false>(base4, mis + S::p1, r0, j, q, w);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (r0 + i < S::v)
+                store_word(P2 + (size_t)((r0 + i) * S::o + j) * S::menc + 4 * q, wd[i] ^ w[i], QuadCfg<SET>::bytes(q));
+    };
     for (;;) {
-        const int chunk = rank + CL * warp_next(s_next, lane);
+        const int item = warp_next(s_next, lane), lc = item / C::PC, piece = item - lc * C::PC;
+        const int chunk = rank + CL * lc;
         if (chunk >= C::CH) break;
         const int u = chunk * 32 + lane, t = u / NQ, q = u - t * NQ, r0 = 4 * t;
         const int qmin = chunk * 32 / NQ, qmax = min((chunk * 32 + 31) / NQ, C::QN - 1);
         QuadAcc<J> acc;
         acc.zero();
         SymRows<SET> rows{mis, (uint32_t)(4 * q), r0, false};
+        const int ca = S::v * piece / C::PC, cb = S::v * (piece + 1) / C::PC;
 #pragma unroll 1
         for (int seg = 0; seg < 2; seg++) {  // from the diagonal on, then the columns left of every row
             rows.lower = seg == 1;
-            quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? 0 : 4 * qmin,
-                                          seg ? 4 * qmin : S::v, seg ? 0 : 4 * qmax + 4, masks, mis == 0);
+            quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? ca : max(ca, 4 * qmin),
+                                             seg ? min(cb, 4 * qmin) : cb, seg ? 0 : 4 * qmax + 4, masks, mis == 0);
         }
 #pragma unroll
         for (int j = 0; j < J; j++) {
-            const G4 f = acc.fold(j);
-            const G4 v = quad_planes(f.p0, f.p1, f.p2, f.p3);
-            const uint32_t wd[4] = {v.p0, v.p1, v.p2, v.p3};
-            uint32_t w[4];
-            p2_words<SET, false>(base4, mis + S::p1, r0, j, q, w);
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-                if (r0 + i < S::v)
-                    store_word(P2 + (size_t)((r0 + i) * S::o + j) * S::menc + 4 * q, wd[i] ^ w[i], QuadCfg<SET>::bytes(q));
+            if constexpr (C::PC > 1) g4_atomic_xor(T + (j * C::CHC + lc) * 32 + lane, acc.fold(j));
+            else store(acc.fold(j), r0, j, q);
+        }
+    }
+    if constexpr (C::PC > 1) {
+        __syncthreads();
+        for (int i = tid; i < J * C::CHC * 32; i += NT) {
+            const int j = i / (C::CHC * 32), lu = i - j * (C::CHC * 32), chunk = rank + CL * (lu >> 5);
+            const int u = chunk * 32 + (lu & 31), t = u / NQ, q = u - t * NQ;
+            if (chunk < C::CH) store(g4_ld(T + i), 4 * t, j, q);
         }
     }
 }
