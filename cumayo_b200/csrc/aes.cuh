@@ -246,13 +246,13 @@ __device__ __forceinline__ void aes_store(uint8_t *out, uint32_t blk, const AesO
 }
 
 // ---------------------------------------------------------------------------------------------
-// Kernel: AES-CTR keystream into a pitched pool.  An item is (instance, chunk): chunk x of an instance
-// takes blocks [x * bpc, min((x + 1) * bpc, nblk_main)) to row + out_off, keyed by 16 bytes at row +
-// key_off.  A CTA builds the tables once and takes items blockIdx.x, + gridDim.x, ...; while its
+// Kernel: AES-CTR keystream of nbytes into a pitched pool.  An item is (instance, chunk): chunk x of an
+// instance takes blocks [x * bpc, (x + 1) * bpc) to row + out_off, keyed by 16 bytes at row + key_off
+// (or derived, see AesDerive).  A CTA builds the tables once and takes items blockIdx.x, + gridDim.x, ...; while its
 // worker warps run one item, the last warp prepares the next one (key schedule, the chunk's AesRuns).
 // The workers take the item's blocks 64 at a time from a counter (32 where an item has few).  When the key overlaps the output
-// (expand-pk, expand-sk keep seed_pk in the last 16 output bytes until expansion), nblk_main
-// excludes the blocks that overlap the key and aes_ctr_tail_kernel finishes them afterwards, one
+// (expand-pk, expand-sk keep seed_pk in the last 16 output bytes until expansion), nbytes ends
+// before the blocks that overlap the key and aes_ctr_tail_kernel finishes them afterwards, one
 // thread per instance.
 // ---------------------------------------------------------------------------------------------
 constexpr int AES_WORKERS = 768, AES_THREADS = AES_WORKERS + 32;  // and the warp that prepares
@@ -261,9 +261,21 @@ constexpr int AES_ITEM_COST = 700;          // what an item costs besides its bl
 constexpr int AES_RUNS = AES_BLOCKS_PER_ITEM / 256 + 2;
 constexpr size_t AES_SMEM = 4 * 256 * 32 * 4;  // T0 and its rotations by 8, 16, 24, each replicated 32 times
 
-static __global__ void __launch_bounds__(AES_THREADS, 1)
-    aes_ctr_kernel(uint8_t *pool, size_t pitch, size_t key_off, size_t out_off, uint32_t nblk_main, uint32_t bpc,
-                   uint32_t chunks, uint32_t items, uint32_t k128) {
+// Where an item's key comes from when the kernel derives it from the secret seed (DERIVE, the
+// smallest batches): seed_pk || O = SHAKE256(seed_sk), seed_sk at the row's start, or first
+// SHAKE128(LE64(rand_index + 2 inst + 1)) where `counter` is set (src/keypair.cu:35-50).  The preparing
+// warp then also writes what the hash kernels would: O to row + o_off and, where key_off is used,
+// seed_pk to row + key_off, for an instance's first chunk, while the workers are at it.
+struct AesDerive {
+    uint32_t sk_bytes, o_bytes, write_key, counter;
+    size_t o_off;
+    uint64_t rand_index;
+};
+
+template <bool DERIVE>
+__global__ void __launch_bounds__(AES_THREADS, 1)
+    aes_ctr_kernel(uint8_t *pool, size_t pitch, size_t key_off, size_t out_off, uint32_t nbytes, uint32_t bpc,
+                   uint32_t chunks, uint32_t items, uint32_t k128, const AesDerive dv) {
     extern __shared__ uint32_t aes_smem[];  // [4][256 * 32] words
     __shared__ uint32_t s_rk[2][44];
     __shared__ uint4 s_run[2][AES_RUNS];
@@ -279,30 +291,90 @@ static __global__ void __launch_bounds__(AES_THREADS, 1)
     }
     __syncthreads();
     const AesLut<4> lut{(uint32_t)__cvta_generic_to_shared(aes_smem + lane), k128};
-    auto prepare = [&](int buf, uint32_t item) {  // the last warp
-        const uint32_t inst = item / chunks, b0 = (item - inst * chunks) * bpc;
+    [[maybe_unused]] WarpKeccak wk;
+    if constexpr (DERIVE) wk.setup(lane);
+    // the last warp; returns its sponge state after the first block of seed_pk || O
+    auto prepare = [&](int buf, uint32_t item) {
+        const uint32_t inst = item / chunks, chunk = item - inst * chunks, b0 = chunk * bpc;
+        uint8_t *row = pool + (size_t)inst * pitch;
+        const uint8_t *key = row + key_off;
+        uint64_t a = 0;
+        if constexpr (DERIVE) {
+            __shared__ uint64_t s_sk[8], s_key[2];  // the counter and the seed; seed_pk
+            const uint8_t *sk = row;
+            if (dv.counter) {
+                if (lane == 0) s_sk[0] = dv.rand_index + (uint64_t)(uint32_t)(2u * inst) + 1;
+                __syncwarp();
+                uint8_t *seed = reinterpret_cast<uint8_t *>(s_sk + 1);
+                warp_shake<168>(seed, (int)dv.sk_bytes, reinterpret_cast<const uint8_t *>(s_sk), 8, wk, lane);
+                for (int i0 = 0; i0 < (int)dv.sk_bytes; i0 += 32) {
+                    if (chunk == 0 && i0 + lane < (int)dv.sk_bytes) row[i0 + lane] = seed[i0 + lane];
+                    __syncwarp();
+                }
+                sk = seed;
+            }
+            const int n = (int)dv.sk_bytes - 8 * lane;  // one block: sk_bytes < 136
+            if (n > 0) a = ld_bytes(sk + 8 * lane, n < 8 ? n : 8);
+            if (n >= 0 && n < 8) a ^= (uint64_t)0x1F << (8 * n);
+            if (lane == 16) a ^= 0x8000000000000000ull;
+            a = wk.permute(lane < 25 ? a : 0, lane);
+            if (lane < 2) s_key[lane] = a;
+            __syncwarp();
+            key = reinterpret_cast<const uint8_t *>(s_key);
+        }
         if (lane == 0) {
-            aes128_key_schedule(pool + (size_t)inst * pitch + key_off, s_rk[buf]);
+            aes128_key_schedule(key, s_rk[buf]);
             s_next[buf] = 0;
         }
         __syncwarp();
         const uint32_t *rk = s_rk[buf];
         const uint32_t runs = ((b0 & 255u) + bpc + 255u) / 256u;
-        for (uint32_t h = (uint32_t)lane; h < runs; h += 32) {
-            const AesRun r = aes_run(lut, rk, (b0 >> 8) + h);
-            s_run[buf][h] = make_uint4(r.ka, r.kb, r.kc, r.kd);
+        for (uint32_t h0 = 0; h0 < runs; h0 += 32) {
+            const uint32_t h = h0 + (uint32_t)lane;
+            if (h < runs) {
+                const AesRun r = aes_run(lut, rk, (b0 >> 8) + h);
+                s_run[buf][h] = make_uint4(r.ka, r.kb, r.kc, r.kd);
+            }
+            __syncwarp();
         }
         if (lane == 0) s_a0[buf] = aes_run_a0(lut, rk);
+        return a;
+    };
+    // seed_pk and O of an instance from the state `a` (an instance's first chunk)
+    auto squeeze = [&](uint32_t item, uint64_t a) {
+        const uint32_t inst = item / chunks;
+        if (item != inst * chunks) return;
+        uint8_t *row = pool + (size_t)inst * pitch;
+        const int total = 16 + (int)dv.o_bytes;
+        for (int o = 0; o < total; o += 136) {
+            if (o) a = wk.permute(a, lane);
+            if (lane < 17) {
+#pragma unroll
+                for (int b = 0; b < 8; b++) {
+                    const int at = o + 8 * lane + b;
+                    const uint8_t v = (uint8_t)(a >> (8 * b));
+                    if (at < 16) {
+                        if (dv.write_key) row[key_off + at] = v;
+                    } else if (at < total) {
+                        row[dv.o_off + at - 16] = v;
+                    }
+                }
+            }
+            __syncwarp();
+        }
     };
     constexpr int PREP = AES_WORKERS / 32;
-    if (warp == PREP) prepare(0, blockIdx.x);  // gridDim.x <= items
+    uint64_t state = 0;
+    if (warp == PREP) state = prepare(0, blockIdx.x);  // gridDim.x <= items
     __syncthreads();
-    const uint32_t grab = bpc < 2 * AES_WORKERS ? 32u : 64u;
+    const uint32_t grab = bpc < 2 * AES_WORKERS ? 32u : 64u, nblk = (nbytes + 15) / 16;
     int buf = 0;
 #pragma unroll 1
     for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, buf ^= 1) {
         if (warp == PREP) {
-            if (item + gridDim.x < items) prepare(buf ^ 1, item + gridDim.x);
+            const uint64_t a = state;
+            if (item + gridDim.x < items) state = prepare(buf ^ 1, item + gridDim.x);
+            if constexpr (DERIVE) squeeze(item, a);
             __syncthreads();
             continue;
         }
@@ -310,7 +382,7 @@ static __global__ void __launch_bounds__(AES_THREADS, 1)
 #pragma unroll
         for (int i = 0; i < 32; i++) rk[i] = s_rk[buf][12 + i];
         const uint32_t a0 = s_a0[buf], k3 = s_rk[buf][3];
-        const uint32_t inst = item / chunks, b0 = (item - inst * chunks) * bpc, b1 = min(b0 + bpc, nblk_main);
+        const uint32_t inst = item / chunks, b0 = (item - inst * chunks) * bpc, b1 = min(b0 + bpc, nblk);
         uint8_t *out = pool + (size_t)inst * pitch + out_off;
         for (;;) {
             uint32_t g = 0;
@@ -324,7 +396,14 @@ static __global__ void __launch_bounds__(AES_THREADS, 1)
                 const uint32_t n[1] = {blk};
                 AesOut o[1];
                 aes128_ctr_blocks(lut, a0, k3, run, rk, n, o);
-                aes_store(out, blk, o[0]);
+                if (16 * blk + 16 <= nbytes) {
+                    aes_store(out, blk, o[0]);
+                } else {  // a last partial block keeps its leading bytes
+                    const uint32_t w[4] = {bswap32(o[0].w0), bswap32(o[0].w1), bswap32(o[0].w2), bswap32(o[0].w3)};
+#pragma unroll
+                    for (uint32_t i = 0; i < 16; i++)
+                        if (16 * blk + i < nbytes) out[(size_t)blk * 16 + i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
+                }
             }
         }
         __syncthreads();

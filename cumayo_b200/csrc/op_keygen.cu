@@ -12,7 +12,8 @@ namespace mayo {
 
 // ---------------------------------------------------------------------------------------------
 // Hash kernels: one thread per instance, Keccak state in registers; or, for batches up to
-// HASH_WARP_MAX, one warp per instance.
+// HASH_WARP_MAX, one warp per instance.  The smallest batches have none: the expansion kernel's
+// preparing warps hash (AesDerive).
 // ---------------------------------------------------------------------------------------------
 // keypair: seed_sk = SHAKE128(LE64(rand_index + 2*inst + 1), SK) (src/keypair.cu:35-45) unless
 // `seeded`; then seed_pk || O = SHAKE256(seed_sk) (src/keypair.cu:47-50).  seed_pk goes to pk[0:16];
@@ -154,6 +155,40 @@ static uint32_t aes_chunks(uint32_t nblk, size_t batch, uint32_t ctas, uint32_t 
     return best;
 }
 
+struct AesPlan {
+    uint32_t ctas, chunks, bpc;
+};
+static bool aes_plan(uint32_t nbytes, size_t batch, AesPlan &p) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return false;
+    p.ctas = (uint32_t)sms;
+    p.chunks = aes_chunks((nbytes + 15) / 16, batch, p.ctas, &p.bpc);
+    return true;
+}
+// The kernel derives the keys itself where each CTA gets one item, so that an instance's hash is on
+// every CTA's path once and the rest of its sponge runs beside the encryption: keypair of one MAYO_1
+// 38.5 -> 31.2 us (of MAYO_2, whose O takes five more blocks of the sponge, 41.7 -> 43.5), of 72 56.7 ->
+// 43.3, of 148 80.0 -> 63.6; expand-sk, whose tail launch goes too, 37.8 -> 27.0 and 63.9 -> 45.8.  With several items per CTA the one preparing
+// warp's Keccak (5 us an item) holds the workers up: MAYO_2 at 1,024 334 us -> 394.
+static bool aes_derives(const AesPlan &p, size_t batch) { return batch * p.chunks <= p.ctas; }
+
+// nbytes of keystream for every row, keyed from row + key_off or, with DERIVE, from the seeds.
+template <bool DERIVE>
+static int aes_main(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, size_t key_off, size_t out_off,
+                    uint32_t nbytes, const AesPlan &p, const AesDerive &dv) {
+    if (!set_smem_attr(aes_ctr_kernel<DERIVE>, AES_SMEM)) return ST_CUDA;
+    // 32-bit item numbers: at most 2^24 instances per launch
+    for (size_t b0 = 0; b0 < batch; b0 += size_t(1) << 24) {
+        const uint32_t nb = (uint32_t)(batch - b0 < (size_t(1) << 24) ? batch - b0 : size_t(1) << 24);
+        const uint32_t items = nb * p.chunks;
+        aes_ctr_kernel<DERIVE><<<items < p.ctas ? items : p.ctas, AES_THREADS, AES_SMEM, st>>>(
+            pool + b0 * pitch, pitch, key_off, out_off, nbytes, p.bpc, p.chunks, items, 128u, dv);
+    }
+    return cudaPeekAtLastError() == cudaSuccess ? ST_OK : ST_CUDA;
+}
+
 static int aes_expand(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, size_t key_off, size_t out_off,
                       uint32_t nbytes, bool key_in_output) {
     // the main kernel writes whole blocks that neither run past nbytes nor touch the key
@@ -161,21 +196,10 @@ static int aes_expand(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st
     if (key_in_output) nblk_main = min(nblk_main, (uint32_t)((key_off - out_off) / 16));
     const uint32_t nblk = (nbytes + 15) / 16;
     if (nblk_main > 0) {
-        if (!set_smem_attr(aes_ctr_kernel, AES_SMEM)) return ST_CUDA;
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return ST_CUDA;
-        const uint32_t ctas = (uint32_t)sms;
-        uint32_t bpc = 0;
-        const uint32_t chunks = aes_chunks(nblk_main, batch, ctas, &bpc);
-        // 32-bit item numbers: at most 2^24 instances per launch
-        for (size_t b0 = 0; b0 < batch; b0 += size_t(1) << 24) {
-            const uint32_t nb = (uint32_t)(batch - b0 < (size_t(1) << 24) ? batch - b0 : size_t(1) << 24);
-            const uint32_t items = nb * chunks;
-            aes_ctr_kernel<<<items < ctas ? items : ctas, AES_THREADS, AES_SMEM, st>>>(
-                pool + b0 * pitch, pitch, key_off, out_off, nblk_main, bpc, chunks, items, 128u);
-        }
+        AesPlan plan;
+        if (!aes_plan(nblk_main * 16, batch, plan)) return ST_CUDA;
+        const int rc = aes_main<false>(pool, pitch, batch, st, key_off, out_off, nblk_main * 16, plan, AesDerive{});
+        if (rc != ST_OK) return rc;
     }
     if (nblk_main < nblk)
         aes_ctr_tail_kernel<<<(unsigned)((batch + AES_TAIL_THREADS - 1) / AES_TAIL_THREADS), AES_TAIL_THREADS, 0, st>>>(
@@ -203,14 +227,22 @@ static int l_cl(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st) {
 template <int SET>
 static int keypair_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, uint64_t rand_index, bool seeded) {
     using S = Set<SET>;
-    if (batch <= HASH_WARP_MAX)
-        keypair_hash_warp_kernel<SET><<<(unsigned)((batch + HASH_WARPS - 1) / HASH_WARPS), 32 * HASH_WARPS, 0, st>>>(
-            pool, pitch, (uint32_t)batch, rand_index, seeded ? 1 : 0);
-    else
-        keypair_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch,
-                                                                                     rand_index, seeded ? 1 : 0);
-    const size_t pk_off = align128(S::sk);
-    int rc = aes_expand(pool, pitch, batch, st, pk_off, pk_off + align128(S::pk), S::p, false);
+    const size_t pk_off = align128(S::sk), p_off = pk_off + align128(S::pk);
+    int rc;
+    AesPlan plan;
+    if (!aes_plan(S::p, batch, plan)) return ST_CUDA;
+    if (aes_derives(plan, batch)) {
+        rc = aes_main<true>(pool, pitch, batch, st, pk_off, p_off, S::p, plan,
+                      AesDerive{(uint32_t)S::sk, (uint32_t)S::o_bytes, 1u, seeded ? 0u : 1u, pk_off + 16, rand_index});
+    } else {
+        if (batch <= HASH_WARP_MAX)
+            keypair_hash_warp_kernel<SET><<<(unsigned)((batch + HASH_WARPS - 1) / HASH_WARPS), 32 * HASH_WARPS, 0, st>>>(
+                pool, pitch, (uint32_t)batch, rand_index, seeded ? 1 : 0);
+        else
+            keypair_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch,
+                                                                                         rand_index, seeded ? 1 : 0);
+        rc = aes_expand(pool, pitch, batch, st, pk_off, p_off, S::p, false);
+    }
     if (rc) return rc;
     switch (cluster_ctas(batch)) {
         case 8: return p3_cl<SET, 8>(pool, pitch, batch, st);
@@ -223,13 +255,21 @@ static int keypair_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st,
 template <int SET>
 static int expandsk_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st) {
     using S = Set<SET>;
-    if (batch <= HASH_WARP_MAX)
-        expandsk_hash_warp_kernel<SET><<<(unsigned)((batch + HASH_WARPS - 1) / HASH_WARPS), 32 * HASH_WARPS, 0, st>>>(
-            pool, pitch, (uint32_t)batch);
-    else
-        expandsk_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch);
     const size_t out_off = S::sk + S::o_bytes;
-    int rc = aes_expand(pool, pitch, batch, st, out_off + S::p - 16, out_off, S::p, true);
+    int rc;
+    AesPlan plan;
+    if (!aes_plan(S::p, batch, plan)) return ST_CUDA;
+    if (aes_derives(plan, batch)) {
+        rc = aes_main<true>(pool, pitch, batch, st, 0, out_off, S::p, plan,
+                      AesDerive{(uint32_t)S::sk, (uint32_t)S::o_bytes, 0u, 0u, (size_t)S::sk, 0});
+    } else {
+        if (batch <= HASH_WARP_MAX)
+            expandsk_hash_warp_kernel<SET><<<(unsigned)((batch + HASH_WARPS - 1) / HASH_WARPS), 32 * HASH_WARPS, 0, st>>>(
+                pool, pitch, (uint32_t)batch);
+        else
+            expandsk_hash_kernel<SET><<<(unsigned)((batch + 127) / 128), 128, 0, st>>>(pool, pitch, (uint32_t)batch);
+        rc = aes_expand(pool, pitch, batch, st, out_off + S::p - 16, out_off, S::p, true);
+    }
     if (rc) return rc;
     switch (cluster_ctas(batch)) {
         case 8: return l_cl<SET, 8>(pool, pitch, batch, st);

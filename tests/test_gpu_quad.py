@@ -110,3 +110,33 @@ def test_keypair_expandsk_launch_edges(case, off):
         assert (rows[:b, at: at + z.pk_bytes].cpu().numpy() == cpk[:b]).all() and not rows[b:, at:].any(), b
         assert (erows[:b, : z.esk_bytes].cpu().numpy() == esk[:b]).all() and not erows[b:, z.sk_bytes:].any(), b
         assert not erows[:, z.esk_bytes:].any(), b
+
+
+@pytest.mark.parametrize("n", [74, 75, 148, 149])
+def test_keypair_keys_derived_or_hashed_first(case, n):
+    """Around the batches from which a hash kernel runs before the expansion (148 SMs: one item each)."""
+    import torch
+    s, seeds, esk, _, _, _, cpk = case
+    m = Mayo(s)
+    z = m.sizes
+    at = (z.sk_bytes + 127) // 128 * 128
+    pick = np.arange(n) % N
+    d_seed = torch.from_numpy(seeds[pick]).cuda()
+    rows = torch.zeros(n, z.pitch_keypair, dtype=torch.uint8, device="cuda")
+    rows[:, : z.sk_bytes] = d_seed
+    m.crypto_sign_keypair_from_seed(rows.view(-1), z.pitch_keypair, n)
+    erows = torch.zeros(n, z.esk_bytes, dtype=torch.uint8, device="cuda")
+    erows[:, : z.sk_bytes] = d_seed
+    m.crypto_sign_expandsk(erows.view(-1), z.esk_bytes, n)
+    # seeds of the counter: the same keypair alone, from the seed that it wrote
+    drawn = torch.zeros(n, z.pitch_keypair, dtype=torch.uint8, device="cuda")
+    m.crypto_sign_keypair(drawn.view(-1), z.pitch_keypair, n, rand_index=5)
+    again = torch.zeros_like(drawn)
+    again[:, : z.sk_bytes] = drawn[:, : z.sk_bytes]
+    m.crypto_sign_keypair_from_seed(again.view(-1), z.pitch_keypair, n)
+    other = torch.zeros(300, z.pitch_keypair, dtype=torch.uint8, device="cuda")
+    m.crypto_sign_keypair(other.view(-1), z.pitch_keypair, 300, rand_index=5)
+    torch.cuda.synchronize()
+    assert (rows[:, at: at + z.pk_bytes].cpu().numpy() == cpk[pick]).all()
+    assert (erows.cpu().numpy() == esk[pick]).all()
+    assert torch.equal(drawn, again) and torch.equal(drawn, other[:n])
