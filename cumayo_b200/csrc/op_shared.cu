@@ -905,16 +905,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SH_GEMM_NT, 1)
 // step share one publish and the live columns fill whole warps); a CTA's last instances past the
 // batch repeat the batch's last instance and write nothing.
 // G (instances per CTA) is a runtime choice of the shared-key shape (mayo_b200_shared_set_shape):
-// 1, 2 or 4, the autotuner's candidates (4 only where the CTA fits in shared memory).
+// 1, 2 or 4, the autotuner's candidates (not 4 of MAYO_5, 640 threads).
 template <int SET, int G>
 struct TailShape {
     // threads per signature: three warps where the elimination's ko + 1 columns fit (MAYO_1: 81,
     // MAYO_2: 69); the row slots shrink with them (R = 3 / 12).  More signatures per SM
     // at the same registers: MAYO_2 G = 4, 4 CTAs of 384 threads at 40 registers (16 signatures
-    // per SM against 12 with 128 threads), 1.643 -> 1.494 ms at 65,536.
+    // per SM against 12 with 128 threads), 1.643 -> 1.505 ms at 65,536.
     static constexpr int TNT = (SET == 1 || SET == 2) ? 96 : (SET == 5 ? 160 : 128);
     static constexpr int NT = TNT * G;
-    // MAYO_5: 5 CTAs of 160 threads per SM held to a register budget (72 registers)
+    // MAYO_5: 5 CTAs of 160 threads per SM (72 registers): at 8,192 2.77 ms, 4 of them 3.00, 6 (60
+    // registers) 2.85, 3 3.47.  MAYO_3: 8 CTAs (64 registers) 1.44 ms, 6 1.51, 5 1.66.  MAYO_1, G = 2 at
+    // 16,384: 5 CTAs 1.22 ms, 4 1.24, 6 1.26.
     // MAYO_2: the elimination's per-step chain needs signatures in flight more than registers.
     // With 128 threads per signature at 65,536: G = 1, 9 CTAs per SM (56 registers) 1.866 ms;
     // G = 2 with 5 CTAs (48 registers) 1.739 ms (4 CTAs: 1.889, 6: 1.777); G = 4 with 3 CTAs
@@ -922,7 +924,7 @@ struct TailShape {
     // CTAs and G = 4 at 4 CTAs per SM (the same registers).
     static constexpr int MINB = SET == 5 ? (G == 1 ? 5 : 2)
                                 : SET == 2 ? (G == 1 ? 1 : G == 2 ? 7 : 4)
-                                : SET == 1 ? (G == 1 ? 8 : G == 2 ? 4 : 2) : 1;
+                                : SET == 1 ? (G == 1 ? 8 : G == 2 ? 5 : 2) : (G == 1 ? 8 : G == 2 ? 4 : 2);
     static constexpr size_t SMEM = (size_t)G * SignTailCfg<SET, TNT>::total;
 };
 template <int SET, int G>
@@ -1142,9 +1144,9 @@ struct SharedShape {
 };
 // Defaults (MAYO_1, 2, 3, 5), measured at 65,536 instances: the pair product is the faster one
 // for every set (MAYO_5 sign 14.0 against 18.5 ms: one CTA's key ring holds only four chunks
-// beside its vectors); signatures per sign-tail CTA: four for MAYO_2 (1.494 ms against 1.631 with
-// two, 1.840 with one), two for MAYO_1 (5.12 ms against 7.11 with one, 8.22 with four), one for
-// MAYO_3 and MAYO_5 (13.49 / 29.73 ms against 14.62 / 36.03 with two).
+// beside its vectors).  Signatures per sign-tail CTA, one, two and four: MAYO_1 at 16,384 1.41, 1.22,
+// 1.19 ms; MAYO_2 at 32,768 0.95, 0.83, 0.77; MAYO_3 at 8,192 1.44, 1.29, 1.30; MAYO_5 at 4,096 1.43, 1.36
+// (no four).
 constexpr int default_tail_g(int si) { return si == 1 ? 4 : si == 0 ? 2 : 1; }
 SharedShape g_shape[4] = {{HASH_NT, default_tail_g(0), 1}, {HASH_NT, default_tail_g(1), 1},
                           {HASH_NT, default_tail_g(2), 1}, {HASH_NT, default_tail_g(3), 1}};
@@ -1189,14 +1191,15 @@ static int launch_product(const uint8_t *key, const uint8_t *vec, size_t vec_str
 
 static unsigned fix_grid(size_t batch) { return (unsigned)(batch < SH_FIX_CTAS ? batch : SH_FIX_CTAS); }
 
-// The sign tail with G instances per CTA (ST_BAD_ARG where such a CTA does not fit).
+// The sign tail with G instances per CTA (ST_BAD_ARG where there is none).
 template <int SET, int G>
 static int launch_sign_tail(const SignIO &io, const uint4 *planes, const uint4 *opl, uint32_t *ctl, uint32_t *retry,
                             size_t batch, cudaStream_t st) {
     using TS = TailShape<SET, G>;
-    if constexpr (TS::SMEM > SH_SMEM_MAX) {
+    if constexpr (SET == 5 && G == 4) {
         return ST_BAD_ARG;
     } else {
+        static_assert(TS::SMEM <= SH_SMEM_MAX, "the CTA fits");
         if (!set_smem_attr(sign_shared_tail_kernel<SET, G>, TS::SMEM)) return ST_CUDA;
         sign_shared_tail_kernel<SET, G><<<(unsigned)((batch + G - 1) / G), TS::NT, TS::SMEM, st>>>(
             io.esk, io.sig, io.sig_stride, io.ws, io.ws_stride, planes, opl, ctl, retry, (uint32_t)batch);
@@ -1300,16 +1303,8 @@ int shared_timing_read(float *ms) {
     return ST_OK;
 }
 
-// Shared memory a sign-tail CTA of g instances needs (0 for a bad set).
-static size_t tail_smem(int set, int g) {
-    switch (set) {
-        case 1: return (size_t)g * SignTailCfg<1, TailShape<1, 1>::TNT>::total;
-        case 2: return (size_t)g * SignTailCfg<2, TailShape<2, 1>::TNT>::total;
-        case 3: return (size_t)g * SignTailCfg<3, TailShape<3, 1>::TNT>::total;
-        case 5: return (size_t)g * SignTailCfg<5, TailShape<5, 1>::TNT>::total;
-        default: return 0;
-    }
-}
+// Whether there is a sign-tail CTA of g instances: not four of MAYO_5.
+static bool tail_exists(int set, int g) { return !(set == 5 && g == 4); }
 
 int shared_set_shape(int set, int hash_nt, int tail_g, int product_ctas) {
     const int si = shape_index(set);
@@ -1317,7 +1312,7 @@ int shared_set_shape(int set, int hash_nt, int tail_g, int product_ctas) {
     if (hash_nt == 0) hash_nt = HASH_NT;
     if (tail_g == 0) tail_g = default_tail_g(si);
     if (hash_nt < 32 || hash_nt > 1024 || hash_nt % 32 || (tail_g != 1 && tail_g != 2 && tail_g != 4)) return ST_BAD_ARG;
-    if (tail_smem(set, tail_g) > SH_SMEM_MAX) return ST_BAD_ARG;
+    if (!tail_exists(set, tail_g)) return ST_BAD_ARG;
     if (product_ctas == 0) product_ctas = 2;
     if (product_ctas != 1 && product_ctas != 2) return ST_BAD_ARG;
     g_shape[si].hash_nt.store(hash_nt);

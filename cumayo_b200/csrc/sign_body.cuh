@@ -33,17 +33,18 @@ struct SignWs {
     static_assert(total <= S::scratch, "workspace fits the reference scratch region");
 };
 
-// Shared memory of what follows the key products, from `at`: M, the pivot buffer, y, hashes, x.
-#define MAYO_SIGN_TAIL_LAYOUT(at)                                                                        \
+// Shared memory of what follows the key products: M from `mpk`, the pivot buffer, y, hashes, x from `at`.
+#define MAYO_SIGN_TAIL_LAYOUT(mpk, at)                                                                    \
     static constexpr int NCOL = S::ko + 1;  /* columns of [A | y] */                                    \
     static constexpr int CPT = (NCOL + NT - 1) / NT;                                                     \
     static constexpr int NW = (S::menc + 3) / 4;                                                         \
     static constexpr size_t sz_acol = (size_t)NCOL * W * 16;                                             \
-    static constexpr size_t off_mpk = (at);                                                              \
-    static constexpr size_t off_piv = off_mpk + pad16((size_t)S::k * S::o * NW * 4);                     \
+    static constexpr size_t off_mpk = (mpk), sz_mpk = pad16((size_t)S::k * S::o * NW * 4);               \
+    static constexpr size_t off_piv = (at);                                                              \
     /* pivot buffer (uint4 items, two of them: step parity): the published pivot column ([w]), the      \
-       pivot row's one-hot words (2 items), the basis multiples of a_p^-1 (1 item; sign_eliminate) */   \
-    static constexpr int PIVQ = W + 3;                                                                   \
+       pivot row's one-hot words (2 items), the basis multiples of a_p^-1 (1 item), the sign of the     \
+       masks (1 item; sign_eliminate) */                                                                \
+    static constexpr int PIVQ = W + 4;                                                                   \
     static_assert(W <= 8, "one-hot words fit in two items");                                             \
     static constexpr size_t off_rhs = off_piv + (size_t)2 * PIVQ * 16;                                   \
     static constexpr size_t off_y = off_rhs + (size_t)W * 16;                                            \
@@ -67,11 +68,14 @@ struct SignTailCfg {
     static constexpr int R = NT / (J * W) < R0 ? NT / (J * W) : R0;
     static_assert(J * W * R <= NT, "row slots");
     static constexpr size_t off_masks = 0;
-    static constexpr size_t off_bs = off_masks + (size_t)S::v * J * 16;  // bit-plane columns of A
-    static constexpr size_t off_x = off_bs + (size_t)(S::ko + 1) * W * 16;
-    static constexpr size_t off_upk = off_x + (size_t)J * J * W * 16;
-    static constexpr size_t off_yext = off_upk + pad16((size_t)S::pairs * ((S::menc + 3) / 4) * 4);
-    MAYO_SIGN_TAIL_LAYOUT(off_yext + 128);
+    // U and M take the place of V's masks, the bit-plane columns of A that of the sums X: what is live
+    // together bounds the CTAs per SM of the larger sets (MAYO_5 68 -> 40 KB)
+    static constexpr size_t off_upk = off_masks, sz_upk = pad16((size_t)S::pairs * ((S::menc + 3) / 4) * 4);
+    static constexpr size_t off_bs = off_masks + (size_t)S::v * J * 16, off_x = off_bs;
+    static constexpr size_t sz_x = (size_t)J * J * W * 16, sz_cols = (size_t)(S::ko + 1) * W * 16;
+    static constexpr size_t off_yext = off_bs + (sz_x > sz_cols ? sz_x : sz_cols);
+    MAYO_SIGN_TAIL_LAYOUT(off_upk + sz_upk, off_yext + 128);
+    static_assert(off_mpk + sz_mpk <= off_bs, "U and M fit");
 };
 
 // The CTA, or cluster of CL CTAs, of a signature under its own key.  The quads -- MQ of columns of L,
@@ -113,7 +117,7 @@ struct SignCfg {
     static constexpr size_t sz_bs =
         cmax(cmax((size_t)J * TU * 16, (size_t)(S::ko + 1) * W * 16), (size_t)(S::o + S::k) * W * 16);
     static constexpr size_t off_yext = off_bs + sz_bs;
-    MAYO_SIGN_TAIL_LAYOUT(off_yext + 128);
+    MAYO_SIGN_TAIL_LAYOUT(off_yext + 128, off_mpk + sz_mpk);
 };
 
 // Columns of L (units of quads x < MQ) and rows of P1 (the others): off0 is the byte offset of row or
