@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 
+#include "ops.h"
+
 namespace mayo {
 
 __host__ __device__ constexpr size_t pad16(size_t x) { return (x + 15) / 16 * 16; }
@@ -21,6 +23,28 @@ template <class K>
 inline bool set_smem_attr(K kernel, size_t bytes) {
     if (bytes <= 48 * 1024) return true;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+}
+
+// Calls f(cl, first, count) -> status for the launches of a batch.  It is one launch, but up to
+// `waves` full waves of one-CTA instances (per_sm CTAs on each SM; 0: never) and a remainder that
+// clusters take are two: alone the remainder holds a few SMs for a whole wave's time.  MAYO_5, us:
+// verify 149 214 -> 150, 301 328 -> 263, 2,077 1,620 -> 1,574; keypair 149 380 -> 325; expand-sk 149
+// 576 -> 442; sign 301 572 -> 525.  Not where an SM's many small CTAs take the remainder up as they
+// finish (MAYO_2: verify 900 76.1 -> 76.5, keypair 940 319 -> 327, sign 900 138 -> 153), nor for a
+// signature after many waves, one of which is ever likelier to hold a second attempt that the
+// remainder would wait for.
+template <class F>
+inline int launch_waves(size_t batch, int per_sm, size_t waves, F f) {
+    if (per_sm == 0) return f(cluster_ctas(batch), size_t(0), batch);
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return ST_CUDA;
+    const size_t slots = (size_t)per_sm * (size_t)sms, rest = batch % slots;
+    if (batch < slots || batch / slots > waves || rest == 0 || cluster_ctas(rest) == 1)
+        return f(cluster_ctas(batch), size_t(0), batch);
+    const int rc = f(1, size_t(0), batch - rest);
+    return rc ? rc : f(cluster_ctas(rest), batch - rest, rest);
 }
 
 // Launch `kernel` on clusters of `cl` CTAs (cl = 1: a plain launch); ctas is a multiple of cl.

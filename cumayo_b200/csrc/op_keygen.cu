@@ -244,12 +244,14 @@ static int keypair_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st,
         rc = aes_expand(pool, pitch, batch, st, pk_off, p_off, S::p, false);
     }
     if (rc) return rc;
-    switch (cluster_ctas(batch)) {
-        case 8: return p3_cl<SET, 8>(pool, pitch, batch, st);
-        case 4: return p3_cl<SET, 4>(pool, pitch, batch, st);
-        case 2: return p3_cl<SET, 2>(pool, pitch, batch, st);
-        default: return p3_cl<SET, 1>(pool, pitch, batch, st);
-    }
+    return launch_waves(batch, SET == 2 ? 0 : KeyCfg<SET>::MINB, ~size_t(0), [&](int cl, size_t first, size_t n) {
+        switch (cl) {
+            case 8: return p3_cl<SET, 8>(pool + first * pitch, pitch, n, st);
+            case 4: return p3_cl<SET, 4>(pool + first * pitch, pitch, n, st);
+            case 2: return p3_cl<SET, 2>(pool + first * pitch, pitch, n, st);
+            default: return p3_cl<SET, 1>(pool + first * pitch, pitch, n, st);
+        }
+    });
 }
 
 template <int SET>
@@ -271,12 +273,14 @@ static int expandsk_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st
         rc = aes_expand(pool, pitch, batch, st, out_off + S::p - 16, out_off, S::p, true);
     }
     if (rc) return rc;
-    switch (cluster_ctas(batch)) {
-        case 8: return l_cl<SET, 8>(pool, pitch, batch, st);
-        case 4: return l_cl<SET, 4>(pool, pitch, batch, st);
-        case 2: return l_cl<SET, 2>(pool, pitch, batch, st);
-        default: return l_cl<SET, 1>(pool, pitch, batch, st);
-    }
+    return launch_waves(batch, LCfg<SET>::MINB, ~size_t(0), [&](int cl, size_t first, size_t n) {
+        switch (cl) {
+            case 8: return l_cl<SET, 8>(pool + first * pitch, pitch, n, st);
+            case 4: return l_cl<SET, 4>(pool + first * pitch, pitch, n, st);
+            case 2: return l_cl<SET, 2>(pool + first * pitch, pitch, n, st);
+            default: return l_cl<SET, 1>(pool + first * pitch, pitch, n, st);
+        }
+    });
 }
 
 template <int SET>

@@ -131,12 +131,14 @@ template <int SET>
 static int sign_t(const SignIO &io, size_t batch, cudaStream_t st) {
     const int rc = launch_sign_hash(SET, io, batch, st);
     if (rc != ST_OK) return rc;
-    switch (cluster_ctas(batch)) {
-        case 8: return sign_cl<SET, 8>(io, batch, st);
-        case 4: return sign_cl<SET, 4>(io, batch, st);
-        case 2: return sign_cl<SET, 2>(io, batch, st);
-        default: return sign_cl<SET, 1>(io, batch, st);
-    }
+    return launch_waves(batch, SET < 3 ? 0 : SignCfg<SET>::MINB, 2, [&](int cl, size_t first, size_t n) {
+        switch (cl) {
+            case 8: return sign_cl<SET, 8>(io.from(first), n, st);
+            case 4: return sign_cl<SET, 4>(io.from(first), n, st);
+            case 2: return sign_cl<SET, 2>(io.from(first), n, st);
+            default: return sign_cl<SET, 1>(io.from(first), n, st);
+        }
+    });
 }
 
 template <int SET>

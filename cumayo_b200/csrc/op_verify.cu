@@ -25,12 +25,14 @@ static int verify_cl(const VerifyIO &io, size_t batch, cudaStream_t st) {
 
 template <int SET>
 static int verify_t(const VerifyIO &io, size_t batch, cudaStream_t st) {
-    switch (cluster_ctas(batch)) {
-        case 8: return verify_cl<SET, 8>(io, batch, st);
-        case 4: return verify_cl<SET, 4>(io, batch, st);
-        case 2: return verify_cl<SET, 2>(io, batch, st);
-        default: return verify_cl<SET, 1>(io, batch, st);
-    }
+    return launch_waves(batch, SET == 2 ? 0 : VerifyCfg<SET>::MINB, ~size_t(0), [&](int cl, size_t first, size_t n) {
+        switch (cl) {
+            case 8: return verify_cl<SET, 8>(io.from(first), n, st);
+            case 4: return verify_cl<SET, 4>(io.from(first), n, st);
+            case 2: return verify_cl<SET, 2>(io.from(first), n, st);
+            default: return verify_cl<SET, 1>(io.from(first), n, st);
+        }
+    });
 }
 
 int launch_verify_io(int set, const VerifyIO &io, size_t batch, cudaStream_t st) {

@@ -52,6 +52,10 @@ struct MsgIO {
     const uint64_t *msg_off;
     const uint32_t *msg_len;
     uint32_t mlen;
+    MsgIO from(size_t i) const {  // of instances i, i + 1, ...
+        return MsgIO{msg_off ? msg : msg + i * msg_stride, msg_stride, msg_off ? msg_off + i : nullptr,
+                     msg_len ? msg_len + i : nullptr, mlen};
+    }
 #ifdef __CUDACC__
     __device__ __forceinline__ const uint8_t *ptr(size_t i) const { return msg_off ? msg + msg_off[i] : msg + i * msg_stride; }
     __device__ __forceinline__ uint32_t len(size_t i) const { return msg_len ? msg_len[i] : mlen; }
@@ -65,6 +69,9 @@ struct SignIO {
     size_t sig_stride;
     uint8_t *ws;  // per-instance workspace of sign_ws_bytes(set) bytes
     size_t ws_stride;
+    SignIO from(size_t i) const {
+        return SignIO{esk + i * esk_stride, esk_stride, m.from(i), sig + i * sig_stride, sig_stride, ws + i * ws_stride, ws_stride};
+    }
 };
 struct VerifyIO {
     const uint8_t *epk;  // P1 || P2 || P3
@@ -74,6 +81,10 @@ struct VerifyIO {
     size_t sig_stride;
     uint8_t *res;  // 0 = accept, 1 = reject
     size_t res_stride;
+    VerifyIO from(size_t i) const {
+        return VerifyIO{epk + i * epk_stride, epk_stride, m.from(i), sig + i * sig_stride, sig_stride, res + i * res_stride,
+                        res_stride};
+    }
 };
 int launch_sign_io(int set, const SignIO &io, size_t batch, cudaStream_t st);
 // Only the hash stage of sign (digest, salt, t, V || r for ctr 0 into io.ws).

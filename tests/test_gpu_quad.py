@@ -140,3 +140,49 @@ def test_keypair_keys_derived_or_hashed_first(case, n):
     assert (rows[:, at: at + z.pk_bytes].cpu().numpy() == cpk[pick]).all()
     assert (erows.cpu().numpy() == esk[pick]).all()
     assert torch.equal(drawn, again) and torch.equal(drawn, other[:n])
+
+
+@pytest.fixture(scope="module")
+def ragged(case):
+    s, _, esk, _, _, _, _ = case
+    rng = np.random.default_rng(900 + s)
+    msgs = [rng.integers(0, 256, int(n), dtype=np.uint8).tobytes() for n in rng.integers(0, 200, N)]
+    return msgs, O.sign_batch(s, esk, msgs)[0]
+
+
+@pytest.mark.parametrize("rest", [1, 12, 13, 32, 33, 72, 73])
+def test_full_waves_and_a_remainder(case, ragged, rest):
+    """Sign and verify of messages at offsets, keypair and expand-sk: 148 or 296 instances and a remainder."""
+    import torch
+    s, seeds, esk, epk, _, _, cpk = case
+    msgs, sig = ragged
+    m = Mayo(s)
+    z = m.sizes
+    lens = np.array([len(x) for x in msgs], np.uint32)
+    start = np.concatenate([[0], np.cumsum(lens[:-1])]).astype(np.uint64)
+    blob = torch.from_numpy(np.frombuffer(b"".join(msgs), np.uint8).copy()).cuda()
+    at = (z.sk_bytes + 127) // 128 * 128
+    for full in {1: (444,), 2: (296, 888), 3: (148, 296), 5: (148, 296)}[s]:
+        n = full + rest
+        pick = (np.arange(n) * 5 + 1) % N
+        d_off, d_len = torch.from_numpy(start[pick]).cuda(), torch.from_numpy(lens[pick]).cuda()
+        out = torch.zeros(n + 1, z.sig_bytes, dtype=torch.uint8, device="cuda")
+        ws = torch.zeros(n * m.sign_ws_bytes(), dtype=torch.uint8, device="cuda")
+        m.sign_many(torch.from_numpy(esk[pick]).cuda(), blob, out, ws, n, msg_off=d_off, msg_len=d_len,
+                    esk_stride=z.esk_bytes)
+        bad = sig[pick].copy()
+        bad[::7, 3] ^= 1
+        res = torch.full((n + 1,), 0xEE, dtype=torch.uint8, device="cuda")
+        m.verify_many(torch.from_numpy(epk[pick]).cuda(), blob, torch.from_numpy(bad).cuda(), res, n, msg_off=d_off,
+                      msg_len=d_len, epk_stride=z.epk_bytes)
+        rows = torch.zeros(n, z.pitch_keypair, dtype=torch.uint8, device="cuda")
+        rows[:, : z.sk_bytes] = torch.from_numpy(seeds[pick]).cuda()
+        m.crypto_sign_keypair_from_seed(rows.view(-1), z.pitch_keypair, n)
+        erows = torch.zeros(n, z.esk_bytes, dtype=torch.uint8, device="cuda")
+        erows[:, : z.sk_bytes] = rows[:, : z.sk_bytes]
+        m.crypto_sign_expandsk(erows.view(-1), z.esk_bytes, n)
+        torch.cuda.synchronize()
+        assert (out[:n].cpu().numpy() == sig[pick]).all() and not out[n:].any()
+        assert (res[:n].cpu().numpy() == (np.arange(n) % 7 == 0)).all() and (res[n:] == 0xEE).all()
+        assert (rows[:, at: at + z.pk_bytes].cpu().numpy() == cpk[pick]).all()
+        assert (erows.cpu().numpy() == esk[pick]).all()
