@@ -6,10 +6,9 @@
 // B200 layout: the round table T0 (Te0 of FIPS-197 in big-endian words) replicated 32 times in
 // shared memory, entry x of copy c at word 32*x + c, so lane c always hits bank c and the 16
 // data-dependent lookups of a round never conflict.  The other three round tables are byte
-// rotations of T0.  The expansion kernel keeps T0, ror8(T0) and ror16(T0) (96 KB, two CTAs of 384
-// threads per SM) and rotates only for the fourth; the work-queue kernel's keypair keeps T0 (and
-// ror16(T0) for MAYO_5) in the area its P3 engine uses next and rotates with PRMT.  The S-box for
-// the last round is byte 1 of T0[x].  Tables are computed at compile time from GF(2^8) arithmetic.
+// rotations of T0.  The expansion kernel keeps all four (128 KB, one persistent CTA per SM); the
+// work-queue kernel's keypair keeps as many as fit in the area its P3 uses next and rotates with PRMT
+// for the others.  The S-box for the last round is byte 1 of T0[x].  Tables are computed at compile time from GF(2^8) arithmetic.
 #pragma once
 
 #include <type_traits>
@@ -109,9 +108,9 @@ __constant__ uint32_t c_aes_stride = 128;
 // address (the multiplier `k128` = 128 is a kernel argument or a constant-bank value, so the
 // address arithmetic stays on the IMAD pipe instead of joining the extractions, rotations and
 // XORs on the logic pipe, which with the table reads sets the pace) and the read.  Measured at
-// MAYO_1's 1,024 x 9,031 blocks: one table with PRMT rotations and shifted-index addresses
-// 0.250 ms, IMAD addresses 0.234, two tables 0.222, three tables in two CTAs of 384 threads per
-// SM 0.203 (byte-exact).
+// MAYO_1's 1,024 x 9,031 blocks, all rounds by lookups: one table 0.234 ms, two 0.222, three (two CTAs
+// of 384 threads per SM) 0.203; with the first two rounds shared (AesRun), persistent CTAs: three
+// 0.197, four and a preparing warp 0.174.  133 lookups of a block at one wavefront each take 0.137.
 template <int NTAB>
 struct AesLut {
     static_assert(NTAB >= 1 && NTAB <= 4, "one to four tables");
@@ -248,11 +247,11 @@ __device__ __forceinline__ void aes_store(uint8_t *out, uint32_t blk, const AesO
 // ---------------------------------------------------------------------------------------------
 // Kernel: AES-CTR keystream of nbytes into a pitched pool.  An item is (instance, chunk): chunk x of an
 // instance takes blocks [x * bpc, (x + 1) * bpc) to row + out_off, keyed by 16 bytes at row + key_off
-// (or derived, see AesDerive).  A CTA builds the tables once and takes items blockIdx.x, + gridDim.x, ...; while its
-// worker warps run one item, the last warp prepares the next one (key schedule, the chunk's AesRuns).
-// The workers take the item's blocks 64 at a time from a counter (32 where an item has few).  When the key overlaps the output
-// (expand-pk, expand-sk keep seed_pk in the last 16 output bytes until expansion), nbytes ends
-// before the blocks that overlap the key and aes_ctr_tail_kernel finishes them afterwards, one
+// (or derived, see AesDerive).  A CTA builds the tables once and takes items blockIdx.x, + gridDim.x,
+// ...; while its worker warps run one item, the last warp prepares the next one (key schedule, the
+// chunk's AesRuns).  The workers take the item's blocks 64 at a time from a counter (32 where an item
+// has few).  When the key overlaps the output (expand-pk, and expand-sk that does not derive, keep
+// seed_pk in the last 16 output bytes until expansion), nbytes ends before the blocks that overlap the key and aes_ctr_tail_kernel finishes them afterwards, one
 // thread per instance.
 // ---------------------------------------------------------------------------------------------
 constexpr int AES_WORKERS = 768, AES_THREADS = AES_WORKERS + 32;  // and the warp that prepares

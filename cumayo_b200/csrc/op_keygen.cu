@@ -1,8 +1,9 @@
 // op_keygen.cu -- batched keypair, expand-sk and expand-pk on B200.
 //
-// keypair  (reference src/keypair.cu:10-121):  hash kernel (thread per instance: seed_sk,
-//          seed_pk || O) -> AES-CTR kernel (P1 || P2 into the row's scratch) -> P3 engine kernel.
-// expandsk (src/expandsk.cu:9-81): hash kernel (O, seed_pk) -> AES-CTR -> L engine kernel.
+// keypair  (reference src/keypair.cu:10-121):  hash kernel (seed_sk, seed_pk || O) -> AES-CTR kernel
+//          (P1 || P2 into the row's scratch) -> P3 kernel.
+// expandsk (src/expandsk.cu:9-81): hash kernel (O, seed_pk) -> AES-CTR -> L kernel.
+//          (Small batches: the AES-CTR kernel hashes too.)
 // expandpk (src/expandpk.cu:9-23): AES-CTR only.
 #include "aes.cuh"
 #include "keygen_body.cuh"
@@ -170,8 +171,9 @@ static bool aes_plan(uint32_t nbytes, size_t batch, AesPlan &p) {
 // The kernel derives the keys itself where each CTA gets one item, so that an instance's hash is on
 // every CTA's path once and the rest of its sponge runs beside the encryption: keypair of one MAYO_1
 // 38.5 -> 31.2 us (of MAYO_2, whose O takes five more blocks of the sponge, 41.7 -> 43.5), of 72 56.7 ->
-// 43.3, of 148 80.0 -> 63.6; expand-sk, whose tail launch goes too, 37.8 -> 27.0 and 63.9 -> 45.8.  With several items per CTA the one preparing
-// warp's Keccak (5 us an item) holds the workers up: MAYO_2 at 1,024 334 us -> 394.
+// 43.3, of 148 80.0 -> 63.6; expand-sk, whose tail launch goes too, 37.8 -> 27.0 and 63.9 -> 45.8.
+// With several items per CTA the one preparing warp's Keccak (5 us an item) holds the workers up:
+// MAYO_2 at 1,024 334 us -> 394.
 static bool aes_derives(const AesPlan &p, size_t batch) { return batch * p.chunks <= p.ctas; }
 
 // nbytes of keystream for every row, keyed from row + key_off or, with DERIVE, from the seeds.

@@ -166,7 +166,7 @@ __device__ ItemRefs queue_refs(const QueueOps &o, uint32_t inst) {
     return r;
 }
 
-// ---- keypair from a caller seed on one CTA: hash (warp 0), AES-CTR (all), P3 (engine) ----
+// ---- keypair from a caller seed on one CTA: hash (warp 0), AES-CTR (all), P3 ----
 template <int SET>
 __device__ void queue_keypair(uint8_t *smem, int tid, const QueueOps &ops, uint32_t inst, uint8_t *scratch) {
     using S = Set<SET>;

@@ -30,9 +30,9 @@
 //         attempt from the planes in a compact CTA) -> sign_shared_fix_kernel (retries of the
 //         rare singular first attempts per instance).
 //   verify: verify_hash_kernel (thread per instance: digest, t) -> product ->
-//         verify_shared_tail_kernel (U from the planes, Horner, compare; a small CTA).
+//         verify_shared_tail_kernel (U from the planes, y, compare; a small CTA).
 //   If the status word shows a failed product, the tails do nothing and the fix-up kernels run
-//   every instance through the per-instance engine, so results stay correct.
+//   every instance through the per-instance kernels' code, so results stay correct.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -899,7 +899,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SH_GEMM_NT, 1)
 }
 
 // ---- sign ----
-// First attempt from the planes, in a CTA without engine staging (more CTAs per SM).  A singular
+// First attempt from the planes, in a CTA without room for the key products (more CTAs per SM).  A singular
 // first attempt goes to the retry list; the fix-up kernel finishes it per instance.
 // SH_TAIL_G instances per CTA (sign_attempt's interleaved elimination: the G pivot owners of a
 // step share one publish and the live columns fill whole warps); a CTA's last instances past the
@@ -911,7 +911,7 @@ struct TailShape {
     // threads per signature: three warps where the elimination's ko + 1 columns fit (MAYO_1: 81,
     // MAYO_2: 69); the row slots shrink with them (R = 3 / 12).  More signatures per SM
     // at the same registers: MAYO_2 G = 4, 4 CTAs of 384 threads at 40 registers (16 signatures
-    // per SM against 12 with 128 threads), 1.643 -> 1.505 ms at 65,536.
+    // per SM against 12 with 128 threads), 1.643 -> 1.492 ms at 65,536.
     static constexpr int TNT = (SET == 1 || SET == 2) ? 96 : (SET == 5 ? 160 : 128);
     static constexpr int NT = TNT * G;
     // MAYO_5: 5 CTAs of 160 threads per SM (72 registers): at 8,192 2.77 ms, 4 of them 3.00, 6 (60
@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(32 * VERIFY_HASH_WARPS)
     warp_shake<136>(t, S::menc, key, S::digest + S::sk, wk, lane);
 }
 
-// U_ij = s_i^T T_j from the planes, y = Horner over the pairs, compare with t.  No engine
+// U_ij = s_i^T T_j from the planes, y from the pairs, compare with t.  No key
 // staging, no hashing: a small CTA.
 template <int SET>
 struct VTailCfg {

@@ -23,7 +23,7 @@
 //     as the products keep the logic pipe (MAYO_1: 62 and 57 clocks per column; measured 89).
 // Verify at 3,552 / 3,552 / 2,072 / 1,036 instances with keys of their own (MAYO_1, 2, 3, 5): 0.33,
 // 0.17, 0.66, 1.46 us per instance with the plane products (16 LOP3, rows staged
-// in shared memory between barriers), 0.153, 0.067, 0.43, 0.85 here.
+// in shared memory between barriers), 0.153, 0.064, 0.381, 0.752 here.
 // Scalars enter only as masks and no address depends on them: constant time.
 #pragma once
 

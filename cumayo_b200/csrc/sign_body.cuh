@@ -67,6 +67,10 @@ struct SignTailCfg {
     static constexpr int R0 = SET == 2 ? 16 : (SET == 1 ? 4 : 2);
     static constexpr int R = NT / (J * W) < R0 ? NT / (J * W) : R0;
     static_assert(J * W * R <= NT, "row slots");
+    // The warp that folds y also sums it up, instead of all warps by atomics: less to issue (MAYO_2's
+    // tail at 65,536 1.505 -> 1.492 ms, MAYO_1 at 16,384 1.222 -> 1.213, MAYO_5 at 8,192 2.777 -> 2.756),
+    // but MAYO_3's 1.443 -> 1.461.
+    static constexpr bool Y_ONE_WARP = SET != 3;
     static constexpr size_t off_masks = 0;
     // U and M take the place of V's masks, the bit-plane columns of A that of the sums X: what is live
     // together bounds the CTAs per SM of the larger sets (MAYO_5 68 -> 40 KB)
@@ -105,6 +109,7 @@ struct SignCfg {
     static constexpr int MINB = CL > 1 ? 1 : (SET == 1 ? 3 : SET == 2 ? 6 : SET == 3 ? 2 : 1);
     // slots of T a part needs: its quads of P1 (a chunk's last lanes write past them)
     static constexpr int TU = CH * 32;
+    static constexpr bool Y_ONE_WARP = false;
     static constexpr size_t off_masks = 0;
     static constexpr size_t sz_masks = (size_t)S::v * ST * 16;
     static constexpr size_t sz_mask2 = (size_t)QL * ST * 16, sz_upk = pad16((size_t)S::pairs * NQ * 4);
@@ -339,7 +344,7 @@ __device__ __forceinline__ void sign_products_pre(uint8_t *smem, int tid, const 
     }
     __syncthreads();
     // ---- the unreduced y = sum z^l U_l, and M unpacked ----
-    y_accumulate<SET>(upk, yext, tid >> 5, NT / 32, tid & 31);
+    if constexpr (!C::Y_ONE_WARP) y_accumulate<SET>(upk, yext, tid >> 5, NT / 32, tid & 31);
     for (int idx = tid; idx < J * S::o * W; idx += NT) {
         const int w = idx % W, jb = idx / W, b = jb % S::o, j = jb / S::o;
         const uint4 pk = g4_to_packed(g4_ld(pre + ((size_t)j * NROWS + S::v + b) * W + w));
@@ -487,6 +492,10 @@ __device__ __forceinline__ bool sign_attempt(uint8_t *smem0, int T, const uint8_
     static_assert(KO < NT, "the right-hand side has a thread in the first pass over the columns");
     if ((tid >> 5) == KO / 32) {
         const int lane = tid & 31;
+        if constexpr (C::Y_ONE_WARP) {
+            y_accumulate<SET>(upk, reinterpret_cast<uint32_t *>(smem + C::off_yext), 0, 1, lane);
+            __syncwarp();
+        }
         const uint32_t y = y_fold<SET>(reinterpret_cast<const uint32_t *>(smem + C::off_yext), lane);
         if (lane < NW) ypk[lane] = y ^ reinterpret_cast<const uint32_t *>(s_t)[lane];
         __syncwarp();
