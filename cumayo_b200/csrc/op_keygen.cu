@@ -138,15 +138,18 @@ __global__ void __launch_bounds__(LCfg<SET, CL>::NT, LCfg<SET, CL>::MINB) l_kern
 // Launchers
 // ---------------------------------------------------------------------------------------------
 // Near-equal chunks per instance: the split whose busiest CTA has the least to do, an item counting
-// its blocks and AES_ITEM_COST.  MAYO_1 (9,031 blocks) at 1,024: 207, 185, 181, 177 us with items of
-// at most 1,536, 3,072, 6,400 and 12,288 blocks; MAYO_5 (52,616) at 128: 140 us with 6,400, 150 with
-// 12,288 (640 items on 148 CTAs).
-static uint32_t aes_chunks(uint32_t nblk, size_t batch, uint32_t ctas, uint32_t *bpc) {
+// its blocks and AES_ITEM_COST, a split instance whose key lies in the output the tail kernel.  MAYO_1
+// (9,031 blocks) at 1,024: 207, 185, 181, 177 us with items of at most 1,536, 3,072, 6,400 and 12,288
+// blocks.  Items of up to a whole MAYO_5 key (52,616) against 12,288: verifyWithepk of 1,024 MAYO_3
+// 832 -> 809 us, of 592 MAYO_5 996 -> 965; expand-sk of 148 MAYO_5 387 -> 356; keypair of 777 1,292 -> 1,273.
+static uint32_t aes_chunks(uint32_t nblk, size_t batch, uint32_t ctas, bool tail, uint32_t *bpc) {
     uint32_t best = 0;
     uint64_t least = ~0ull;
-    for (uint32_t c = (nblk + AES_BLOCKS_PER_ITEM - 1) / AES_BLOCKS_PER_ITEM; c <= (nblk + AES_WORKERS / 2 - 1) / (AES_WORKERS / 2); c++) {
+    const uint32_t least_c = (nblk + AES_BLOCKS_PER_ITEM - 1) / AES_BLOCKS_PER_ITEM;
+    for (uint32_t c = least_c; c <= (nblk + AES_WORKERS / 2 - 1) / (AES_WORKERS / 2); c++) {
         const uint32_t n = (nblk + c - 1) / c;
-        const uint64_t cost = ((uint64_t)batch * c + ctas - 1) / ctas * (n + AES_ITEM_COST);
+        const uint64_t cost =
+            ((uint64_t)batch * c + ctas - 1) / ctas * (n + AES_ITEM_COST) + (tail && c > 1 ? AES_TAIL_COST : 0);
         if (cost < least) {
             least = cost;
             best = c;
@@ -159,13 +162,13 @@ static uint32_t aes_chunks(uint32_t nblk, size_t batch, uint32_t ctas, uint32_t 
 struct AesPlan {
     uint32_t ctas, chunks, bpc;
 };
-static bool aes_plan(uint32_t nbytes, size_t batch, AesPlan &p) {
+static bool aes_plan(uint32_t nbytes, size_t batch, bool key_in_output, AesPlan &p) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return false;
     p.ctas = (uint32_t)sms;
-    p.chunks = aes_chunks((nbytes + 15) / 16, batch, p.ctas, &p.bpc);
+    p.chunks = aes_chunks((nbytes + 15) / 16, batch, p.ctas, key_in_output, &p.bpc);
     return true;
 }
 // The kernel derives the keys itself where each CTA gets one item, so that an instance's hash is on
@@ -198,12 +201,12 @@ static int aes_main(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, 
 static int aes_expand(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, size_t key_off, size_t out_off,
                       uint32_t nbytes, bool key_in_output) {
     AesPlan plan;
-    if (!aes_plan(nbytes, batch, plan)) return ST_CUDA;
+    if (!aes_plan(nbytes, batch, key_in_output, plan)) return ST_CUDA;
     if (!key_in_output || plan.chunks == 1)
         return aes_main<false>(pool, pitch, batch, st, key_off, out_off, nbytes, plan, AesDerive{});
     // the main kernel writes whole blocks that do not touch the key
     const uint32_t nblk_main = min(nbytes / 16, (uint32_t)((key_off - out_off) / 16));
-    if (!aes_plan(nblk_main * 16, batch, plan)) return ST_CUDA;
+    if (!aes_plan(nblk_main * 16, batch, true, plan)) return ST_CUDA;
     const int rc = aes_main<false>(pool, pitch, batch, st, key_off, out_off, nblk_main * 16, plan, AesDerive{});
     if (rc != ST_OK) return rc;
     aes_ctr_tail_kernel<<<(unsigned)((batch + AES_TAIL_THREADS - 1) / AES_TAIL_THREADS), AES_TAIL_THREADS, 0, st>>>(
@@ -234,7 +237,7 @@ static int keypair_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st,
     const size_t pk_off = align128(S::sk), p_off = pk_off + align128(S::pk);
     int rc;
     AesPlan plan;
-    if (!aes_plan(S::p, batch, plan)) return ST_CUDA;
+    if (!aes_plan(S::p, batch, false, plan)) return ST_CUDA;
     if (aes_derives(plan, batch)) {
         rc = aes_main<true>(pool, pitch, batch, st, pk_off, p_off, S::p, plan,
                       AesDerive{(uint32_t)S::sk, (uint32_t)S::o_bytes, 1u, seeded ? 0u : 1u, pk_off + 16, rand_index});
@@ -264,7 +267,7 @@ static int expandsk_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st
     const size_t out_off = S::sk + S::o_bytes;
     int rc;
     AesPlan plan;
-    if (!aes_plan(S::p, batch, plan)) return ST_CUDA;
+    if (!aes_plan(S::p, batch, false, plan)) return ST_CUDA;
     if (aes_derives(plan, batch)) {
         rc = aes_main<true>(pool, pitch, batch, st, 0, out_off, S::p, plan,
                       AesDerive{(uint32_t)S::sk, (uint32_t)S::o_bytes, 0u, 0u, (size_t)S::sk, 0});
