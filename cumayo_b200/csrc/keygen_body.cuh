@@ -266,7 +266,7 @@ __device__ __forceinline__ void l_instance(uint8_t *smem, int tid, const uint8_t
                 store_word(P2 + (size_t)((r0 + i) * S::o + j) * S::menc + 4 * q, wd[i] ^ w[i], QuadCfg<SET>::bytes(q));
     };
     for (;;) {
-        const int item = warp_next(s_next, lane), lc = item / C::PC, piece = item - lc * C::PC;
+        const int item = warp_next(s_next, lane), lc = C::PC > 1 ? item / C::PC : item, piece = item - lc * C::PC;
         const int chunk = rank + CL * lc;
         if (chunk >= C::CH) break;
         const int u = chunk * 32 + lane, t = u / NQ, q = u - t * NQ, r0 = 4 * t;
@@ -274,17 +274,23 @@ __device__ __forceinline__ void l_instance(uint8_t *smem, int tid, const uint8_t
         QuadAcc<J> acc;
         acc.zero();
         SymRows<SET> rows{mis, (uint32_t)(4 * q), r0, false};
-        const int ca = S::v * piece / C::PC, cb = S::v * (piece + 1) / C::PC;
 #pragma unroll 1
         for (int seg = 0; seg < 2; seg++) {  // from the diagonal on, then the columns left of every row
             rows.lower = seg == 1;
-            quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), seg ? ca : max(ca, 4 * qmin),
-                                             seg ? min(cb, 4 * qmin) : cb, seg ? 0 : 4 * qmax + 4, masks, mis == 0);
+            int c0 = seg ? 0 : 4 * qmin, c1 = seg ? 4 * qmin : S::v;
+            if constexpr (C::PC > 1) {  // the piece's columns
+                c0 = max(c0, S::v * piece / C::PC);
+                c1 = min(c1, S::v * (piece + 1) / C::PC);
+            }
+            quad_columns<SET, J, true, C::D>(acc, rows, base4, QuadCfg<SET>::bytes(q), c0, c1, seg ? 0 : 4 * qmax + 4, masks,
+                                             mis == 0);
         }
+        if constexpr (C::PC > 1) {
 #pragma unroll
-        for (int j = 0; j < J; j++) {
-            if constexpr (C::PC > 1) g4_atomic_xor(T + (j * C::CHC + lc) * 32 + lane, acc.fold(j));
-            else store(acc.fold(j), r0, j, q);
+            for (int j = 0; j < J; j++) g4_atomic_xor(T + (j * C::CHC + lc) * 32 + lane, acc.fold(j));
+        } else {
+#pragma unroll
+            for (int j = 0; j < J; j++) store(acc.fold(j), r0, j, q);
         }
     }
     if constexpr (C::PC > 1) {
