@@ -396,7 +396,7 @@ struct WarpKeccak {
 
 // Bytes p .. p + n - 1 (n <= 8; none for n <= 0) as a little-endian word, from the aligned 8-byte
 // words that hold them.
-__device__ __forceinline__ uint64_t ld_bytes(const uint8_t *p, int n) {
+__host__ __device__ __forceinline__ uint64_t ld_bytes(const uint8_t *p, int n) {
     if (n <= 0) return 0;
     const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 7u);
     const uint64_t *q = reinterpret_cast<const uint64_t *>(p - off);
@@ -405,27 +405,29 @@ __device__ __forceinline__ uint64_t ld_bytes(const uint8_t *p, int n) {
     return n < 8 ? w & (~0ull >> (64 - 8 * n)) : w;
 }
 
+// Word `lane` (< RATE / 8) of the block at `in`, of whose input `left` bytes are still to come; the
+// last block (left < RATE) is padded.  A length is any 32-bit number: messages may pass 2 GiB.
+template <int RATE>
+__host__ __device__ __forceinline__ uint64_t shake_word(const uint8_t *in, uint32_t left, int lane) {
+    const int n = (int)(left < (uint32_t)RATE ? left : (uint32_t)RATE) - 8 * lane;  // input bytes from this word on
+    uint64_t w = ld_bytes(in + 8 * lane, n < 8 ? n : 8);
+    if (left < (uint32_t)RATE) {
+        if (n >= 0 && n < 8) w ^= (uint64_t)0x1F << (8 * n);
+        if (lane == RATE / 8 - 1) w ^= 0x8000000000000000ull;
+    }
+    return w;
+}
+
 // A warp's SHAKE sponge over byte strings in any memory space: lane l < RATE / 8 absorbs and squeezes
 // word l of a block.  in_len / out_len in bytes; `in` and `out` must not overlap.
 template <int RATE>
-__device__ void warp_shake(uint8_t *out, int out_len, const uint8_t *in, int in_len, const WarpKeccak &wk,
+__device__ void warp_shake(uint8_t *out, int out_len, const uint8_t *in, uint32_t in_len, const WarpKeccak &wk,
                            int lane) {
     uint64_t a = 0;
-    int off = 0;
-    for (;;) {
-        const bool last = (in_len - off) < RATE;
-        if (lane < RATE / 8) {
-            const int at = off + lane * 8, n = min(in_len - at, 8);
-            uint64_t w = ld_bytes(in + at, n);
-            if (last) {
-                if (n >= 0 && n < 8) w ^= (uint64_t)0x1F << (8 * n);
-                if (lane == RATE / 8 - 1) w ^= 0x8000000000000000ull;
-            }
-            a ^= w;
-        }
-        if (last) break;
+    for (uint32_t off = 0;; off += RATE) {
+        if (lane < RATE / 8) a ^= shake_word<RATE>(in + off, in_len - off, lane);
+        if (in_len - off < (uint32_t)RATE) break;
         a = wk.permute(a, lane);
-        off += RATE;
     }
     for (int o = 0; o < out_len; o += RATE) {
         a = wk.permute(a, lane);

@@ -1010,7 +1010,7 @@ __global__ void __launch_bounds__(32 * VERIFY_HASH_WARPS)
     uint8_t *key = reinterpret_cast<uint8_t *>(s_key[w]), *t = tws + (size_t)inst * tws_stride;
     WarpKeccak wk;
     wk.setup(lane);
-    warp_shake<136>(key, S::digest, io.m.ptr(inst), (int)io.m.len(inst), wk, lane);
+    warp_shake<136>(key, S::digest, io.m.ptr(inst), io.m.len(inst), wk, lane);
     const uint8_t *salt = io.sig + (size_t)inst * io.sig_stride + S::k * S::n / 2;
     for (int i = lane; i < S::sk; i += 32) key[S::digest + i] = salt[i];
     for (int i = S::menc + lane; i < (S::menc + 3) / 4 * 4; i += 32) t[i] = 0;

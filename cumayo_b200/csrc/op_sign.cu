@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(32 * SIGN_HASH_WARPS) sign_hash_warp_kernel(co
         key[S::digest + S::sk + i] = seed_sk[i];
     }
     if (lane == 0) key[KEY - 1] = 0;
-    warp_shake<136>(key, S::digest, io.m.ptr(inst), (int)io.m.len(inst), wk, lane);  // sign.cu:225
+    warp_shake<136>(key, S::digest, io.m.ptr(inst), io.m.len(inst), wk, lane);  // sign.cu:225
     warp_shake<136>(salt, S::sk, key, S::digest + 2 * S::sk, wk, lane);              // sign.cu:230-238
     for (int i = lane; i < S::sk; i += 32) key[S::digest + i] = salt[i];
     __syncwarp();

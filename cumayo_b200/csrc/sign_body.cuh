@@ -251,7 +251,7 @@ __device__ __forceinline__ void sign_hash_cta(uint8_t *smem, int tid, const uint
         const int lane = tid;
         WarpKeccak wk;
         wk.setup(lane);
-        warp_shake<136>(s_key, S::digest, msg, (int)mlen, wk, lane);
+        warp_shake<136>(s_key, S::digest, msg, mlen, wk, lane);
         for (int i = lane; i < S::sk; i += 32) {
             s_key[S::digest + i] = 0;
             s_key[S::digest + S::sk + i] = esk[i];

@@ -105,7 +105,7 @@ __device__ __forceinline__ void verify_instance(uint8_t *smem, int tid, const ui
     if (rank == 0 && warp == 0) {  // digest and target t (src/verify.cu:37-48)
         WarpKeccak wk;
         wk.setup(lane);
-        warp_shake<136>(s_key, S::digest, msg, (int)mlen, wk, lane);
+        warp_shake<136>(s_key, S::digest, msg, mlen, wk, lane);
         for (int i = lane; i < S::sk; i += 32) s_key[S::digest + i] = s_sig[S::k * S::n / 2 + i];
         __syncwarp();
         warp_shake<136>(s_t, S::menc, s_key, S::digest + S::sk, wk, lane);
