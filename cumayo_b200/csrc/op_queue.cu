@@ -24,10 +24,8 @@
 
 #include "../../include/mayo_b200.h"
 #include "aes.cuh"
-#include "keygen_body.cuh"
 #include "ops.h"
-#include "sign_body.cuh"
-#include "verify_body.cuh"
+#include "queue_cfg.cuh"
 
 namespace mayo {
 
@@ -36,42 +34,6 @@ constexpr uint32_t Q_STOP = 0xFFFFFFFEu;
 constexpr uint32_t Q_ABANDONED = 0xFFFFFFFDu;  // a slot past the tail whose ticket was given up (no item has op 3)
 constexpr int Q_BUCKETS = 12;             // (set index) * 3 + op
 constexpr int Q_CTRL_WORDS = 16;          // control words per bucket; block 12 counts invalid ops
-
-template <int SET, int OP>
-struct QueueCfg;
-
-template <int SET>
-struct QueueCfg<SET, MAYO_B200_OP_KEYPAIR> {
-    using S = Set<SET>;
-    // MAYO_2: four warps instead of the batched kernel's two, for the expansion's sake
-    using KC = KeyCfg<SET, 1, SET == 2 ? 4 : 0>;
-    static constexpr int NT = KC::NT, MINB = KC::MINB;
-    // as many replicated round tables as the P3 area below O holds (MAYO_1: T0; MAYO_2: T0 and
-    // ror16(T0); MAYO_3: three; MAYO_5: all four) and the round keys; dead once the keystream is written
-    static constexpr size_t runs = ((size_t)S::p / 16 + 256) / 256 + 1;  // AesRuns of an instance
-    static constexpr size_t aes_bytes(int n) { return (size_t)n * 256 * 32 * 4 + 44 * 4 + 16 * runs; }
-    static constexpr int NTAB = KC::off_o >= aes_bytes(4) ? 4 : KC::off_o >= aes_bytes(3) ? 3 : KC::off_o >= aes_bytes(2) ? 2 : 1;
-    static constexpr size_t run = (size_t)NTAB * 256 * 32 * 4 + 44 * 4;  // after the round keys (16-byte aligned)
-    static constexpr size_t aes_end = aes_bytes(NTAB);
-    static_assert(KC::off_o >= aes_end, "O must not overlap the AES tables");
-    static constexpr size_t seedpk = KC::off_o + pad16(S::o_bytes);
-    static constexpr size_t smem = seedpk + 16;
-    static constexpr size_t scratch = pad16((size_t)S::p + 16);  // P1 || P2 of one keypair
-};
-
-template <int SET>
-struct QueueCfg<SET, MAYO_B200_OP_SIGN> {
-    static constexpr int NT = SignCfg<SET>::NT, MINB = SignCfg<SET>::MINB;
-    static constexpr size_t smem = SignCfg<SET>::total;
-    static constexpr size_t scratch = 0;
-};
-
-template <int SET>
-struct QueueCfg<SET, MAYO_B200_OP_VERIFY> {
-    static constexpr int NT = VerifyCfg<SET>::NT, MINB = VerifyCfg<SET>::MINB;
-    static constexpr size_t smem = VerifyCfg<SET>::total;
-    static constexpr size_t scratch = 0;
-};
 
 using QueueOps = mayo_b200_queue_ops;
 
