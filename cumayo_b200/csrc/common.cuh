@@ -427,9 +427,10 @@ __device__ void warp_shake(uint8_t *out, int out_len, const uint8_t *in, uint32_
                            int lane) {
     uint64_t a = 0;
 #pragma unroll 1
-    for (;; in += RATE, in_len -= RATE) {
-        if (lane < RATE / 8) a ^= shake_word<RATE>(in, in_len, lane);
-        if (in_len < (uint32_t)RATE) break;
+    for (size_t off = 0;; off += RATE) {
+        const uint32_t left = in_len - (uint32_t)off;
+        if (lane < RATE / 8) a ^= shake_word<RATE>(in + off, left, lane);
+        if (left < (uint32_t)RATE) break;
         a = wk.permute(a, lane);
     }
     for (int o = 0; o < out_len; o += RATE) {

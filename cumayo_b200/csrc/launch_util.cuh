@@ -25,6 +25,13 @@ inline bool set_smem_attr(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
 }
 
+// The current device's SMs.
+inline bool device_sms(int &sms) {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+}
+
 // Calls f(cl, first, count) -> status for the launches of a batch.  It is one launch, but up to
 // `waves` full waves of one-CTA instances (per_sm CTAs on each SM; 0: never) and a remainder that
 // clusters take are two: alone the remainder holds a few SMs for a whole wave's time.  MAYO_5, us:
@@ -36,10 +43,8 @@ inline bool set_smem_attr(K kernel, size_t bytes) {
 template <class F>
 inline int launch_waves(size_t batch, int per_sm, size_t waves, F f) {
     if (per_sm == 0) return f(cluster_ctas(batch), size_t(0), batch);
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return ST_CUDA;
+    int sms = 0;
+    if (!device_sms(sms)) return ST_CUDA;
     const size_t slots = (size_t)per_sm * (size_t)sms, rest = batch % slots;
     if (batch < slots || batch / slots > waves || rest == 0 || cluster_ctas(rest) == 1)
         return f(cluster_ctas(batch), size_t(0), batch);

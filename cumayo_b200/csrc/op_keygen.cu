@@ -163,10 +163,8 @@ struct AesPlan {
     uint32_t ctas, chunks, bpc;
 };
 static bool aes_plan(uint32_t nbytes, size_t batch, bool key_in_output, AesPlan &p) {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return false;
+    int sms = 0;
+    if (!device_sms(sms)) return false;
     p.ctas = (uint32_t)sms;
     p.chunks = aes_chunks((nbytes + 15) / 16, batch, p.ctas, key_in_output, &p.bpc);
     return true;

@@ -56,8 +56,9 @@ struct VerifyCfg {
 
 // Verify one instance; every thread of the CTA (VerifyCfg::NT of them), or of every CTA of the
 // cluster (rank = this CTA's), must call it.  Writes 0 (accept) or 1 (reject) to *res.  `smem` holds
-// VerifyCfg<SET, CL>::total bytes, at the same address in every CTA of a cluster.
-template <int SET, int CL = 1>
+// VerifyCfg<SET, CL>::total bytes, at the same address in every CTA of a cluster.  HASHED: the message's
+// digest is at off_key already (the caller's stores need no barrier), `msg` and `mlen` are not used.
+template <int SET, int CL = 1, bool HASHED = false>
 __device__ __forceinline__ void verify_instance(uint8_t *smem, int tid, const uint8_t *epk, const uint8_t *msg,
                                                 uint32_t mlen, const uint8_t *sig, uint8_t *res, int rank = 0) {
     using S = Set<SET>;
@@ -105,7 +106,7 @@ __device__ __forceinline__ void verify_instance(uint8_t *smem, int tid, const ui
     if (rank == 0 && warp == 0) {  // digest and target t (src/verify.cu:37-48)
         WarpKeccak wk;
         wk.setup(lane);
-        warp_shake<136>(s_key, S::digest, msg, mlen, wk, lane);
+        if constexpr (!HASHED) warp_shake<136>(s_key, S::digest, msg, mlen, wk, lane);
         for (int i = lane; i < S::sk; i += 32) s_key[S::digest + i] = s_sig[S::k * S::n / 2 + i];
         __syncwarp();
         warp_shake<136>(s_t, S::menc, s_key, S::digest + S::sk, wk, lane);
