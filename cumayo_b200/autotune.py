@@ -6,7 +6,8 @@ order in which the bucket kernels are launched (the first one launched takes the
 later ones fill in as its CTAs finish) — and keeps the fastest.
 
 tune_shared: for one set's sign_shared + verify_shared on a given batch it times the block shapes
-the library can run — threads per CTA of the thread-per-instance hash kernels (32..256) and
+the library can run — threads per CTA of the thread-per-instance hash kernels (32..256; batches above
+HASH_WARP_MAX only, smaller ones hash by a warp per instance) and
 signatures per sign-tail CTA (1, or 2 or 4 with the instances' elimination columns interleaved) and
 CTAs per key-product tile (1, or a CTA pair sharing each tile's key rows) — and sets the fastest
 (mayo_b200_shared_set_shape).
@@ -117,6 +118,12 @@ def tune_queue(q: "Q.Queue", items: np.ndarray, repeats: int = 2, use_cache: boo
 
 
 SHARED_CANDIDATES = [(h, g, p) for p in (1, 2) for g in (1, 2, 4) for h in (32, 64, 128, 256)]
+HASH_WARP_MAX = 2048  # batches up to this hash by a warp per instance (csrc/ops.h): hash_threads has no effect
+
+
+def shared_candidates(batch: int) -> list:
+    """The block shapes that differ at `batch`: up to HASH_WARP_MAX one hash size, the default."""
+    return [c for c in SHARED_CANDIDATES if batch > HASH_WARP_MAX or c[0] == 64]
 
 
 def _lib_id() -> str:
@@ -143,7 +150,7 @@ def tune_shared(m, run, batch: int, repeats: int = 3, flush=None, use_cache: boo
         best = cache[key]
     else:
         trials = []
-        for h, g, p in SHARED_CANDIDATES:
+        for h, g, p in shared_candidates(batch):
             try:
                 m.set_shared_shape(h, g, p)
             except Exception:  # a shape this set's kernels cannot take (shared memory)
