@@ -257,7 +257,10 @@ __device__ __forceinline__ void aes_store(uint8_t *out, uint32_t blk, const AesO
 constexpr int AES_WORKERS = 768, AES_THREADS = AES_WORKERS + 32;  // and the warp that prepares
 constexpr int AES_BLOCKS_PER_ITEM = 53248;  // at most (a MAYO_5 key has 52,616)
 constexpr int AES_ITEM_COST = 700;          // what an item costs besides its blocks, in blocks (its workers drain)
-constexpr int AES_TAIL_COST = 5000;         // what the tail kernel costs, in blocks (11 us)
+// What the tail kernel costs, in blocks: its launch and the one (MAYO_2) or two it takes one after the
+// other.  Expand-pk of 32 / 40 / 48 MAYO_2, one item per key and no tail 26.7 us, split with the tail
+// 22.2, 23.3, 25.4; of 48 / 52 MAYO_1 split 31.1, one item 34.
+constexpr int AES_TAIL_COST = 2500, AES_TAIL_BLOCK_COST = 1250;
 constexpr int AES_RUNS = AES_BLOCKS_PER_ITEM / 256 + 2;
 constexpr size_t AES_SMEM = 4 * 256 * 32 * 4;  // T0 and its rotations by 8, 16, 24, each replicated 32 times
 

@@ -142,14 +142,14 @@ __global__ void __launch_bounds__(LCfg<SET, CL>::NT, LCfg<SET, CL>::MINB) l_kern
 // (9,031 blocks) at 1,024: 207, 185, 181, 177 us with items of at most 1,536, 3,072, 6,400 and 12,288
 // blocks.  Items of up to a whole MAYO_5 key (52,616) against 12,288: verifyWithepk of 1,024 MAYO_3
 // 832 -> 809 us, of 592 MAYO_5 996 -> 965; expand-sk of 148 MAYO_5 387 -> 356; keypair of 777 1,292 -> 1,273.
-static uint32_t aes_chunks(uint32_t nblk, size_t batch, uint32_t ctas, bool tail, uint32_t *bpc) {
+static uint32_t aes_chunks(uint32_t nblk, size_t batch, uint32_t ctas, uint32_t tail, uint32_t *bpc) {
     uint32_t best = 0;
     uint64_t least = ~0ull;
     const uint32_t least_c = (nblk + AES_BLOCKS_PER_ITEM - 1) / AES_BLOCKS_PER_ITEM;
     for (uint32_t c = least_c; c <= (nblk + AES_WORKERS / 2 - 1) / (AES_WORKERS / 2); c++) {
         const uint32_t n = (nblk + c - 1) / c;
         const uint64_t cost =
-            ((uint64_t)batch * c + ctas - 1) / ctas * (n + AES_ITEM_COST) + (tail && c > 1 ? AES_TAIL_COST : 0);
+            ((uint64_t)batch * c + ctas - 1) / ctas * (n + AES_ITEM_COST) + (c > 1 ? tail : 0);
         if (cost < least) {
             least = cost;
             best = c;
@@ -162,11 +162,12 @@ static uint32_t aes_chunks(uint32_t nblk, size_t batch, uint32_t ctas, bool tail
 struct AesPlan {
     uint32_t ctas, chunks, bpc;
 };
-static bool aes_plan(uint32_t nbytes, size_t batch, bool key_in_output, AesPlan &p) {
+// tail: what the tail kernel costs a split instance (0: none is needed).
+static bool aes_plan(uint32_t nbytes, size_t batch, uint32_t tail, AesPlan &p) {
     int sms = 0;
     if (!device_sms(sms)) return false;
     p.ctas = (uint32_t)sms;
-    p.chunks = aes_chunks((nbytes + 15) / 16, batch, p.ctas, key_in_output, &p.bpc);
+    p.chunks = aes_chunks((nbytes + 15) / 16, batch, p.ctas, tail, &p.bpc);
     return true;
 }
 // The kernel derives the keys itself where each CTA gets one item, so that an instance's hash is on
@@ -199,12 +200,13 @@ static int aes_main(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, 
 static int aes_expand(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st, size_t key_off, size_t out_off,
                       uint32_t nbytes, bool key_in_output) {
     AesPlan plan;
-    if (!aes_plan(nbytes, batch, key_in_output, plan)) return ST_CUDA;
+    // where there is a tail kernel, the main kernel writes the whole blocks that do not touch the key
+    const uint32_t nblk_main = key_in_output ? min(nbytes / 16, (uint32_t)((key_off - out_off) / 16)) : 0;
+    const uint32_t tail = key_in_output ? AES_TAIL_COST + AES_TAIL_BLOCK_COST * ((nbytes + 15) / 16 - nblk_main) : 0;
+    if (!aes_plan(nbytes, batch, tail, plan)) return ST_CUDA;
     if (!key_in_output || plan.chunks == 1)
         return aes_main<false>(pool, pitch, batch, st, key_off, out_off, nbytes, plan, AesDerive{});
-    // the main kernel writes whole blocks that do not touch the key
-    const uint32_t nblk_main = min(nbytes / 16, (uint32_t)((key_off - out_off) / 16));
-    if (!aes_plan(nblk_main * 16, batch, true, plan)) return ST_CUDA;
+    if (!aes_plan(nblk_main * 16, batch, tail, plan)) return ST_CUDA;
     const int rc = aes_main<false>(pool, pitch, batch, st, key_off, out_off, nblk_main * 16, plan, AesDerive{});
     if (rc != ST_OK) return rc;
     aes_ctr_tail_kernel<<<(unsigned)((batch + AES_TAIL_THREADS - 1) / AES_TAIL_THREADS), AES_TAIL_THREADS, 0, st>>>(
@@ -235,7 +237,7 @@ static int keypair_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st,
     const size_t pk_off = align128(S::sk), p_off = pk_off + align128(S::pk);
     int rc;
     AesPlan plan;
-    if (!aes_plan(S::p, batch, false, plan)) return ST_CUDA;
+    if (!aes_plan(S::p, batch, 0, plan)) return ST_CUDA;
     if (aes_derives(plan, batch)) {
         rc = aes_main<true>(pool, pitch, batch, st, pk_off, p_off, S::p, plan,
                       AesDerive{(uint32_t)S::sk, (uint32_t)S::o_bytes, 1u, seeded ? 0u : 1u, pk_off + 16, rand_index});
@@ -265,7 +267,7 @@ static int expandsk_t(uint8_t *pool, size_t pitch, size_t batch, cudaStream_t st
     const size_t out_off = S::sk + S::o_bytes;
     int rc;
     AesPlan plan;
-    if (!aes_plan(S::p, batch, false, plan)) return ST_CUDA;
+    if (!aes_plan(S::p, batch, 0, plan)) return ST_CUDA;
     if (aes_derives(plan, batch)) {
         rc = aes_main<true>(pool, pitch, batch, st, 0, out_off, S::p, plan,
                       AesDerive{(uint32_t)S::sk, (uint32_t)S::o_bytes, 0u, 0u, (size_t)S::sk, 0});
