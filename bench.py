@@ -886,7 +886,7 @@ def setup_mixed_queue(args, dist, batch, seed, st):
     per = [batch // 12 + (1 if i < batch % 12 else 0) for i in range(12)]
     operands, entries, plain_parts = {}, [], []
     h2d_list, d2h_list, h_res_parts = [], [], []
-    work_macs = 0.0
+    work_ops = 0.0
     for si, s in enumerate(sets):
         m = M.Mayo(s)
         z = m.sizes
@@ -909,8 +909,8 @@ def setup_mixed_queue(args, dist, batch, seed, st):
                                     vf_mlen=mlen, vf_sig=d_sig_vf, vf_res=d_res)
         entries += [(Q.OP_KEYPAIR, s, i) for i in range(n_kp)] + [(Q.OP_SIGN, s, i) for i in range(n_sg)] + \
                    [(Q.OP_VERIFY, s, i) for i in range(n_vf)]
-        mc = mac_counts(s)
-        work_macs += n_kp * mc["keypair"] + n_sg * mc["sign"] + n_vf * mc["verify"]
+        ops = lane_ops(s, False)
+        work_ops += n_kp * ops["keypair"] + n_sg * ops["sign"] + n_vf * ops["verify"]
         # plain per-(set, op) launches doing the same work
         kpool, kpch = m.alloc_pool("keypair", n_kp)
         kpool.view(n_kp, kpch)[:, : z.sk_bytes].copy_(d_seeds)
@@ -973,7 +973,7 @@ def setup_mixed_queue(args, dist, batch, seed, st):
                      "capacity": q.capacity, "autotune_trials": tuned.get("trials")},
            "graph": "CUDA graph (queue reset, partition, 12 persistent (set, op) kernels) replayed per step",
            "l2": "flushed between steps (256 MiB write)"}
-    return ([("queue", queue_op)], h2d, d2h, h2d_bytes, d2h_bytes, batch, {"queue": work_macs},
+    return ([("queue", queue_op)], h2d, d2h, h2d_bytes, d2h_bytes, batch, {"queue": work_ops},
             {"queue": 0}, cfg, expected, res_dev, h_res, plain, 14)
 
 
