@@ -486,7 +486,7 @@ def run_ours(args, dist: Dist):
         K2[:, : z.sk_bytes].copy_(h_seeds)
         S2[:, msg_s: msg_s + mlen].copy_(h_msgs)
         V2[:, msg_v: msg_v + mlen].copy_(h_msgs)
-        launches_per_step = 13  # keypair 4 (hash, AES, tail, P3), signWithesk 6, verifyWithepk 3
+        launches_per_step = 10  # keypair 3 (hash, AES, P3), signWithesk 5 (hash, AES, L, hash, sign), verifyWithepk 2
 
         def keypair_op():
             m.crypto_sign_keypair_from_seed(kpool, kp, batch, st)
