@@ -129,7 +129,7 @@ def test_inject(kind: int, arg: int = 0, spin: int = 0) -> None:
     INJECT_QUEUE_LOST_PUSH gives every queue bucket a slot nothing publishes, so its bounded
     wait runs out (MAYO_B200_QUEUE_ERR_TIMEOUT); INJECT_PRODUCT_STALL stops the tensor-core
     product's key loader after `arg` chunks with waits of `spin` polls (the status word becomes
-    1 and the per-instance engine computes the results); INJECT_NONE turns it off."""
+    1 and the per-instance kernels' code computes the results); INJECT_NONE turns it off."""
     _check(lib().mayo_b200_test_inject(kind, arg, spin), "test_inject")
 
 

@@ -295,15 +295,6 @@ struct Sponge {
             }
         }
     }
-    __device__ __forceinline__ void absorb_byte(uint8_t b) {
-#pragma unroll
-        for (int i = 0; i < RW; i++)
-            if (i == (pos >> 3)) s[i] ^= (uint64_t)b << (8 * (pos & 7));
-        if (++pos == RATE) {
-            keccak_f1600(s);
-            pos = 0;
-        }
-    }
     __device__ __forceinline__ void finalize() {
 #pragma unroll
         for (int i = 0; i < RW; i++)

@@ -20,8 +20,9 @@ struct KeyCfg {
     // Warps and CTAs per SM, keypairs at 2,072 (us per instance): MAYO_1 three CTAs of four warps 0.321
     // against 0.330 with four CTAs (128 registers, spills); MAYO_2 (153 accumulators) two warps 0.312
     // against 0.322 with four and 0.486 with three CTAs of three warps (spills); MAYO_3 two CTAs of
-    // six warps 0.796 against 0.809 with four warps and two columns ahead (then 0.698; eight warps in one CTA 0.729);
-    // MAYO_5 one CTA of eight warps, two columns ahead, 1.55 against 1.69 with eleven, one ahead.
+    // six warps (168 registers, a few words spilled) 0.796 against 0.809 with four warps and two columns
+    // ahead; beside a faster expansion 0.698 against 0.729 with eight warps in one CTA; MAYO_5 one CTA of
+    // eight warps, two columns ahead, 1.55 against 1.69 with eleven, one ahead.
     static constexpr int CW = CW_ ? CW_ : CL > 1 ? 8 : (SET == 1 ? 4 : SET == 2 ? 2 : SET == 3 ? 6 : 8);
     static constexpr int NT = 32 * CW;
     static constexpr int PC = CL > 1 ? (2 * CW + CH - 1) / CH : 1;

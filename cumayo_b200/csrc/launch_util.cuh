@@ -37,9 +37,10 @@ inline bool device_sms(int &sms) {
 // clusters take are two: alone the remainder holds a few SMs for a whole wave's time.  MAYO_5, us:
 // verify 149 214 -> 150, 301 328 -> 263, 2,077 1,620 -> 1,574; keypair 149 380 -> 325; expand-sk 149
 // 576 -> 442; sign 301 572 -> 525.  Not where an SM's many small CTAs take the remainder up as they
-// finish (MAYO_2: verify 900 76.1 -> 76.5, keypair 940 319 -> 327, sign 900 138 -> 153), nor for a
-// signature after many waves, one of which is ever likelier to hold a second attempt that the
-// remainder would wait for.
+// finish (MAYO_2: verify 900 76.1 -> 76.5, keypair 940 319 -> 327, sign 900 138 -> 153; MAYO_1's three
+// in sign: 450 204 -> 254), nor for a signature after more waves than two: the remainder waits for
+// every second attempt of the first launch (MAYO_5, 777, five waves: 1,105 -> 1,254; one and two waves
+// gained in sign, three and four were not measured).
 template <class F>
 inline int launch_waves(size_t batch, int per_sm, size_t waves, F f) {
     if (per_sm == 0) return f(cluster_ctas(batch), size_t(0), batch);

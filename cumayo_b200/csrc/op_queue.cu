@@ -9,7 +9,8 @@
 // Each (set, op) has its own kernel because their CTAs need 23-205 KB of shared memory and 96-255
 // registers per thread: one kernel shaped for the largest would run every set at one CTA per SM
 // (MAYO_1 runs three, MAYO_2's sign and verify six).  Each kernel has the
-// shape of the batched kernel for its (set, op).  On forked streams the kernels share the SMs,
+// shape of the batched kernel for its (set, op), but MAYO_2's keypair (four warps, queue_cfg.cuh); the
+// item loop around the same code costs all of them a few spilled words.  On forked streams the kernels share the SMs,
 // and the CTAs of a kernel launched later take the SMs of one whose bucket has drained, so one
 // bucket's tail overlaps another's work.
 //

@@ -1142,11 +1142,12 @@ struct SharedShape {
     std::atomic<int> tail_g;   // instances per sign-tail CTA
     std::atomic<int> pair;     // the key product on CTA pairs (shared_gemm2_kernel)
 };
-// Defaults (MAYO_1, 2, 3, 5), measured at 65,536 instances: the pair product is the faster one
-// for every set (MAYO_5 sign 14.0 against 18.5 ms: one CTA's key ring holds only four chunks
-// beside its vectors).  Signatures per sign-tail CTA, one, two and four: MAYO_1 at 16,384 1.41, 1.22,
-// 1.19 ms; MAYO_2 at 32,768 0.95, 0.83, 0.77; MAYO_3 at 8,192 1.44, 1.29, 1.30; MAYO_5 at 4,096 1.43, 1.36
-// (no four).
+// Defaults (MAYO_1, 2, 3, 5).  The pair product is the faster one for every set at 65,536 instances
+// (MAYO_5 sign 14.0 against 18.5 ms: one CTA's key ring holds only four chunks beside its vectors).
+// Signatures per sign-tail CTA, one, two and four: MAYO_1 at 16,384 1.41, 1.22, 1.19 ms; MAYO_2 at 32,768
+// 0.95, 0.83, 0.77; MAYO_3 at 8,192 1.44, 1.29, 1.30; MAYO_5 at 4,096 1.43, 1.36 (no four).  The defaults
+// are part of the interface (the header's 2, 4, 1, 1) and so are not the fastest for MAYO_1, 3 and 5;
+// mayo_b200_shared_set_shape or the autotuner chooses those.
 constexpr int default_tail_g(int si) { return si == 1 ? 4 : si == 0 ? 2 : 1; }
 SharedShape g_shape[4] = {{HASH_NT, default_tail_g(0), 1}, {HASH_NT, default_tail_g(1), 1},
                           {HASH_NT, default_tail_g(2), 1}, {HASH_NT, default_tail_g(3), 1}};

@@ -13,9 +13,13 @@ namespace mayo {
 // SM, so small CTAs spread a batch evenly over the 148 SMs (whole waves).
 constexpr int HASH_NT = 64;
 // Batches up to this are hashed by a warp per instance: a thread's Keccak-f takes about 5 us however
-// few there are, a warp's 2.4 us, and a batch of a few thousand warps still fits the GPU.  Sign hash,
-// us, warp against thread per instance (MAYO_1 / 5): one instance 29 / 45 against 51 / 90, 1,024
-// 38 / 57 against 86 / 150, 2,048 51 / 79 against 87 / 152, 4,096 78 / 122 against 88 / 150.
+// few there are, a warp's 2.4 us, and a batch of a few thousand warps still fits the GPU.  One line for
+// all hash kernels: at 2,048 the warp form is the faster one of every kernel and set, at 4,096 only of
+// sign's for MAYO_1, 3 and 5.  us, warp / thread per instance, MAYO_1, 2, 3, 5:
+//   keypair    2,048  17 / 21, 27 / 33, 27 / 33, 36 / 44;  4,096  27 / 21, 42 / 33, 42 / 33, 58 / 45
+//   expand-sk  2,048  18 / 23, 27 / 33, 27 / 33, 37 / 44;  4,096  27 / 23, 43 / 33, 43 / 34, 58 / 45
+//   sign       2,048  40 / 67, 29 / 33, 45 / 84, 67 / 120;  4,096  64 / 69, 46 / 33, 72 / 86, 107 / 123
+//   verify (shared key)  2,048  13 / 17 (all);  4,096  20 / 17
 constexpr size_t HASH_WARP_MAX = 2048;
 
 // Status codes shared with include/mayo_b200.h.

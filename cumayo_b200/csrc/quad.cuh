@@ -117,7 +117,8 @@ __device__ __forceinline__ void quad_forms(uint32_t s0, uint32_t s1, uint32_t s2
 // the address arithmetic at an add, a shift and an IMAD.WIDE, and are the funnel shift's amount
 // (modulo 32) as they stand.  SAFE: the second word is read only where the n bytes reach it (n < 4
 // in the last word of an m-vector); otherwise it may hold only bytes of the entry that follows, so
-// the caller uses SAFE for the last entry of a buffer.
+// the caller uses SAFE for the last entry of a buffer: quad_columns for the last column of its range,
+// past which the entry that follows may lie in another buffer.
 struct RawWord {
     uint32_t lo, hi;
 };

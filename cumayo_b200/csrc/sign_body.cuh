@@ -157,9 +157,6 @@ struct SignRows {
     }
 };
 
-// Position of pair (a <= b) in the A-assembly order (sign.cu:333-392): i = 0..k-1, j = k-1..i.
-__device__ __forceinline__ int ell_of(int a, int b, int k) { return a * k - (a * (a - 1)) / 2 + (k - 1 - b); }
-
 // Packed word q (8 coordinates) of z^ell * u for a packed m-vector u (NW words in shared memory),
 // without the fold: coordinates >= m are dropped.
 template <int SET>
@@ -520,7 +517,7 @@ __device__ __forceinline__ bool sign_attempt(uint8_t *smem0, int T, const uint8_
             for (int q = 0; q < OVW; q++) ovs[q] = 0;
 #pragma unroll 1
             for (int j = 0; j < S::k; j++) {
-                const int ell = i <= j ? ell_of(i, j, S::k) : ell_of(j, i, S::k);
+                const int ell = i <= j ? pair_ell(i, j, S::k) : pair_ell(j, i, S::k);  // sign.cu:333-392
                 const uint32_t *u = mpk + ((size_t)j * S::o + b) * NW;
                 if constexpr (NW <= 10) {
                     // z^ell u without the fold: the packed words shifted up by 4 ell bits -- a

@@ -82,7 +82,7 @@ MAYO_B200_API int mayo_b200_last_cuda_error(void);
  *   MAYO_B200_INJECT_PRODUCT_STALL: in mayo_b200_sign_shared / _verify_shared the key loader of
  *     each tensor-core product CTA stops after `arg` chunks without telling the other warps,
  *     and the product's waits give up after `spin` polls (0 = the default bound).  The product
- *     then sets its status word to 1 and the per-instance engine computes every result.
+ *     then sets its status word to 1 and the per-instance kernels' code computes every result.
  * MAYO_B200_ERR_ARG for an unknown kind. */
 enum {
     MAYO_B200_INJECT_NONE = 0,
@@ -178,7 +178,7 @@ MAYO_B200_API int mayo_b200_verify_many(int set, const uint8_t *epk, size_t epk_
  * the rest of each operation runs per instance as in _many.  `ws` is device memory of
  * mayo_b200_*_shared_ws_bytes(set, batch) bytes, 16-byte aligned; its first 4 bytes hold a
  * status word after the call (0 = the tensor-core product ran; 1 = a bounded wait in it ran
- * out and the per-instance engine produced the results instead). */
+ * out and the per-instance kernels' code produced the results instead). */
 MAYO_B200_API size_t mayo_b200_sign_shared_ws_bytes(int set, size_t batch);
 MAYO_B200_API int mayo_b200_sign_shared(int set, const uint8_t *esk, const uint8_t *msgs, const uint64_t *msg_off,
                                         const uint32_t *msg_len, size_t msg_stride, size_t mlen, uint8_t *sig,
