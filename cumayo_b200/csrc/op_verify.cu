@@ -22,13 +22,14 @@ __global__ void __launch_bounds__(VerifyCfg<SET, CL>::NT, VerifyCfg<SET, CL>::MI
 // us one by one / by groups, at 4,096, 8,192 and 32,768 bytes:
 //   MAYO_1   500  274 / 250,   468 / 327,   1,622 / 947;     4,096  1,414 / 1,199, 2,466 / 1,555,  8,776 / 3,713
 //   MAYO_3   300  405 / 305,   716 / 420,   2,515 / 1,088;   4,096  3,707 / 2,147, 6,512 / 2,646, 23,288 / 5,673
-//   MAYO_5   300  (6,145) 604 / 546, 761 / 599, 2,565 / 1,205;  4,096  5,671 / 4,219, 7,076 / 4,422, 23,876 / 7,028
-// The lines lie where the two meet in batches of a few waves.  MAYO_2's six CTAs per SM hash side by
+//   MAYO_5   300      -      761 / 599, 2,565 / 1,205;  4,096      -         7,076 / 4,422, 23,876 / 7,028
+// The lines lie where the two meet in batches of two waves, which gain least (MAYO_1, 450: 3,072 bytes 218 /
+// 219; MAYO_3, 149: 2,049 160 / 173, 3,072 202 / 197; MAYO_5, 149: 6,145 395 / 421, 8,192 492 / 470).  MAYO_2's six CTAs per SM hash side by
 // side as it is.  By the host's length only: with lengths on the device either kernel would have to
 // look at each, which cost short messages 0.3 to 12 %.
 template <int SET>
 struct VerifyLong {
-    static constexpr size_t len = SET == 1 ? 3328 : SET == 2 ? ~size_t(0) : SET == 3 ? 2048 : 6144;
+    static constexpr size_t len = SET == 1 ? 3328 : SET == 2 ? ~size_t(0) : SET == 3 ? 3072 : 7168;
 };
 template <int SET>
 static bool verify_is_long(const MsgIO &m) {

@@ -13,7 +13,7 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 N = 13  # distinct keys and messages: no multiple of a group
-LIMIT = {1: 3328, 2: 3328, 3: 2048, 5: 6144}
+LIMIT = {1: 3328, 2: 3328, 3: 3072, 5: 7168}
 BATCHES = {1: (444, 445, 1335, 1775, 1777), 2: (900,), 3: (148, 149, 1183, 1185), 5: (148, 149, 299, 1185)}
 
 
